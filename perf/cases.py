@@ -185,7 +185,10 @@ def _nested_dissection(n, side, layers, hubs, pad_of):
 @functools.lru_cache(maxsize=None)
 def _pattern(kind, size, seed):
     """(circuit, preprocessing arrays, symbolic analysis) of one pattern."""
-    c = gen.mna_netlist(size, seed) if kind == "mna" else gen.power_grid(size, seed)
+    if kind == "mna":
+        c = gen.mna_netlist(size, seed)
+    else:                                    # small meshes with the tests' pads and hubs
+        c = gen.power_grid(size, seed, **(dict(pads=16, hubs=4) if size < 128 else {}))
     path = os.path.join(_GOLDEN, f"nicslu_{kind}{size}_s{seed}.npz")
     if os.path.exists(path):
         nic = glu.NicsluArrays.from_npz(path)
