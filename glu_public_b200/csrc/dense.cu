@@ -1,8 +1,8 @@
 // Dense-phase kernels for sm_100a (FP64): the trailing block that fill has made dense.
 //
 // Per panel step k (width NB):
-//   k_dense_diag_rows / k_dense_diag
-//                  one CTA per instance factors the NB x NB diagonal block (a row per thread in
+//   k_dense_diag64 / k_dense_diag
+//                  one CTA per instance factors the NB x NB diagonal block (8 columns per warp in
 //                  registers for NB = 64, 16 x 16 register tiles for NB = 128); per pivot the
 //                  reference's column math: pivot (perturbed if |d| < pert and the column has
 //                  an L part, src/numeric.cu:139-140), L(:,kk) /= d (src/numeric.cu:37-47), then
@@ -126,63 +126,206 @@ __global__ void __launch_bounds__(256) k_dense_diag(DenseView V,
     for (int j = 0; j < R; ++j) D[(tx + 16 * i) + (int64_t)(ty + 16 * j) * ld] = a[i][j];
 }
 
-// Pivot step KK of k_dense_diag_rows, instantiated per pivot so that the row stays in registers
-// (every index into a[] is a compile-time constant).
-template <int KK>
-__device__ __forceinline__ void diag_rows_step(double (&a)[64], double (&prow)[2][64], int i,
-                                               double pv, const uint8_t* __restrict__ hasl,
-                                               int32_t* status, int b, int nv) {
-  if constexpr (KK < 64) {
-    if (KK >= nv) return;                        // the rest is identity padding
-    if constexpr (KK >= 0) {
-      if (i > KK) {
-        const double* __restrict__ r = prow[KK & 1];
-        const double l = a[KK] / r[KK];
-        a[KK] = l;
+__device__ __forceinline__ bool finite_bits(double x) {
+  return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+
+// x / d from r = 1 / d with one FMA correction (Markstein's division: q = x r, e = x - q d,
+// q + e r; Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., sec. 4.7): within an ulp
+// of x / d, three dependent operations, and no slow path for the zeros a padded or nearly dense
+// block is full of.  An infinite or NaN first quotient (zero pivot, overflow) is returned as it is.
+__device__ __forceinline__ double quotient(double x, double d, double r) {
+  const double q = x * r;
+  const double e = fma(fma(-q, d, x), r, q);
+  return finite_bits(q) ? e : q;
+}
+
+__device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+constexpr int kDiagSt = 68;          // == 4 (mod 16) doubles: conflict-free DMMA fragments
+
+// The 8 x 8 block at pivot 8 s of the factorization below, by one warp: a row per lane (lanes past
+// 8 repeat them).  Pivot row c goes to the other lanes through Ub[8 c ..] (shared memory), which
+// is also its final value, so a lane whose pivot is done computes on without being preserved;
+// L(j, c) goes to Lb[8 c + j] and the pivots' reciprocals to rcp.  Kept to the instructions of
+// the chain itself: one warp issues at its latency here, some 7 cycles per instruction.
+template <bool PERT>
+__device__ __forceinline__ void diag64_block(const double* __restrict__ T, double* __restrict__ Ub,
+                                             double* __restrict__ Lb, double* __restrict__ rcp,
+                                             int s, int lane, double pv, unsigned hasl,
+                                             int32_t* status, int b) {
+  const int i = lane & 7;
+  const double* __restrict__ P = T + s * 8 * (kDiagSt + 1) + i;
+  double a[8];
 #pragma unroll
-        for (int j = KK + 1; j < 64; ++j) a[j] -= l * r[j];
-      }
-    }
-    if constexpr (KK + 1 < 64) {
-      if (i == KK + 1) {                         // row KK + 1 is final: pivot and publish it
-        const double d0 = a[KK + 1];
-        const bool perturbed = pv > 0.0 && hasl[KK + 1] && fabs(d0) < pv;
-        const double d = perturbed ? pv : d0;
-        a[KK + 1] = d;
-        pivot_flags(status, b, d, perturbed);
+  for (int j = 0; j < 8; ++j) a[j] = P[j * kDiagSt];
 #pragma unroll
-        for (int j = KK + 1; j < 64; ++j) prow[(KK + 1) & 1][j] = a[j];
-      }
+  for (int c = 0; c < 8; ++c) {
+    double2* __restrict__ rw = reinterpret_cast<double2*>(Ub + c * 8);
+    if (PERT && lane == c && ((hasl >> c) & 1u) && fabs(a[c]) < pv) {
+      a[c] = pv;
+      atomicOr(status + b, GLU_INST_PERTURBED);
     }
-    __syncthreads();
-    diag_rows_step<KK + 1>(a, prow, i, pv, hasl, status, b, nv);
+    if (lane == c) {
+#pragma unroll
+      for (int j = c / 2; j < 4; ++j) rw[j] = make_double2(a[2 * j], a[2 * j + 1]);
+    }
+    __syncwarp();
+    double u[8];
+#pragma unroll
+    for (int j = c / 2; j < 4; ++j) {
+      const double2 v = rw[j];
+      u[2 * j] = v.x;
+      u[2 * j + 1] = v.y;
+    }
+    const double r = 1.0 / u[c];
+    const double q = quotient(a[c], u[c], r);
+#pragma unroll
+    for (int j = c + 1; j < 8; ++j) a[j] -= q * u[j];
+    Lb[c * 8 + i] = q;                         // entries i <= c are never read
+    rcp[c] = r;
   }
 }
 
-// Same factorization of a 64 x 64 diagonal block with one thread per row, the row held in
-// registers: per pivot kk every lower row divides by the pivot and applies the rank-1 update with
-// the pivot row read from a double-buffered shared copy; the thread owning row kk + 1 -- the last
-// writer of the next pivot -- applies the perturbation and publishes its row right away, so one
-// barrier per pivot suffices.  Lower latency than the 16 x 16 tiled kernel above, which matters
-// when one block sits on the critical path.
-__device__ __forceinline__ void diag_rows_body(const DenseView& V, const double* __restrict__ pert,
-                                               int32_t* status, int k, int b) {
-  constexpr int NB = 64;
-  __shared__ __align__(16) double prow[2][NB];
-  const int i = threadIdx.x;
-  const int64_t ld = V.ld;
-  double* __restrict__ D = V.base + (int64_t)b * V.stride + (int64_t)k + (int64_t)k * ld;
-  double a[NB];
+// Rows 8 w .. of L (lanes 0-7) and columns 8 w .. of U (lanes 8-15) of panel s, a row or column
+// per lane, one instruction stream for both: x_c /= U(c, c) (L only), x_j -= x_c U(c, j) or
+// x_j -= x_c L(j, c).
+__device__ __forceinline__ void diag64_rows(double* __restrict__ T, const double* __restrict__ Ub,
+                                            const double* __restrict__ Lb,
+                                            const double* __restrict__ rcp, int s, int w, int lane) {
+  if (lane >= 16) return;
+  const bool lower = lane < 8;
+  const double2* __restrict__ B = reinterpret_cast<const double2*>(lower ? Ub : Lb);
+  double* __restrict__ X =
+      lower ? T + s * 8 * kDiagSt + 8 * w + lane : T + (8 * w + lane - 8) * kDiagSt + s * 8;
+  const int sx = lower ? kDiagSt : 1;
+  double x[8];
 #pragma unroll
-  for (int j = 0; j < NB; ++j) a[j] = D[i + (int64_t)j * ld];
-  diag_rows_step<-1>(a, prow, i, pert[b], V.hasl + k, status, b, min(NB, V.nvalid - k));
+  for (int c = 0; c < 8; ++c) x[c] = X[c * sx];
 #pragma unroll
-  for (int j = 0; j < NB; ++j) D[i + (int64_t)j * ld] = a[j];
+  for (int c = 0; c < 8; ++c) {
+    double m[8];
+#pragma unroll
+    for (int j = c / 2; j < 4; ++j) {
+      const double2 v = B[c * 4 + j];
+      m[2 * j] = v.x;
+      m[2 * j + 1] = v.y;
+    }
+    const double q = quotient(x[c], Ub[c * 9], rcp[c]);
+    x[c] = lower ? q : x[c];
+#pragma unroll
+    for (int j = c + 1; j < 8; ++j) x[j] -= x[c] * m[j];
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) X[c * sx] = x[c];
 }
 
-__global__ void __launch_bounds__(64) k_dense_diag_rows(DenseView V, const double* __restrict__ pert,
-                                                        int32_t* status, int k) {
-  diag_rows_body(V, pert, status, k, blockIdx.x);
+// Tile (r, w) minus the rank-8 product of panel s, on the FP64 tensor cores.
+__device__ __forceinline__ void diag64_tile(double* __restrict__ T, int s, int r, int w, int g,
+                                            int t) {
+  double* __restrict__ C = T + (8 * w + 2 * t) * kDiagSt + 8 * r + g;
+  const double* __restrict__ A = T + (8 * s + t) * kDiagSt + 8 * r + g;
+  const double* __restrict__ B = T + (8 * w + g) * kDiagSt + 8 * s + t;
+  double c0 = C[0], c1 = C[kDiagSt];
+  dmma884(c0, c1, A[0], -B[0]);
+  dmma884(c0, c1, A[4 * kDiagSt], -B[4]);
+  C[0] = c0;
+  C[kDiagSt] = c1;
+}
+
+// LU without pivoting of the 64 x 64 block T (T[i + kDiagSt * j], shared memory, 16-byte aligned)
+// by 8 warps, in panels of 8 pivots: warp s factors the 8 x 8 block of panel s, then warp w > s
+// solves its 8 rows of L and 8 columns of U, then the trailing tiles take the rank-8 product (two
+// DMMA each).  Tile column w belongs to warp w, except that warp s + 1 updates only its diagonal
+// tile and goes on to factor it while the others are still updating (the rest of its column is
+// done by the warps of those rows).  So the chain through the block is, per panel, 8 pivots, 8
+// steps of the row solve, one tile and two barriers.
+// Every entry takes its updates pivot by pivot in increasing order; per pivot the reference's
+// column math (perturbation src/numeric.cu:139-140, L /= d src/numeric.cu:37-47, rank-1 update
+// src/numeric.cu:78-83).  Panels past nv are identity padding and are skipped.
+//
+// Bound by latency (64 dependent pivots: broadcast, reciprocal, quotient, update).
+// Measured, one block: 12.5 us (10 us of it the factorization) against 25-28 us of a thread per row
+// with all 64 pivot steps unrolled, which was bound by fetching its straight-line code; a warp per
+// 8 columns exchanging the pivot rows by shuffles took 18 us (twice the instructions on the chain).
+constexpr int kDiagSmem = 64 * kDiagSt + 2 * 64 + 8;   // doubles: T, Ub, Lb, rcp
+
+template <bool PERT>
+__device__ __forceinline__ void diag64_steps(double* T, double pv,
+                                             const uint8_t* __restrict__ hasl, int32_t* status,
+                                             int b, int np) {
+  const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
+  const int g = lane >> 2, t = lane & 3;
+  double* Ub = T + 64 * kDiagSt;
+  double* Lb = Ub + 64;
+  double* rcp = Lb + 64;
+  unsigned hm = 0;
+  if (PERT) hm = __ballot_sync(0xffffffffu, lane < 8 && hasl[warp * 8 + (lane & 7)] != 0);
+#pragma unroll 1
+  for (int s = 0; s < np; ++s) {
+    if (warp == s) diag64_block<PERT>(T, Ub, Lb, rcp, s, lane, pv, hm, status, b);
+    __syncthreads();
+    if (warp > s) {
+      diag64_rows(T, Ub, Lb, rcp, s, warp, lane);
+    } else if (warp == s) {                    // the block's factors back to T
+      for (int e = lane; e < 64; e += 32) {
+        const int i = e % 8, j = e / 8;
+        T[s * 8 * (kDiagSt + 1) + i + j * kDiagSt] = i > j ? Lb[j * 8 + i] : Ub[i * 8 + j];
+      }
+    }
+    __syncthreads();
+    if (warp == s + 1) {
+      diag64_tile(T, s, warp, warp, g, t);
+      __syncwarp();
+    } else if (warp > s) {
+      diag64_tile(T, s, warp, s + 1, g, t);
+#pragma unroll 2
+      for (int r = s + 1; r < 8; ++r) diag64_tile(T, s, r, warp, g, t);
+    }
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void diag64(double* T, double pv, const uint8_t* __restrict__ hasl,
+                                       int32_t* status, int b, int nv) {
+  const int np = min(8, (nv + 7) / 8);
+  if (pv > 0.0) diag64_steps<true>(T, pv, hasl, status, b, np);
+  else diag64_steps<false>(T, pv, hasl, status, b, np);
+  if (threadIdx.x < nv) {
+    const double d = T[threadIdx.x * (kDiagSt + 1)];
+    if (d == 0.0) atomicOr(status + b, GLU_INST_ZERO_PIVOT);
+    else if (!finite_bits(d)) atomicOr(status + b, GLU_INST_NAN_PIVOT);
+  }
+}
+
+// The diagonal block at pivot k of instance b (256 threads).
+__device__ __forceinline__ void diag64_body(const DenseView& V, const double* __restrict__ pert,
+                                            int32_t* status, int k, int b) {
+  extern __shared__ double sm[];
+  double* T = sm;
+  const int64_t ld = V.ld;
+  double* __restrict__ D = V.base + (int64_t)b * V.stride + (int64_t)k + (int64_t)k * ld;
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int e = threadIdx.x + q * 256;
+    T[e % 64 + (e / 64) * kDiagSt] = D[e % 64 + (int64_t)(e / 64) * ld];
+  }
+  __syncthreads();
+  diag64(T, pert[b], V.hasl + k, status, b, min(64, V.nvalid - k));
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int e = threadIdx.x + q * 256;
+    D[e % 64 + (int64_t)(e / 64) * ld] = T[e % 64 + (e / 64) * kDiagSt];
+  }
+}
+
+__global__ void __launch_bounds__(256) k_dense_diag64(DenseView V, const double* __restrict__ pert,
+                                                      int32_t* status, int k) {
+  diag64_body(V, pert, status, k, blockIdx.x);
 }
 
 // The dense view of front f's buffer (instances `fstride` doubles apart in F).
@@ -192,13 +335,13 @@ __device__ __forceinline__ DenseView front_view(const PlanDev& P, const FrontGeo
 }
 
 // Diagonal block at pivot k of every front f0 + blockIdx.y of a level (grid (count, fronts)) that
-// still has a pivot there; the same body as k_dense_diag_rows.
-__global__ void __launch_bounds__(64) k_front_diag(PlanDev P, double* F, int64_t fstride, int f0,
+// still has a pivot there; the same body as k_dense_diag64.
+__global__ void __launch_bounds__(256) k_front_diag(PlanDev P, double* F, int64_t fstride, int f0,
                                                   const double* __restrict__ pert,
                                                   int32_t* status, int k) {
   const FrontGeom g = P.fgeom[f0 + blockIdx.y];
   if (k >= g.w) return;
-  diag_rows_body(front_view(P, g, F, fstride), pert, status, k, blockIdx.x);
+  diag64_body(front_view(P, g, F, fstride), pert, status, k, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -333,12 +476,6 @@ __device__ __forceinline__ void cp_async_wait() {
 // -x by flipping the sign bit on the integer pipe (keeps the negation off the FP64 pipe)
 __device__ __forceinline__ double neg(double x) {
   return __hiloint2double(__double2hiint(x) ^ 0x80000000, __double2loint(x));
-}
-
-__device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
 }
 
 // The trailing update at pivot k of the fronts of a level, as GEMM problems: blockIdx.z =
@@ -928,7 +1065,7 @@ int sm_count() {
 void launch_dense_diag(const DenseView& V, int count, const double* pert, int32_t* status, int k,
                        int nb, cudaStream_t s, LaunchCounter& lc) {
   if (nb == 128) k_dense_diag<128><<<count, 256, 0, s>>>(V, pert, status, k);
-  else k_dense_diag_rows<<<count, 64, 0, s>>>(V, pert, status, k);
+  else k_dense_diag64<<<count, 256, kDiagSmem * 8, s>>>(V, pert, status, k);
   lc.n++;
 }
 
@@ -1107,7 +1244,7 @@ void launch_front_level(const PlanDev& P, const FrontLevel& L, double* vals, int
   ensure_smem_limit((const void*)k_gemm_sub<64, 64, 32, 32, 2, 16, true>, G::SMEM);
   for (size_t i = 0; i < L.mmax.size(); ++i) {
     const int k = 64 * (int)i;
-    k_front_diag<<<dim3(count, nf), 64, 0, s>>>(P, F, fstride, L.f0, pert, status, k);
+    k_front_diag<<<dim3(count, nf), 256, kDiagSmem * 8, s>>>(P, F, fstride, L.f0, pert, status, k);
     lc.n++;
     if (L.tiles1[i] > 0) {      // some front has rows below or columns right of this panel
       if ((int64_t)L.tiles4[i] * nfc >= 2 * sm_count())
