@@ -10,7 +10,10 @@
 //   k_dense_trsm_mma
 //                  L21 = A21 U11^-1 and U12 = L11^-1 A12: 8-column blocks updated by DMMA, 8 x 8
 //                  triangles solved one row per lane in the reference's order (k_dense_trsm, a
-//                  warp-shuffle recurrence, serves NB = 128).
+//                  warp-shuffle recurrence, serves NB = 128; k_dense_trsm8, 8 rows per warp,
+//                  grids that leave SMs idle).
+//   k_dense_step   few matrices: the update by one panel with the next diagonal block's
+//                  factorization in the CTA that holds it.
 //   k_gemm_sub / k_gemm_sub16
 //                  updates C -= A * B on the FP64 tensor cores (DMMA, mma.sync m8n8k4 or
 //                  m16n8k8): accumulators start from -C and collect +A*B, the result is stored
@@ -864,6 +867,234 @@ __global__ void __launch_bounds__(WARPS * 32) k_front_trsm(PlanDev P, double* F,
 }
 
 // ---------------------------------------------------------------------------------------------
+// Panel steps for few matrices: the chain of panels sets the time, not the rate of any kernel.
+// ---------------------------------------------------------------------------------------------
+
+// L21 / U12 of a panel step, 64 rows (or columns, as rows of U12^T) per CTA and 8 per warp: the
+// form of trsm_mma_body for grids that leave SMs idle.  A warp's chain is 8 triangles of 8 pivots
+// and the products between them on one 8-row tile, the tile and the diagonal block are fetched by
+// 256 threads, and no warp waits for another after that.
+// Bound by latency (64 dependent pivots a row).  Measured, one panel of 448 rows and columns: 8 us
+// against 13 us of one-warp CTAs of 32 rows.
+__device__ __forceinline__ void trsm8_body(const DenseView& V, int k, int mt, int tile, int b) {
+  constexpr int ST = 68;                      // == 4 (mod 16) doubles: conflict-free fragments
+  extern __shared__ double sm[];
+  double* T = sm;                             // diagonal block, T[i + j * ST]
+  double* X = sm + 64 * ST;                   // L21: X[c * ST + r]; U12: X[r * ST + c]
+  double* R = X + 64 * ST;                    // reciprocals of the pivots
+  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
+  const int g = lane >> 2, t = lane & 3;
+  const bool lower = tile < mt;
+  const int64_t ld = V.ld;
+  double* __restrict__ D = V.base + (int64_t)b * V.stride;
+  double* __restrict__ Xg = lower ? D + (int64_t)(k + 64 + tile * 64) + (int64_t)k * ld
+                                  : D + (int64_t)k + (int64_t)(k + 64 + (tile - mt) * 64) * ld;
+  for (int idx = tid; idx < 64 * 32; idx += 256) {
+    const int i = (idx % 32) * 2, j = idx / 32;
+    cp_async16(T + i + j * ST, D + (int64_t)(k + i) + (int64_t)(k + j) * ld, true);
+    cp_async16(X + i + j * ST, Xg + i + (int64_t)j * ld, true);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (lower) {
+    if (tid < 64) R[tid] = 1.0 / T[tid * (ST + 1)];
+    __syncthreads();
+  }
+  const int xr = lower ? 1 : ST, xc = lower ? ST : 1;   // X(r, c) = X[r * xr + c * xc]
+  const int sk = lower ? 1 : ST, sn = lower ? ST : 1;   // B operand: T(kk, n) = T[kk * sk + n * sn]
+  double* __restrict__ Xw = X + warp * 8 * xr;          // the warp's 8 rows
+  const int nblk = min(8, (V.nvalid - k + 7) / 8);      // blocks past it: padding, stay zero
+#pragma unroll 1
+  for (int blk = 0; blk < nblk; ++blk) {
+    const int c0 = blk * 8;
+    double tri[36];                           // the triangle, loaded ahead of its use
+#pragma unroll
+    for (int c = 0, q = 0; c < 8; ++c)
+#pragma unroll
+      for (int j = c; j < 8; ++j, ++q) tri[q] = T[(c0 + c) * sk + (c0 + j) * sn];
+    if (blk > 0) {
+      double* xp = Xw + g * xr + (c0 + 2 * t) * xc;
+      double a0 = neg(xp[0]), a1 = neg(xp[xc]);
+#pragma unroll 4
+      for (int kk = 0; kk < c0; kk += 4)
+        dmma884(a0, a1, Xw[g * xr + (kk + t) * xc], T[(kk + t) * sk + (c0 + g) * sn]);
+      xp[0] = neg(a0);
+      xp[xc] = neg(a1);
+      __syncwarp();
+    }
+    if (lane < 8) {
+      double x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = Xw[lane * xr + (c0 + j) * xc];
+#pragma unroll
+      for (int c = 0, q = 0; c < 8; ++c) {
+        if (lower) x[c] = quotient(x[c], tri[q], R[c0 + c]);
+        ++q;
+#pragma unroll
+        for (int j = c + 1; j < 8; ++j, ++q) x[j] -= x[c] * tri[q];
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) Xw[lane * xr + (c0 + j) * xc] = x[j];
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int idx = tid; idx < 64 * 64; idx += 256) {
+    const int i = idx % 64, j = idx / 64;
+    Xg[i + (int64_t)j * ld] = X[i + j * ST];
+  }
+}
+
+constexpr int kTrsm8Smem = (2 * 64 * 68 + 64) * 8;
+
+__global__ void __launch_bounds__(256) k_dense_trsm8(DenseView V, int k, int mt) {
+  trsm8_body(V, k, mt, blockIdx.x, blockIdx.y);
+}
+
+// The same at pivot k of the fronts of a level: grid (most tiles of a front, fronts * count).
+__global__ void __launch_bounds__(256) k_front_trsm8(PlanDev P, double* F, int64_t fstride, int f0,
+                                                     int count, int k) {
+  const FrontGeom g = P.fgeom[f0 + blockIdx.y / count];
+  if (k >= g.w) return;
+  const int mt = (g.ld - k - 64) / 64, nt = (g.cols - k - 64) / 64;
+  if ((int)blockIdx.x >= mt + nt) return;
+  trsm8_body(front_view(P, g, F, fstride), k, mt, blockIdx.x, blockIdx.y % count);
+}
+
+// One 64 x 64 tile of the update by panel k (the rank-64 product of its L21 and U12), and, in the
+// CTA of the tile holding the next panel's diagonal block, that block's factorization in shared
+// memory (diag64): the serial 64 pivots run beside the other tiles of the update instead of in
+// a launch of their own.  Tile idx of the region: its first `wide` tile columns and tile rows of
+// the trailing block (everything when wide covers it), enumerated columns first.
+// Accumulators start from -C and collect +A*B as in k_gemm_sub, same sums in the same order.
+// Bound by the diagonal block's latency: 14 us with it and 4.4 us without on a 448 x 448 block, where
+// the launches it stands for took 26 (diagonal block) + 2 x 24 us (in-group products of up to 7
+// panels); n = 4,960 refactorization, panels and products: 1.27 -> 0.59 ms.
+__device__ __forceinline__ void step_body(const DenseView& V, const double* __restrict__ pert,
+                                          int32_t* status, int k, int wide, int idx, int b) {
+  constexpr int ST = 68;
+  extern __shared__ double sm[];
+  double* As = sm;                            // As[kk * ST + m]
+  double* Bs = sm + 64 * ST;                  // Bs[n * ST + kk]
+  const int mt = (V.rows - k - 64) / 64, nt = (V.cols - k - 64) / 64;
+  const int gc = min(wide, nt), gr = min(wide, mt);
+  int ti, tj;
+  if (idx < gc * mt) {
+    ti = idx % mt;
+    tj = idx / mt;
+  } else {
+    idx -= gc * mt;
+    if (gr == 0 || idx >= gr * (nt - gc)) return;
+    ti = idx % gr;
+    tj = gc + idx / gr;
+  }
+  const int kv = min(64, V.nvalid - k);
+  if (kv <= 0) return;
+  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
+  const int64_t ld = V.ld;
+  double* __restrict__ D = V.base + (int64_t)b * V.stride;
+  const int m0 = k + 64 + ti * 64, n0 = k + 64 + tj * 64;
+  const double* __restrict__ A = D + m0 + (int64_t)k * ld;
+  const double* __restrict__ B = D + k + (int64_t)n0 * ld;
+  double* __restrict__ C = D + m0 + (int64_t)n0 * ld;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {               // 16 pivots per copy group
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = tid + h * 256;
+      cp_async16(As + (q * 16 + e / 32) * ST + (e % 32) * 2,
+                 A + (e % 32) * 2 + (int64_t)(q * 16 + e / 32) * ld, true);
+      cp_async16(Bs + (e / 8) * ST + q * 16 + (e % 8) * 2,
+                 B + q * 16 + (e % 8) * 2 + (int64_t)(e / 8) * ld, true);
+    }
+    cp_async_commit();
+  }
+  const int wm = (warp % 2) * 32 + (lane >> 2), wn = (warp / 2) * 16;
+  double acc[4][2][2];
+#pragma unroll
+  for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        acc[mi][ni][e] =
+            neg(C[(wm + mi * 8) + (int64_t)(wn + ni * 8 + (lane & 3) * 2 + e) * ld]);
+  auto steps = [&](int q) {
+#pragma unroll
+    for (int k4 = 0; k4 < 4; ++k4) {
+      const int kk = q * 16 + k4 * 4 + (lane & 3);
+      double a[4], bf[2];
+#pragma unroll
+      for (int mi = 0; mi < 4; ++mi) a[mi] = As[kk * ST + wm + mi * 8];
+#pragma unroll
+      for (int ni = 0; ni < 2; ++ni) bf[ni] = Bs[(wn + ni * 8 + (lane >> 2)) * ST + kk];
+#pragma unroll
+      for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int ni = 0; ni < 2; ++ni) dmma884(acc[mi][ni][0], acc[mi][ni][1], a[mi], bf[ni]);
+    }
+  };
+  cp_async_wait<3>();
+  __syncthreads();
+  steps(0);
+  cp_async_wait<2>();
+  __syncthreads();
+  if (kv > 16) steps(1);
+  cp_async_wait<1>();
+  __syncthreads();
+  if (kv > 32) steps(2);
+  cp_async_wait<0>();
+  __syncthreads();
+  if (kv > 48) steps(3);
+  if (ti > 0 || tj > 0 || k + 64 >= V.nvalid) {
+#pragma unroll
+    for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+      for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          C[(wm + mi * 8) + (int64_t)(wn + ni * 8 + (lane & 3) * 2 + e) * ld] =
+              neg(acc[mi][ni][e]);
+    return;
+  }
+  // the next panel's diagonal block, in shared memory
+  __syncthreads();                            // every warp is done with As and Bs
+#pragma unroll
+  for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+    for (int ni = 0; ni < 2; ++ni)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        As[(wn + ni * 8 + (lane & 3) * 2 + e) * ST + wm + mi * 8] = neg(acc[mi][ni][e]);
+  __syncthreads();
+  diag64(As, pert[b], V.hasl + k + 64, status, b, min(64, V.nvalid - k - 64));
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int e = tid + q * 256;
+    C[e % 64 + (int64_t)(e / 64) * ld] = As[e % 64 + (e / 64) * ST];
+  }
+}
+
+constexpr int kStepSmem = 2 * 64 * 68 * 8;
+
+__global__ void __launch_bounds__(256) k_dense_step(DenseView V, const double* __restrict__ pert,
+                                                    int32_t* status, int k, int wide) {
+  step_body(V, pert, status, k, wide, blockIdx.x, blockIdx.y);
+}
+
+// The same at pivot k of the fronts of a level, the whole trailing block of each: grid (most
+// tiles of a front, fronts * count).
+__global__ void __launch_bounds__(256) k_front_step(PlanDev P, double* F, int64_t fstride, int f0,
+                                                    int count, const double* __restrict__ pert,
+                                                    int32_t* status, int k) {
+  const FrontGeom g = P.fgeom[f0 + blockIdx.y / count];
+  if (k >= g.w) return;
+  step_body(front_view(P, g, F, fstride), pert, status, k, 1 << 20, blockIdx.x,
+            blockIdx.y % count);
+}
+
+// ---------------------------------------------------------------------------------------------
 // sparse-to-dense contributions
 // ---------------------------------------------------------------------------------------------
 __global__ void k_gather(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
@@ -1079,17 +1310,16 @@ void launch_dense_trsm(const DenseView& V, int count, int k, int nb, cudaStream_
     ensure_smem_limit((const void*)k_dense_trsm<128>, smem);
     k_dense_trsm<128><<<dim3(nrb + ncb, count), 256, smem, s>>>(V, k, nrb);
   } else {
-    // 128 rows per CTA (4 warps sharing the staged diagonal block), or 32 when that leaves
-    // fewer than two CTAs per SM (one instance, short panels)
-    constexpr int smem4 = (64 * 68 + 4 * 64 * 36 + 64) * 8, smem1 = (64 * 68 + 64 * 36 + 64) * 8;
-    ensure_smem_limit((const void*)k_dense_trsm_mma<64, 4>, smem4);
-    ensure_smem_limit((const void*)k_dense_trsm_mma<64, 1>, smem1);
+    // 128 rows per CTA (4 warps sharing the staged diagonal block), or the 64-row CTAs of the panel
+    // steps when that leaves fewer than two CTAs per SM (short panels)
+    constexpr int smem4 = (64 * 68 + 4 * 64 * 36 + 64) * 8;
     const int nrt = (V.rows - k - nb + 127) / 128, nct = (V.cols - k - nb + 127) / 128;
     if ((int64_t)(nrt + nct) * count >= 2 * sm_count()) {
+      ensure_smem_limit((const void*)k_dense_trsm_mma<64, 4>, smem4);
       k_dense_trsm_mma<64, 4><<<dim3(nrt + nct, count), 128, smem4, s>>>(V, k, nrt);
     } else {
-      const int nr1 = (V.rows - k - nb + 31) / 32, nc1 = (V.cols - k - nb + 31) / 32;
-      k_dense_trsm_mma<64, 1><<<dim3(nr1 + nc1, count), 32, smem1, s>>>(V, k, nr1);
+      ensure_smem_limit((const void*)k_dense_trsm8, kTrsm8Smem);
+      k_dense_trsm8<<<dim3(nrb + ncb, count), 256, kTrsm8Smem, s>>>(V, k, nrb);
     }
   }
   lc.n++;
@@ -1108,6 +1338,23 @@ void launch_dense_update(const DenseView& V, int count, int k, int nb, int varia
                   V.stride, s, lc, variant);
 }
 
+// Whether blocks of `rows` rows, `count` of them, take the panel steps for few matrices: their
+// chain of launches is then shorter (2 per panel instead of 4, the diagonal block beside the
+// update), while with more row tiles the grids are deep and the kernels made for rate win.
+// Measured, panels + in-group products, steps against the others: n = 4,960 0.59 / 1.27 ms (18 row
+// tiles), 8 x n = 20,000 5.8 / 7.4 ms (552), 256 x n = 2,000 1.14 / 1.14 ms (1,792),
+// 64 x n = 20,000 34.3 / 29.6 ms (4,416).
+bool few_matrices(int64_t rows, int64_t count) { return rows / 64 * count <= 1200; }
+
+// Whether each step then updates the whole trailing block instead of the rest of its group of
+// panels (with one product of all the group's pivots for the rest): fewer launches while a block's
+// tiles are few, but C is read and written once per panel.  Measured: n = 4,960 (324 tiles)
+// 0.59 / 0.66 ms, n = 20,000 (4,761) 4.08 / 4.20 ms, 16 x n = 4,960 (5,184) 1.27 / 1.28 ms,
+// 8 x n = 20,000 (38,088) 21.2 / 18.1 ms.
+bool step_whole_block(int64_t rows, int64_t cols, int64_t count) {
+  return (rows / 64) * (cols / 64) * count <= 5000;
+}
+
 // Right-looking LU of the first npiv pivots of a batch of dense blocks, in groups of `depth`
 // panels: inside a group each panel first takes the updates of the group's earlier panels on
 // its own column block and row block (two thin DMMA products), then is factored (diagonal block,
@@ -1119,6 +1366,43 @@ void launch_dense_update(const DenseView& V, int count, int k, int nb, int varia
 void launch_dense_factor(const DenseView& V, int count, const double* pert, int32_t* status,
                          int npiv, int nb, int depth, int variant, cudaStream_t s,
                          LaunchCounter& lc, const std::function<void(int, int64_t)>& mark) {
+  if (nb == 64 && few_matrices(V.rows, count)) {
+    // the panel chain sets the time: per panel one launch for L21 / U12 and one for the update of
+    // the group's later panels together with the next diagonal block
+    ensure_smem_limit((const void*)k_dense_trsm8, kTrsm8Smem);
+    ensure_smem_limit((const void*)k_dense_step, kStepSmem);
+    const int np = (std::min(npiv, V.nvalid) + 63) / 64;
+    const int group = step_whole_block(V.rows, V.cols, count) ? np : depth;
+    for (int p0 = 0; p0 < np; p0 += group) {
+      const int dd = std::min(group, np - p0);
+      for (int j = 0; j < dd; ++j) {
+        const int c = (p0 + j) * 64;
+        const int mt = (V.rows - c) / 64 - 1, nt = (V.cols - c) / 64 - 1;
+        int64_t c0 = lc.n;
+        if (j == 0) launch_dense_diag(V, count, pert, status, c, nb, s, lc);
+        if (mt + nt > 0) {
+          k_dense_trsm8<<<dim3(mt + nt, count), 256, kTrsm8Smem, s>>>(V, c, mt);
+          lc.n++;
+        }
+        mark(2, c0);
+        c0 = lc.n;
+        const int wide = group == np ? 1 << 20 : dd - 1 - j;
+        const int gc = std::min(wide, nt), gr = std::min(wide, mt);
+        const int tiles = gc * mt + gr * (nt - gc);
+        if (tiles > 0) {
+          k_dense_step<<<dim3(tiles, count), 256, kStepSmem, s>>>(V, pert, status, c, wide);
+          lc.n++;
+          mark(6, c0);
+        }
+      }
+      if (group < np) {
+        const int64_t c0 = lc.n;
+        launch_dense_update(V, count, p0 * 64, dd * 64, variant, s, lc);
+        mark(3, c0);
+      }
+    }
+    return;
+  }
   double* D = V.base;
   const int64_t ld = V.ld;
   for (int k0 = 0; k0 < npiv; k0 += depth * nb) {
@@ -1237,20 +1521,42 @@ void launch_front_level(const PlanDev& P, const FrontLevel& L, double* vals, int
   lc.n += 2;
   // 2. their pivots, 64 at a time: diagonal blocks, L21 / U12, trailing update (the same kernels'
   //    bodies as the trailing block's, every front of the level in one launch per stage)
-  constexpr int smem4 = (64 * 68 + 4 * 64 * 36 + 64) * 8, smem1 = (64 * 68 + 64 * 36 + 64) * 8;
+  constexpr int smem4 = (64 * 68 + 4 * 64 * 36 + 64) * 8;
+  // half the L21 + U12 tiles of the largest front stand for its row tiles
+  const bool few = !L.tiles1.empty() && few_matrices(16 * (int64_t)L.tiles1[0], nfc);
+  ensure_smem_limit((const void*)k_front_trsm8, kTrsm8Smem);
+  ensure_smem_limit((const void*)k_front_step, kStepSmem);
   ensure_smem_limit((const void*)k_front_trsm<4>, smem4);
-  ensure_smem_limit((const void*)k_front_trsm<1>, smem1);
   using G = Gemm<64, 64, 32, 32, 2, 16>;
   ensure_smem_limit((const void*)k_gemm_sub<64, 64, 32, 32, 2, 16, true>, G::SMEM);
   for (size_t i = 0; i < L.mmax.size(); ++i) {
     const int k = 64 * (int)i;
+    if (few) {
+      // one launch for L21 / U12 and one for the update with the next diagonal blocks
+      if (i == 0) {
+        k_front_diag<<<dim3(count, nf), 256, kDiagSmem * 8, s>>>(P, F, fstride, L.f0, pert, status, k);
+        lc.n++;
+      }
+      if (L.tiles1[i] > 0) {
+        k_front_trsm8<<<dim3(L.tiles1[i] / 2, nfc), 256, kTrsm8Smem, s>>>(P, F, fstride, L.f0,
+                                                                        count, k);
+        lc.n++;
+      }
+      if (L.mmax[i] > 0 && L.nmax[i] > 0) {
+        k_front_step<<<dim3((L.mmax[i] / 64) * (L.nmax[i] / 64), nfc), 256, kStepSmem, s>>>(
+            P, F, fstride, L.f0, count, pert, status, k);
+        lc.n++;
+      }
+      continue;
+    }
     k_front_diag<<<dim3(count, nf), 256, kDiagSmem * 8, s>>>(P, F, fstride, L.f0, pert, status, k);
     lc.n++;
     if (L.tiles1[i] > 0) {      // some front has rows below or columns right of this panel
       if ((int64_t)L.tiles4[i] * nfc >= 2 * sm_count())
         k_front_trsm<4><<<dim3(L.tiles4[i], nfc), 128, smem4, s>>>(P, F, fstride, L.f0, count, k);
       else
-        k_front_trsm<1><<<dim3(L.tiles1[i], nfc), 32, smem1, s>>>(P, F, fstride, L.f0, count, k);
+        k_front_trsm8<<<dim3(L.tiles1[i] / 2, nfc), 256, kTrsm8Smem, s>>>(P, F, fstride, L.f0,
+                                                                        count, k);
       lc.n++;
     }
     if (L.mmax[i] > 0 && L.nmax[i] > 0) {
