@@ -125,6 +125,8 @@ struct glu_batch_s {
   int64_t r_vectors = 0;
   int64_t ylen = 0;
   int64_t y_vectors = 0;
+  double* xbuf = nullptr;       // solved values of the dense block (2 ntp per vector; trsv.cu),
+                                // then the solve's failure word
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaStream_t own_stream = nullptr;
@@ -145,7 +147,7 @@ struct glu_batch_s {
   unsigned* pbar = nullptr;     // pgroups barrier counters, then the failure word
   int pgroups = 0;
   int pextra = 0;               // test hook: arrivals added to every barrier target
-  double pwait_ms = 1000.0;
+  double pwait_ms = 1000.0;     // bound of every wait of the cooperative launches
 };
 
 namespace {
@@ -165,9 +167,13 @@ int ensure_workspace(glu_batch_t b, int64_t vectors, cudaStream_t s) {
     return set_error(GLU_NOT_READY, "solve workspace must be allocated before stream capture "
                      "(run one solve with the same nrhs first)");
   if (b->y) cudaFree(b->y);
+  if (b->xbuf) cudaFree(b->xbuf);
   b->y = nullptr;
+  b->xbuf = nullptr;
   b->y_vectors = 0;
-  if (cudaMalloc(&b->y, sizeof(double) * b->ylen * vectors) != cudaSuccess) {
+  if (cudaMalloc(&b->y, sizeof(double) * b->ylen * vectors) != cudaSuccess ||
+      cudaMalloc(&b->xbuf, sizeof(double) * (2 * (size_t)b->plan->P.ntp * vectors + 1)) !=
+          cudaSuccess) {
     cudaGetLastError();
     return set_error(GLU_MEMORY_OVERFLOW, "solve workspace allocation failed");
   }
@@ -342,7 +348,12 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
   double* y = b->y;
   const int64_t yl = b->ylen;
   const int cnt = b->count;
-  glu::launch_solve_permute_in(P, cnt, nrhs, B, y, yl, transpose, s, lc);
+  int* serr = reinterpret_cast<int*>(b->xbuf + 2 * (int64_t)P.ntp * b->y_vectors);
+  glu::launch_solve_permute_in(P, cnt, nrhs, B, y, yl, transpose, b->xbuf, serr, s, lc);
+  auto dense = [&] {
+    glu::launch_dense_solve(P, b->vals, cnt, nrhs, y, yl, transpose != 0, b->xbuf, serr, b->status,
+                            b->pwait_ms, s, lc);
+  };
   const int nl = (int)hp.lptr.size() - 1, nu = (int)hp.uptr.size() - 1;
   // one solve level: its single columns, then its fronts (independent of each other)
   auto lvl = [&](bool L, int l, int which) {
@@ -372,22 +383,19 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
                              hp.lptr[l + 1] - hp.lptr[l], 0, s, lc);
     if (P.nt > 0)    // rows of the dense block take their L21 part (columns < t)
       glu::launch_rows_solve(P, b->vals, cnt, nrhs, y, yl, nullptr, (int)P.t, (int)P.nt, 0, s, lc);
-    glu::launch_dense_trsv(P, b->vals, cnt, nrhs, y, yl, 0, s, lc);
-    glu::launch_dense_trsv(P, b->vals, cnt, nrhs, y, yl, 1, s, lc);
+    dense();
     for (int l = 0; l < nu; ++l)    // U rows, the border U(r < t, j >= t) included
       glu::launch_rows_solve(P, b->vals, cnt, nrhs, y, yl, pl->d_ucols, hp.uptr[l],
                              hp.uptr[l + 1] - hp.uptr[l], 1, s, lc);
   } else if (!transpose) {
     for (int l = 0; l < nl; ++l) lvl(true, l, 0);
-    glu::launch_dense_trsv(P, b->vals, cnt, nrhs, y, yl, 0, s, lc);
-    glu::launch_dense_trsv(P, b->vals, cnt, nrhs, y, yl, 1, s, lc);
+    dense();
     glu::launch_border(P, b->vals, cnt, nrhs, y, yl, 0, s, lc);
     for (int l = 0; l < nu; ++l) lvl(false, l, 1);
   } else {
     for (int l = nu - 1; l >= 0; --l) lvl(false, l, 2);
     glu::launch_border(P, b->vals, cnt, nrhs, y, yl, 1, s, lc);
-    glu::launch_dense_trsv(P, b->vals, cnt, nrhs, y, yl, 2, s, lc);
-    glu::launch_dense_trsv(P, b->vals, cnt, nrhs, y, yl, 3, s, lc);
+    dense();
     for (int l = nl - 1; l >= 0; --l) lvl(true, l, 3);
   }
   glu::launch_solve_permute_out(P, cnt, nrhs, y, X, yl, transpose, s, lc);
@@ -1013,6 +1021,7 @@ int glu_batch_destroy(glu_batch_t b) {
   if (b->status) cudaFree(b->status);
   if (b->asm_flag) cudaFree(b->asm_flag);
   if (b->y) cudaFree(b->y);
+  if (b->xbuf) cudaFree(b->xbuf);
   if (b->gbuf) cudaFree(b->gbuf);
   if (b->fbuf) cudaFree(b->fbuf);
   if (b->rbuf) cudaFree(b->rbuf);

@@ -23,6 +23,7 @@
 #include "glu_b200.h"
 #include "kernels.cuh"
 #include "residual.cuh"
+#include "wait.cuh"
 
 namespace glu {
 
@@ -300,18 +301,6 @@ __global__ void __launch_bounds__(256) k_sparse_pull(PlanDev P, double* vals, in
 // sparse phase: a run of consecutive levels in ONE cooperative launch
 // ---------------------------------------------------------------------------------------------
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
 // Barrier among the CTAs of one group: every CTA adds one arrival to the group's counter and
 // waits until it reaches `target`.  The wait is bounded: after `budget_ns` of waiting, or as soon
 // as another CTA has reported a failure in *err, it gives up, records the failure in *err and
@@ -434,9 +423,14 @@ __global__ void __launch_bounds__(256) k_sparse_persistent(PlanDev P, double* va
 // solves
 // ---------------------------------------------------------------------------------------------
 
+// Also marks the vector's values of the dense solve unsolved and clears its failure word.
 __global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm, double* y,
-                             int64_t ylen, int transpose) {
+                             int64_t ylen, int transpose, double* xbuf, int* err) {
   const int64_t v = blockIdx.y;                 // instance * nrhs + rhs
+  if (blockIdx.x == 0 && v == 0 && threadIdx.x == 0) *err = 0;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 2 * (int64_t)P.ntp;
+       k += (int64_t)gridDim.x * blockDim.x)
+    xbuf[v * 2 * P.ntp + k] = __longlong_as_double(kUnsolved);
   const double* bv = Bm + v * P.n;
   double* yv = y + v * ylen;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < ylen;
@@ -760,25 +754,9 @@ __global__ void k_border_chunks(PlanDev P, const double* vals, int nrhs, double*
     atomicAdd(yv + P.bord_row[e], -(V[P.bord_slot[e]] * xj));
 }
 
-// Copies the 64 x 64 diagonal block at (kb, kb) of a column-major matrix into shared memory
-// (Ds[i + 64 j]) with 16-byte asynchronous copies, all in flight at once; the caller waits with
-// cp.async.wait_group and a barrier.  kb, ld and the instance offsets are even, so every copied
-// row pair is 16-byte aligned.
-__device__ __forceinline__ void stage_diag_block(const double* __restrict__ D, int64_t ld, int kb,
-                                                 double* Ds, int tid, int nthreads) {
-  for (int idx = tid; idx < 64 * 32; idx += nthreads) {
-    const int i = (idx % 32) * 2, j = idx / 32;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(Ds + i + j * 64);
-    const double* src = D + (int64_t)(kb + i) + (int64_t)(kb + j) * ld;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
-  }
-  asm volatile("cp.async.commit_group;\n" ::);
-}
-__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group 0;\n" ::); }
-
-// The 64x64 diagonal block of a dense triangular solve, by one warp in registers (rows lane and
-// lane + 32), the block read from shared memory (Ds[i + 64 j], see stage_diag_block).
-// which: 0 = L (unit lower, forward), 1 = U (backward), 2 = U^T (forward), 3 = L^T (backward).
+// The 64x64 triangle of a front's push solve, by one warp in registers (rows lane and lane + 32),
+// the block read from shared memory (Ds[i + 64 j]).  which: 0 = L (unit lower, forward), 1 = U
+// (backward).
 // yb[0 .. 64) must already hold every contribution from outside the block.
 __device__ __forceinline__ void dense_block_solve(int which, const double* __restrict__ Ds,
                                                   double* yb, int lane, double* xs) {
@@ -791,7 +769,7 @@ __device__ __forceinline__ void dense_block_solve(int which, const double* __res
       if (lane > i) r0 -= col[lane] * xi;
       if (lane + 32 > i) r1 -= col[lane + 32] * xi;
     }
-  } else if (which == 1) {
+  } else {
     for (int i = TB - 1; i >= 0; --i) {
       const double* col = Ds + i * TB;
       if (lane == (i & 31)) {
@@ -800,31 +778,6 @@ __device__ __forceinline__ void dense_block_solve(int which, const double* __res
       const double xi = __shfl_sync(0xffffffffu, i < 32 ? r0 : r1, i & 31);
       if (lane < i) r0 -= col[lane] * xi;
       if (lane + 32 < i) r1 -= col[lane + 32] * xi;
-    }
-  } else if (which == 2) {
-    // w_j = (w_j - sum_{kb <= i < j} U(i,j) w_i) / U(j,j), forward
-    for (int j = 0; j < TB; ++j) {
-      const double* col = Ds + j * TB;
-      double s = 0.0;
-      const double w0 = r0, w1 = r1;
-      if (lane < j) s += col[lane] * w0;
-      if (lane + 32 < j) s += col[lane + 32] * w1;
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == (j & 31)) {
-        if (j < 32) r0 = (r0 - s) / col[j]; else r1 = (r1 - s) / col[j];
-      }
-    }
-  } else {
-    // w_j = w_j - sum_{j < i < kb+64} L(i,j) w_i, backward
-    for (int j = TB - 1; j >= 0; --j) {
-      const double* col = Ds + j * TB;
-      double s = 0.0;
-      if (lane > j) s += col[lane] * r0;
-      if (lane + 32 > j) s += col[lane + 32] * r1;
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == (j & 31)) {
-        if (j < 32) r0 -= s; else r1 -= s;
-      }
     }
   }
   yb[lane] = r0;
@@ -1080,148 +1033,6 @@ __global__ void __launch_bounds__(256) k_front_solve_tail(PlanDev P, const doubl
   }
 }
 
-// Dense triangular solves on the ntp x ntp block, one CTA (256 threads) per vector, in 64-row
-// blocks: the 64x64 diagonal block is solved by warp 0 in registers (rows lane, lane+32), the
-// rest of the block column/row is applied by all threads with coalesced column reads.  Used when
-// the batch has enough vectors to fill the GPU.
-// which: 0 = L (unit lower, forward), 1 = U (backward), 2 = U^T (forward), 3 = L^T (backward)
-__global__ void __launch_bounds__(256) k_dense_trsv(PlanDev P, const double* vals, int nrhs,
-                                                    double* y, int64_t ylen, int which) {
-  constexpr int TB = 64;
-  __shared__ double xs[TB];
-  __shared__ __align__(16) double Ds[TB * TB];
-  const int64_t v = blockIdx.x;
-  const double* __restrict__ D = vals + (v / nrhs) * P.blob + P.dbase;
-  double* yd = y + v * ylen + P.t;
-  const int64_t ld = P.ntp;
-  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
-  const int nblk = (int)(P.ntp / TB);
-  for (int bi = 0; bi < nblk; ++bi) {
-    const int kb = (which == 0 || which == 2) ? bi * TB : (nblk - 1 - bi) * TB;
-    stage_diag_block(D, ld, kb, Ds, tid, blockDim.x);
-    if (which >= 2) {
-      // pull the already-solved part into the block: w_j -= sum_i M(i, j) w_i
-      for (int jj = warp; jj < TB; jj += 8) {
-        const int j = kb + jj;
-        double s = 0.0;
-        if (which == 2) {
-          for (int i = lane; i < kb; i += kWarp) s += D[i + (int64_t)j * ld] * yd[i];
-        } else {
-          for (int i = kb + TB + lane; i < (int)P.ntp; i += kWarp) s += D[i + (int64_t)j * ld] * yd[i];
-        }
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) yd[j] -= s;
-      }
-      __syncthreads();
-    }
-    stage_wait();
-    __syncthreads();
-    if (warp == 0) dense_block_solve(which, Ds, yd + kb, lane, xs);
-    __syncthreads();
-    if (which == 0) {          // rows below the block: y_r -= L(r, blk) x_blk
-      for (int r = kb + TB + tid; r < (int)P.ntp; r += blockDim.x) {
-        double s = 0.0;
-#pragma unroll 8
-        for (int i = 0; i < TB; ++i) s += D[r + (int64_t)(kb + i) * ld] * xs[i];
-        yd[r] -= s;
-      }
-    } else if (which == 1) {   // rows above the block: y_r -= U(r, blk) x_blk
-      for (int r = tid; r < kb; r += blockDim.x) {
-        double s = 0.0;
-#pragma unroll 8
-        for (int i = 0; i < TB; ++i) s += D[r + (int64_t)(kb + i) * ld] * xs[i];
-        yd[r] -= s;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// Blocked variant for few vectors (one matrix, few right-hand sides): per 64-block, one launch
-// solves the diagonal block of every vector (a warp each), one launch pushes the solved block
-// into the rest of the vector with many CTAs, so the triangle is read once at full bandwidth.
-// Grid (instances, ceil(nrhs / 8)): the CTA stages its instance's diagonal block once and each
-// warp solves one right-hand side.
-__global__ void __launch_bounds__(256) k_trsv_blk_diag(PlanDev P, const double* vals, int nrhs,
-                                                       double* y, int64_t ylen, int which, int kb) {
-  __shared__ __align__(16) double Ds[64 * 64];
-  const int64_t inst = blockIdx.x;
-  const int k = blockIdx.y * 8 + threadIdx.x / kWarp;
-  stage_diag_block(vals + inst * P.blob + P.dbase, P.ntp, kb, Ds, threadIdx.x, blockDim.x);
-  stage_wait();
-  __syncthreads();
-  if (k >= nrhs) return;
-  dense_block_solve(which, Ds, y + (inst * nrhs + k) * ylen + P.t + kb, threadIdx.x % kWarp,
-                    nullptr);
-}
-
-// Push of a solved block kb: which 0/1 update rows (y_r -= M(r, blk) x_blk), which 2/3 update
-// columns (w_j -= sum_i M(i, j) w_i over the block's rows); rows/columns [lo, hi); grid
-// (chunks of 32, instances), 256 threads.  Vectors of one instance are processed 8 at a time
-// from shared memory, so each matrix element is loaded once per 8 right-hand sides.  Rows: each
-// of the 32 rows of a CTA is summed by 8 threads over 8 columns each (coalesced column reads),
-// partial sums reduced in shared memory in a fixed order; columns: a warp per column of M reads
-// the block's 64 rows of it (coalesced) and reduces with shuffles.
-__global__ void __launch_bounds__(256) k_trsv_blk_update(PlanDev P, const double* vals, int nrhs,
-                                                         double* y, int64_t ylen, int which,
-                                                         int kb, int lo, int hi) {
-  constexpr int TB = 64, VC = 8, RW = 32;
-  __shared__ double xs[VC][TB];
-  __shared__ double part[8][VC][RW];
-  const int64_t inst = blockIdx.y;
-  const double* __restrict__ D = vals + inst * P.blob + P.dbase;
-  const int64_t ld = P.ntp;
-  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
-  for (int vc = 0; vc < nrhs; vc += VC) {
-    const int nv = nrhs - vc < VC ? nrhs - vc : VC;
-    __syncthreads();
-    for (int idx = tid; idx < VC * TB; idx += blockDim.x) {
-      const int v = idx / TB, i = idx % TB;
-      xs[v][i] = v < nv ? y[(inst * nrhs + vc + v) * ylen + P.t + kb + i] : 0.0;
-    }
-    __syncthreads();
-    if (which < 2) {
-      const int r = lo + blockIdx.x * RW + lane, g = warp;   // row, column group of 8
-      double acc[VC];
-#pragma unroll
-      for (int v = 0; v < VC; ++v) acc[v] = 0.0;
-      if (r < hi) {
-#pragma unroll
-        for (int ii = 0; ii < 8; ++ii) {
-          const int i = g * 8 + ii;
-          const double m = D[r + (int64_t)(kb + i) * ld];
-#pragma unroll
-          for (int v = 0; v < VC; ++v) acc[v] += m * xs[v][i];
-        }
-      }
-#pragma unroll
-      for (int v = 0; v < VC; ++v) part[g][v][lane] = acc[v];
-      __syncthreads();
-      if (tid < VC * RW) {
-        const int v = tid / RW, rr = tid % RW, row = lo + blockIdx.x * RW + rr;
-        if (v < nv && row < hi) {
-          double sum = 0.0;
-#pragma unroll
-          for (int gg = 0; gg < 8; ++gg) sum += part[gg][v][rr];
-          y[(inst * nrhs + vc + v) * ylen + P.t + row] -= sum;
-        }
-      }
-    } else {
-      for (int jj = warp; jj < RW; jj += 8) {
-        const int r = lo + blockIdx.x * RW + jj;
-        if (r >= hi) break;
-        const double* colp = D + (int64_t)r * ld + kb;
-        const double m0 = colp[lane], m1 = colp[lane + 32];
-        for (int v = 0; v < nv; ++v) {
-          double sum = m0 * xs[v][lane] + m1 * xs[v][lane + 32];
-          for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-          if (lane == 0) y[(inst * nrhs + vc + v) * ylen + P.t + r] -= sum;
-        }
-      }
-    }
-  }
-}
-
 __global__ void k_grad(PlanDev P, int nrhs, const double* __restrict__ lambda,
                        const double* __restrict__ x, double* __restrict__ ga) {
   const int64_t b = blockIdx.y;
@@ -1420,9 +1231,10 @@ void launch_sparse_persistent(const PlanDev& P, double* vals, int count, const d
 }
 
 void launch_solve_permute_in(const PlanDev& P, int count, int nrhs, const double* B, double* y,
-                             int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc) {
+                             int64_t ylen, int transpose, double* xbuf, int* err, cudaStream_t s,
+                             LaunchCounter& lc) {
   k_permute_in<<<dim3(grid1(ylen, 256, 256), count * nrhs), 256, 0, s>>>(P, nrhs, B, y, ylen,
-                                                                        transpose);
+                                                                        transpose, xbuf, err);
   lc.n++;
 }
 
@@ -1514,29 +1326,6 @@ void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, do
   else
     k_border<<<dim3((P.nt + 7) / 8, count * nrhs), 256, 0, s>>>(P, vals, nrhs, y, ylen, transpose);
   lc.n++;
-}
-
-void launch_dense_trsv(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                       int64_t ylen, int which, cudaStream_t s, LaunchCounter& lc) {
-  if (P.ntp == 0) return;
-  const int64_t nvec = (int64_t)count * nrhs;
-  if (nvec >= 256 || P.ntp < 1024) {       // enough vectors to fill the GPU: one CTA each
-    k_dense_trsv<<<(unsigned)nvec, 256, 0, s>>>(P, vals, nrhs, y, ylen, which);
-    lc.n++;
-    return;
-  }
-  const int nblk = (int)(P.ntp / 64);
-  for (int bi = 0; bi < nblk; ++bi) {
-    const int kb = (which == 0 || which == 2) ? bi * 64 : (nblk - 1 - bi) * 64;
-    k_trsv_blk_diag<<<dim3((unsigned)count, (unsigned)((nrhs + 7) / 8)), 256, 0, s>>>(
-        P, vals, nrhs, y, ylen, which, kb);
-    const int lo = (which == 0 || which == 2) ? kb + 64 : 0;
-    const int hi = (which == 0 || which == 2) ? (int)P.ntp : kb;
-    if (hi > lo)
-      k_trsv_blk_update<<<dim3((unsigned)((hi - lo + 31) / 32), (unsigned)count), 256, 0, s>>>(
-          P, vals, nrhs, y, ylen, which, kb, lo, hi);
-    lc.n += hi > lo ? 2 : 1;
-  }
 }
 
 void launch_residual(const PlanDev& P, int count, int nrhs, const double* a, const double* X,

@@ -124,7 +124,8 @@ void launch_gemm_sub(int M, int N, int K, const double* A, int lda, const double
 
 // solves; y: [count][nrhs][ylen] workspace, ylen = n + (ntp - nt)
 void launch_solve_permute_in(const PlanDev& P, int count, int nrhs, const double* B, double* y,
-                             int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc);
+                             int64_t ylen, int transpose, double* xbuf, int* err, cudaStream_t s,
+                             LaunchCounter& lc);
 void launch_solve_permute_out(const PlanDev& P, int count, int nrhs, const double* y, double* X,
                               int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc);
 void launch_sparse_lsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
@@ -146,8 +147,12 @@ void launch_front_solve(const PlanDev& P, const double* vals, int count, int nrh
                         cudaStream_t s, LaunchCounter& lc);
 void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                    int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc);
-void launch_dense_trsv(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                       int64_t ylen, int which, cudaStream_t s, LaunchCounter& lc);
+// L then U (transpose: U^T then L^T) of the dense block for every vector, one cooperative launch
+// (trsv.cu); xbuf, err: 2 ntp values a vector and the failure word, set up by
+// launch_solve_permute_in; a wait of more than budget_ms marks the instances GLU_INST_TIMEOUT
+void launch_dense_solve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                        int64_t ylen, bool transpose, double* xbuf, int* err, int32_t* status,
+                        double budget_ms, cudaStream_t s, LaunchCounter& lc);
 // r = b - op(A) x on the original matrix (R may be null) and per-vector norms; resid (may be
 // null) receives ||r||_inf / (||A||_inf ||x||_inf + ||b||_inf) per (instance, rhs)
 void launch_residual(const PlanDev& P, int count, int nrhs, const double* a, const double* X,

@@ -1,0 +1,371 @@
+// Triangular solves with the dense trailing block, every vector of the batch, in one launch.
+//
+// L then U of the block (or U^T then L^T) in row blocks of 64, as a dataflow among the CTAs of one
+// cooperative launch: the CTAs of a unit (an instance and up to NV of its right-hand sides) own
+// its row blocks in turn; a CTA subtracts the products with the blocks solved before from its own,
+// tile by tile as they become known, solves its 64 x 64 triangle and publishes the 64 values.  The
+// tiles do not depend on the solution, so they are fetched ahead of it, and the chain through the
+// block is, per 64 rows, one hand-over between CTAs, one tile product and one triangle.
+//
+// The solved values themselves are the signal: they go to a buffer that launch_solve_permute_in
+// has filled with kUnsolved, a NaN of a payload that no arithmetic produces, and a reader polls
+// the value it needs.  One 8-byte relaxed load that is not kUnsolved is the value, so a hand-over
+// needs neither a fence nor a flag behind the data.
+//
+// Bound by latency with few vectors (a hand-over and 64 dependent pivots per 64 rows), by HBM with
+// many.  Measured, L and U of n = 20,000's block (69 blocks of rows, 156 MB read): 0.38 ms for one
+// vector and 0.50 ms for 32, where a triangle launch and a push launch per block took 1.65 and
+// 2.36 ms; 256 x n = 2,000 0.13 ms, one CTA per vector with barriers between the steps 0.26 ms.
+// U is divided row by row by its diagonal while the CTA waits (one more rounding of each entry, a
+// division less on the chain of pivots: 0.94 -> 0.38 ms together with the polled values, against
+// progress counters that needed a fence and a second look).
+//
+// It replaces the reference's dense part of Symbolic_Matrix::solve (src/symbolic.cc:221-236).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "glu_b200.h"
+#include "kernels.cuh"
+#include "wait.cuh"
+
+namespace glu {
+
+namespace {
+
+constexpr int kWarp = 32;
+constexpr int kB = 64;               // rows of a block
+constexpr int kDs = 66;              // column stride of a staged triangle: rows by lane, 2-way at most
+
+template <int NV>
+constexpr int flow_smem() {
+  return (kB * kDs + 2 * kB * NV + 4 * NV * kB + kB) * 8;
+}
+
+// x / d from r = 1 / d with one FMA correction (see quotient in dense.cu)
+__device__ __forceinline__ double quotient_r(double x, double d, double r) {
+  const double q = x * r;
+  const double e = fma(fma(-q, d, x), r, q);
+  return (__double2hiint(q) & 0x7ff00000) != 0x7ff00000 ? e : q;
+}
+
+// The 64 x 64 triangle at T (T[i + kDs * j]) for one vector, rows lane and lane + 32 in r0 and r1.
+// which: 0 = L (unit lower, forward), 1 = U (backward), 2 = U^T (forward), 3 = L^T (backward).
+// Each solved value is broadcast and pushed into the remaining rows.  DIV: divide by the diagonal
+// (which 1, 2) with its reciprocals rc; otherwise the rows were divided by it beforehand.
+template <int WHICH, bool DIV>
+__device__ __forceinline__ void triangle(const double* __restrict__ T,
+                                         const double* __restrict__ rc, int lane, double& r0,
+                                         double& r1) {
+  constexpr bool fwd = WHICH == 0 || WHICH == 2;
+  constexpr int si = WHICH < 2 ? 1 : kDs, sj = WHICH < 2 ? kDs : 1;   // M(i, j) = T[i si + j sj]
+  const double* __restrict__ c0 = T + lane * si;
+  const double* __restrict__ c1 = T + (lane + 32) * si;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {               // the half of the rows that pivots lie in
+    const bool lo = fwd ? h == 0 : h == 1;
+#pragma unroll 8
+    for (int q = 0; q < 32; ++q) {
+      const int p = fwd ? q : 31 - q;         // lane of the pivot
+      const int j = lo ? p : p + 32;
+      double x = lo ? r0 : r1;
+      if (DIV) x = quotient_r(x, T[j * (kDs + 1)], rc[j]);
+      const double xj = __shfl_sync(0xffffffffu, x, p);
+      if (DIV && lane == p) (lo ? r0 : r1) = xj;
+      const bool rest = fwd ? lane > p : lane < p;
+      if (lo) {
+        if (rest) r0 -= c0[j * sj] * xj;
+        if (fwd) r1 -= c1[j * sj] * xj;
+      } else {
+        if (rest) r1 -= c1[j * sj] * xj;
+        if (!fwd) r0 -= c0[j * sj] * xj;
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ double ld_relaxed(const double* p) {
+  double v;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed(double* p, double v) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ bool unsolved(double v) {
+  return __double_as_longlong(v) == kUnsolved;
+}
+
+// The value at p, the first look at which gave v, once it is solved.  Bounded: after `budget_ns`
+// (recorded in *err), or once another CTA has recorded a failure there, *fail is set.
+__device__ __forceinline__ double wait_value(const double* p, double v, int* err,
+                                             unsigned long long budget_ns, int* fail) {
+  if (!unsolved(v)) return v;
+  const unsigned long long t0 = global_ns();
+  for (int spin = 1; unsolved(v = ld_relaxed(p)); ++spin) {
+    if (spin % 64) continue;
+    if (*(volatile int*)err) {
+      *fail = 1;
+      break;
+    }
+    if (global_ns() - t0 > budget_ns) {
+      atomicExch(err, 1);
+      *fail = 1;
+      break;
+    }
+  }
+  return v;
+}
+
+// One phase (WHICH as in triangle) of a unit (an instance's nv vectors) for CTA r of G.  rhs: the
+// block's right-hand side, to be waited for if `wait_rhs`; xb: the solved values (vectors xl
+// apart), also written to yd (vectors yl apart) if not null.  Returns false if a wait gave up.
+template <int NV, int WHICH>
+__device__ bool flow_phase(const double* __restrict__ D, int64_t ld, int nblk, const double* rhs,
+                           int64_t rl, bool wait_rhs, double* xb, int64_t xl, double* yd,
+                           int64_t yl, int nv, int r, int G, int* err,
+                           unsigned long long budget_ns, double* sm) {
+  constexpr bool fwd = WHICH == 0 || WHICH == 2;
+  constexpr bool trans = WHICH >= 2;
+  constexpr bool diag = WHICH == 1 || WHICH == 2;
+  constexpr int NX = (kB * NV + 255) / 256;   // values of a solved block per thread
+  double* Ds = sm;
+  double* xs = Ds + kB * kDs;                 // [2][kB][NV]
+  double* red = xs + 2 * kB * NV;             // [4][NV][kB]
+  double* rc = red + 4 * NV * kB;
+  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
+  const int vec = warp % NV;                  // the vector whose triangle this warp solves
+  for (int o = r; o < nblk; o += G) {
+    const int b = (fwd ? o : nblk - 1 - o) * kB;
+    // the diagonal block, the first tile and the right-hand side are on their way meanwhile
+    for (int e = tid; e < kB * kB / 2; e += 256) {
+      const int i = (e % 32) * 2, j = e / 32;
+      const unsigned dst = (unsigned)__cvta_generic_to_shared(Ds + i + j * kDs);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst),
+                   "l"(D + b + i + (int64_t)(b + j) * ld));
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    // a thread's 16 entries of the tile against block k: !trans, row tid % 64 of 16 columns;
+    // trans, two rows (of the solved block) of 8 columns
+    double m[16], xn[NX];
+    auto fetch = [&](int k, double (&t)[16]) {
+      const int kb = (fwd ? k : nblk - 1 - k) * kB;
+      if (!trans) {
+        const double* __restrict__ p = D + b + (tid & 63) + (int64_t)(kb + (tid >> 6) * 16) * ld;
+#pragma unroll
+        for (int q = 0; q < 16; ++q, p += ld) t[q] = *p;
+      } else {
+        const double* __restrict__ p = D + kb + 2 * lane + (int64_t)(b + warp * 8) * ld;
+#pragma unroll
+        for (int q = 0; q < 8; ++q, p += ld) {
+          const double2 v = *reinterpret_cast<const double2*>(p);
+          t[2 * q] = v.x;
+          t[2 * q + 1] = v.y;
+        }
+      }
+    };
+    // the address of value e (row e % 64 of vector e / 64) of solved block k; vectors past nv
+    // repeat the last one
+    auto xaddr = [&](int k, int e) {
+      return xb + (int64_t)min(e / kB, nv - 1) * xl + (fwd ? k : nblk - 1 - k) * kB + e % kB;
+    };
+    if (o > 0) {
+      fetch(0, m);
+#pragma unroll
+      for (int h = 0; h < NX; ++h)
+        if (tid + h * 256 < kB * NV) xn[h] = ld_relaxed(xaddr(0, tid + h * 256));
+    }
+    const double* ry = rhs + (int64_t)min(vec, nv - 1) * rl + b + lane;
+    double y0 = ld_relaxed(ry), y1 = ld_relaxed(ry + 32);
+    double acc[trans ? 8 * NV : NV];
+#pragma unroll
+    for (int i = 0; i < (trans ? 8 * NV : NV); ++i) acc[i] = 0.0;
+    int fail = 0;
+    bool plain = true;                        // the triangle needs no division on its chain
+    auto finish_stage = [&]() {
+      asm volatile("cp.async.wait_group 0;\n" ::);
+      __syncthreads();
+      if (diag) {
+        bool odd = false;
+        if (tid < kB) {
+          const double d = Ds[tid * (kDs + 1)];
+          rc[tid] = 1.0 / d;
+          const int ex = (__double2hiint(d) >> 20) & 0x7ff;
+          odd = ex < 64 || ex > 0x7ff - 64;
+        }
+        plain = !__syncthreads_or(odd);
+        // rows of the triangle divided by their diagonal (U: row i; U^T: column i of U): the
+        // division leaves the chain of pivots for one more rounding of each entry
+        if (plain) {
+          for (int e = tid; e < kB * kB; e += 256) {
+            const int i = e % kB, j = e / kB, d = trans ? j : i;
+            if (i < j) Ds[i + j * kDs] = quotient_r(Ds[i + j * kDs], Ds[d * (kDs + 1)], rc[d]);
+          }
+        }
+      }
+    };
+    for (int k = 0; k < o; ++k) {
+      if (k == o - 1) finish_stage();         // before waiting for the last block
+      double* x = xs + (k & 1) * kB * NV;
+#pragma unroll
+      for (int h = 0; h < NX; ++h) {
+        const int e = tid + h * 256;
+        if (e < kB * NV)
+          x[(e % kB) * NV + e / kB] = wait_value(xaddr(k, e), xn[h], err, budget_ns, &fail);
+      }
+      if (__syncthreads_or(fail)) return false;
+      if (k + 1 < o) {
+#pragma unroll
+        for (int h = 0; h < NX; ++h)
+          if (tid + h * 256 < kB * NV) xn[h] = ld_relaxed(xaddr(k + 1, tid + h * 256));
+      }
+      if (!trans) {
+#pragma unroll
+        for (int q = 0; q < 16; ++q)
+#pragma unroll
+          for (int v = 0; v < NV; ++v) acc[v] += m[q] * x[((tid >> 6) * 16 + q) * NV + v];
+      } else {
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const double x0 = x[2 * lane * NV + v], x1 = x[(2 * lane + 1) * NV + v];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[q * NV + v] += m[2 * q] * x0 + m[2 * q + 1] * x1;
+        }
+      }
+      if (k + 1 < o) fetch(k + 1, m);         // on its way while block k + 1 is waited for
+    }
+    if (o == 0) finish_stage();
+    if (!trans) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) red[((tid >> 6) * NV + v) * kB + (tid & 63)] = acc[v];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8 * NV; ++i) {
+        double t = acc[i];
+        for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+        if (lane == 0) red[(i % NV) * kB + warp * 8 + i / NV] = t;
+      }
+    }
+    if (wait_rhs) {
+      y0 = wait_value(ry, y0, err, budget_ns, &fail);
+      y1 = wait_value(ry + 32, y1, err, budget_ns, &fail);
+    }
+    if (__syncthreads_or(fail)) return false;  // sums, triangle and reciprocals are there too
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int q = 0; q < (trans ? 1 : 4); ++q) {
+      s0 += red[(q * NV + vec) * kB + lane];
+      s1 += red[(q * NV + vec) * kB + lane + 32];
+    }
+    y0 -= s0;
+    y1 -= s1;
+    // every warp solves (NV < 8: some the same vector), so that no branch holds the shuffles
+    if (!diag) {
+      triangle<WHICH, false>(Ds, rc, lane, y0, y1);
+    } else if (plain) {
+      y0 = quotient_r(y0, Ds[lane * (kDs + 1)], rc[lane]);
+      y1 = quotient_r(y1, Ds[(lane + 32) * (kDs + 1)], rc[lane + 32]);
+      triangle<WHICH, false>(Ds, rc, lane, y0, y1);
+    } else {
+      triangle<WHICH, true>(Ds, rc, lane, y0, y1);
+    }
+    if (warp < nv) {
+      double* xo = xb + vec * xl + b + lane;
+      st_relaxed(xo, unsolved(y0) ? __longlong_as_double(kNaN) : y0);
+      st_relaxed(xo + 32, unsolved(y1) ? __longlong_as_double(kNaN) : y1);
+      if (yd) {
+        yd[vec * yl + b + lane] = y0;
+        yd[vec * yl + b + lane + 32] = y1;
+      }
+    }
+    __syncthreads();                          // smem reuse by the next block
+  }
+  return true;
+}
+
+// Grid: groups of G CTAs; group g takes units g, g + groups, ...  xbuf: 2 ntp values a vector.
+template <int NV, bool TRANS>
+__global__ void __launch_bounds__(256, NV * (TRANS ? 2 : 1) >= 8 ? 1 : 2)
+    k_dense_flow(PlanDev P, const double* vals, int count, int nrhs, double* y, int64_t ylen,
+                 int G, double* xbuf, int* err, int32_t* status, unsigned long long budget_ns) {
+  extern __shared__ double sm[];
+  const int chunks = (nrhs + NV - 1) / NV;
+  const int units = count * chunks, groups = gridDim.x / G;
+  const int r = blockIdx.x % G, nblk = (int)(P.ntp / kB);
+  const int64_t xl = 2 * (int64_t)P.ntp;
+  for (int u = blockIdx.x / G; u < units; u += groups) {
+    const int inst = u / chunks, v0 = (u % chunks) * NV;
+    const int nv = min(NV, nrhs - v0);
+    const int64_t vec = (int64_t)inst * nrhs + v0;
+    const double* D = vals + (int64_t)inst * P.blob + P.dbase;
+    double* yd = y + vec * ylen + P.t;
+    double* x1 = xbuf + vec * xl;
+    double* x2 = x1 + P.ntp;
+    const bool ok =
+        flow_phase<NV, TRANS ? 2 : 0>(D, P.ntp, nblk, yd, ylen, false, x1, xl, nullptr, 0, nv, r, G,
+                                      err, budget_ns, sm) &&
+        flow_phase<NV, TRANS ? 3 : 1>(D, P.ntp, nblk, x1, xl, true, x2, xl, yd, ylen, nv, r, G, err,
+                                      budget_ns, sm);
+    if (!ok) {                                // a wait gave up: this unit and the rest are void
+      if (threadIdx.x == 0)
+        for (int w = u; w < units; w += groups) atomicOr(status + w / chunks, GLU_INST_TIMEOUT);
+      return;
+    }
+  }
+}
+
+template <int NV, bool TRANS>
+bool flow_launch(const PlanDev& P, const double* vals, int count, int nrhs, double* y, int64_t ylen,
+                 double* xbuf, int* err, int32_t* status, double budget_ms, cudaStream_t s,
+                 LaunchCounter& lc) {
+  const auto kern = k_dense_flow<NV, TRANS>;
+  ensure_smem_limit((const void*)kern, flow_smem<NV>());
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, flow_smem<NV>()) !=
+          cudaSuccess || per_sm < 1)
+    return false;
+  const int cap = per_sm * sm_count(), nblk = (int)(P.ntp / kB);
+  // the vectors' units share the CTAs that fit on the device: all of a block's rows in flight for
+  // a few vectors, down to one CTA walking the blocks of each of many
+  const int64_t units = (int64_t)count * ((nrhs + NV - 1) / NV);
+  const int G = (int)std::max<int64_t>(1, std::min<int64_t>(nblk, cap / units));
+  const int64_t groups = std::min<int64_t>(units, cap / G);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(groups * G));
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = flow_smem<NV>();
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;      // every CTA resident at once
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, P, vals, count, nrhs, y, ylen, G, xbuf, err, status,
+                     (unsigned long long)(budget_ms * 1e6));
+  lc.n++;
+  return true;
+}
+
+}  // namespace
+
+void launch_dense_solve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                        int64_t ylen, bool transpose, double* xbuf, int* err, int32_t* status,
+                        double budget_ms, cudaStream_t s, LaunchCounter& lc) {
+  if (P.ntp == 0) return;
+#define GLU_FLOW(NV, T)                                                                        \
+  flow_launch<NV, T>(P, vals, count, nrhs, y, ylen, xbuf, err, status, budget_ms, s, lc)
+  if (!transpose) {
+    if (nrhs == 1) GLU_FLOW(1, false);
+    else if (nrhs == 2) GLU_FLOW(2, false);
+    else if (nrhs <= 4) GLU_FLOW(4, false);
+    else GLU_FLOW(8, false);
+  } else {
+    if (nrhs == 1) GLU_FLOW(1, true);
+    else if (nrhs == 2) GLU_FLOW(2, true);
+    else GLU_FLOW(4, true);
+  }
+#undef GLU_FLOW
+}
+
+}  // namespace glu

@@ -1,0 +1,25 @@
+// What the bounded device-side waits of the cooperative kernels share.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace glu {
+
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// A value of the dense solve that has not been solved yet (a NaN payload no arithmetic produces),
+// and the NaN stored in its place should a solved value have these bits.
+constexpr long long kUnsolved = 0x7ff4a1c35e6b2d97ll;
+constexpr long long kNaN = 0x7ff8000000000000ll;
+
+}  // namespace glu
