@@ -360,12 +360,17 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
     const std::vector<int32_t>& ptr = L ? hp.lptr : hp.uptr;
     const std::vector<int32_t>& fptr = L ? hp.lfr_ptr : hp.ufr_ptr;
     const int ncols = ptr[l + 1] - ptr[l];
+    const int nlong = (L ? hp.llong : hp.ulng)[l];
     if (ncols > 0) {
       const int32_t* cols = L ? pl->d_lcols : pl->d_ucols;
-      if (which == 0) glu::launch_sparse_lsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, s, lc);
-      if (which == 1) glu::launch_sparse_usolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, s, lc);
-      if (which == 2) glu::launch_sparse_utsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, s, lc);
-      if (which == 3) glu::launch_sparse_ltsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, s, lc);
+      if (which == 0) glu::launch_sparse_lsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
+                                                  nlong, s, lc);
+      if (which == 1) glu::launch_sparse_usolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
+                                                  nlong, s, lc);
+      if (which == 2) glu::launch_sparse_utsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
+                                                  nlong, s, lc);
+      if (which == 3) glu::launch_sparse_ltsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
+                                                  nlong, s, lc);
     }
     const int nf = fptr[l + 1] - fptr[l];
     if (nf > 0) {

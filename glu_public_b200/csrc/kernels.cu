@@ -465,100 +465,179 @@ __global__ void k_permute_out(PlanDev P, int nrhs, const double* __restrict__ y,
   }
 }
 
-// Right-hand sides one warp handles together in the push-form sparse solves: the column's
-// indices and values are loaded once for all of them.
+// Right-hand sides handled together in the push-form sparse solves: a column's indices and values
+// are loaded once for all of them.
 constexpr int kSolveVecs = 4;
 
-// L solve, column oriented with unit diagonal (symbolic.cc:221-226), one warp per column and
-// group of up to kSolveVecs right-hand sides of one instance (grid.y = instance * groups + group).
-__global__ void k_sparse_lsolve(PlanDev P, const double* vals, int nrhs, double* y, int64_t ylen,
-                                const int32_t* __restrict__ cols, int begin, int ncols) {
-  const int w = blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
-  if (w >= ncols) return;
-  const int lane = threadIdx.x % kWarp;
-  const int groups = (nrhs + kSolveVecs - 1) / kSolveVecs;
-  const int64_t inst = blockIdx.y / groups;
-  const int k0 = (blockIdx.y % groups) * kSolveVecs;
-  const int nk = min(kSolveVecs, nrhs - k0);
-  const double* V = vals + inst * P.blob;
-  double* y0 = y + (inst * nrhs + k0) * ylen;
-  const uint32_t c = (uint32_t)cols[begin + w];
-  double yc[kSolveVecs];
+// The threads that share one column of a sparse solve level: kSolveLong or more entries take a CTA
+// of their own (the level's first nlong columns, one per CTA), else a warp each, eight columns
+// per CTA; i = the column's place in the level, -1 past its end.  Loads of kSolveUnroll entries
+// are in flight per thread: what bounds these kernels is the latency of the loads, a wide level's
+// columns being short and a few columns of the netlists (next to the dense block) thousands of
+// entries long.  Measured at n = 20,000, one vector: 30 L levels 0.93 -> 0.12 ms, 30 L^T levels
+// 0.70 -> 0.17 ms (before: one warp per column, one load in flight); 256 x n = 2,000, 14 L + 14 U
+// levels 0.253 -> 0.204 ms (a form of the kernels for one vector, no unrolling of short columns).
+constexpr int kSolveUnroll = 4;
+
+struct SolveShare {
+  int i, first, step;          // place in the level; first entry and stride of this thread
+  bool cta;
+};
+
+__device__ __forceinline__ SolveShare solve_share(int ncols, int nlong) {
+  if ((int)blockIdx.x < nlong)
+    return SolveShare{(int)blockIdx.x, (int)threadIdx.x, (int)blockDim.x, true};
+  const int i = nlong + ((int)blockIdx.x - nlong) * (int)(blockDim.x / kWarp) +
+                (int)(threadIdx.x / kWarp);
+  return SolveShare{i < ncols ? i : -1, (int)(threadIdx.x % kWarp), kWarp, false};
+}
+
+// Entries [p0, p1) of a column pushed into nk vectors: y(ri[p]) -= V[p] xc.
+template <int NV>
+__device__ __forceinline__ void solve_push(const PlanDev& P, const double* __restrict__ V,
+                                           double* y0, int64_t ylen, int nk,
+                                           const double (&xc)[NV], uint32_t p0, uint32_t p1,
+                                           const SolveShare& sh) {
+  uint32_t p = p0 + sh.first;
+  if (p1 - p0 <= 2 * (uint32_t)sh.step) {      // short columns: most of them, in a netlist
+    for (; p < p1; p += sh.step) {
+      const uint32_t r = P.ri[p];
+      const double m = V[p];
 #pragma unroll
-  for (int k = 0; k < kSolveVecs; ++k) yc[k] = k < nk ? y0[k * ylen + c] : 0.0;
-  for (uint32_t p = P.lp[c] + 1 + lane; p < P.cp[c + 1]; p += kWarp) {
-    const uint32_t r = P.ri[p];
-    const double l = V[p];
+      for (int k = 0; k < NV; ++k)
+        if (k < nk) atomicAdd(y0 + k * ylen + r, -(m * xc[k]));
+    }
+    return;
+  }
+  for (; p < p1; p += kSolveUnroll * sh.step) {
+    uint32_t r[kSolveUnroll];
+    double m[kSolveUnroll];
 #pragma unroll
-    for (int k = 0; k < kSolveVecs; ++k)
-      if (k < nk) atomicAdd(y0 + k * ylen + r, -(l * yc[k]));
+    for (int u = 0; u < kSolveUnroll; ++u) {
+      const uint32_t q = p + u * sh.step;
+      r[u] = q < p1 ? P.ri[q] : 0xffffffffu;
+      m[u] = q < p1 ? V[q] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kSolveUnroll; ++u) {
+      if (r[u] == 0xffffffffu) break;
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (k < nk) atomicAdd(y0 + k * ylen + r[u], -(m[u] * xc[k]));
+    }
   }
 }
 
-// U solve (symbolic.cc:228-236), one warp per column and group of right-hand sides.
-__global__ void k_sparse_usolve(PlanDev P, const double* vals, int nrhs, double* y, int64_t ylen,
-                                const int32_t* __restrict__ cols, int begin, int ncols) {
-  const int w = blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
-  if (w >= ncols) return;
-  const int lane = threadIdx.x % kWarp;
-  const int groups = (nrhs + kSolveVecs - 1) / kSolveVecs;
+// L solve, column oriented with unit diagonal (symbolic.cc:221-226), up to NV (1 or kSolveVecs)
+// right-hand sides of one instance together (grid.y = instance * groups + group).
+template <int NV>
+__global__ void __launch_bounds__(256) k_sparse_lsolve(PlanDev P, const double* vals, int nrhs,
+                                                       double* y, int64_t ylen,
+                                                       const int32_t* __restrict__ cols, int begin,
+                                                       int ncols, int nlong) {
+  const SolveShare sh = solve_share(ncols, nlong);
+  if (sh.i < 0) return;
+  const int groups = (nrhs + NV - 1) / NV;
   const int64_t inst = blockIdx.y / groups;
-  const int k0 = (blockIdx.y % groups) * kSolveVecs;
-  const int nk = min(kSolveVecs, nrhs - k0);
+  const int k0 = (blockIdx.y % groups) * NV;
+  const int nk = min(NV, nrhs - k0);
+  double* y0 = y + (inst * nrhs + k0) * ylen;
+  const uint32_t c = (uint32_t)cols[begin + sh.i];
+  double yc[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) yc[k] = k < nk ? y0[k * ylen + c] : 0.0;
+  solve_push(P, vals + inst * P.blob, y0, ylen, nk, yc, P.lp[c] + 1, P.cp[c + 1], sh);
+}
+
+// U solve (symbolic.cc:228-236).
+template <int NV>
+__global__ void __launch_bounds__(256) k_sparse_usolve(PlanDev P, const double* vals, int nrhs,
+                                                       double* y, int64_t ylen,
+                                                       const int32_t* __restrict__ cols, int begin,
+                                                       int ncols, int nlong) {
+  const SolveShare sh = solve_share(ncols, nlong);
+  if (sh.i < 0) return;
+  const int groups = (nrhs + NV - 1) / NV;
+  const int64_t inst = blockIdx.y / groups;
+  const int k0 = (blockIdx.y % groups) * NV;
+  const int nk = min(NV, nrhs - k0);
   const double* V = vals + inst * P.blob;
   double* y0 = y + (inst * nrhs + k0) * ylen;
-  const uint32_t c = (uint32_t)cols[begin + w];
+  const uint32_t c = (uint32_t)cols[begin + sh.i];
   const double d = V[P.lp[c]];
-  double xc[kSolveVecs];
+  double xc[NV];
 #pragma unroll
-  for (int k = 0; k < kSolveVecs; ++k) xc[k] = k < nk ? y0[k * ylen + c] / d : 0.0;
-  __syncwarp();
-  if (lane < nk) {                             // lane k stores x_c of right-hand side k
+  for (int k = 0; k < NV; ++k) xc[k] = k < nk ? y0[k * ylen + c] / d : 0.0;
+  if (sh.cta) __syncthreads(); else __syncwarp();   // every thread has read y_c
+  if (sh.first < nk) {                         // thread k stores x_c of right-hand side k
     double xv = xc[0];
 #pragma unroll
-    for (int k = 1; k < kSolveVecs; ++k)
-      if (lane == k) xv = xc[k];
-    y0[lane * ylen + c] = xv;
+    for (int k = 1; k < NV; ++k)
+      if (sh.first == k) xv = xc[k];
+    y0[sh.first * ylen + c] = xv;
   }
-  for (uint32_t p = P.cp[c] + lane; p < P.lp[c]; p += kWarp) {
-    const uint32_t r = P.ri[p];
-    const double u = V[p];
-#pragma unroll
-    for (int k = 0; k < kSolveVecs; ++k)
-      if (k < nk) atomicAdd(y0 + k * ylen + r, -(u * xc[k]));
-  }
+  solve_push(P, V, y0, ylen, nk, xc, P.cp[c], P.lp[c], sh);
 }
 
-// U^T solve (row j of U^T = column j of U), pull form, one warp per column.
-__global__ void k_sparse_utsolve(PlanDev P, const double* vals, int nrhs, double* y, int64_t ylen,
-                                 const int32_t* __restrict__ cols, int begin, int ncols) {
-  const int w = blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
-  if (w >= ncols) return;
-  const int lane = threadIdx.x % kWarp;
+// Sum of V[p] y(ri[p]) over the entries [p0, p1) of a column, in every thread of a warp share, in
+// thread 0 of a CTA share; the same order of additions in every run.
+__device__ __forceinline__ double solve_pull(const PlanDev& P, const double* __restrict__ V,
+                                             const double* yv, uint32_t p0, uint32_t p1,
+                                             const SolveShare& sh) {
+  __shared__ double part[8];
+  double s = 0.0;
+  uint32_t p = p0 + sh.first;
+  if (p1 - p0 <= 2 * (uint32_t)sh.step)
+    for (; p < p1; p += sh.step) s += V[p] * yv[P.ri[p]];
+  for (; p < p1; p += kSolveUnroll * sh.step) {
+    double m[kSolveUnroll], x[kSolveUnroll];
+#pragma unroll
+    for (int u = 0; u < kSolveUnroll; ++u) {
+      const uint32_t q = p + u * sh.step;
+      m[u] = q < p1 ? V[q] : 0.0;
+      x[u] = q < p1 ? yv[P.ri[q]] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kSolveUnroll; ++u) s += m[u] * x[u];
+  }
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (sh.cta) {                                // the same for the whole CTA
+    if (threadIdx.x % kWarp == 0) part[threadIdx.x / kWarp] = s;
+    __syncthreads();
+    s = 0.0;
+    for (int w = 0; w < (int)(blockDim.x / kWarp); ++w) s += part[w];
+  }
+  return s;
+}
+
+// U^T solve (row j of U^T = column j of U), pull form.
+__global__ void __launch_bounds__(256) k_sparse_utsolve(PlanDev P, const double* vals, int nrhs,
+                                                        double* y, int64_t ylen,
+                                                        const int32_t* __restrict__ cols,
+                                                        int begin, int ncols, int nlong) {
+  const SolveShare sh = solve_share(ncols, nlong);
+  if (sh.i < 0) return;
   const int64_t v = blockIdx.y;
   const double* V = vals + (v / nrhs) * P.blob;
   double* yv = y + v * ylen;
-  const uint32_t j = (uint32_t)cols[begin + w];
-  double s = 0.0;
-  for (uint32_t p = P.cp[j] + lane; p < P.lp[j]; p += kWarp) s += V[p] * yv[P.ri[p]];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) yv[j] = (yv[j] - s) / V[P.lp[j]];
+  const uint32_t j = (uint32_t)cols[begin + sh.i];
+  const double s = solve_pull(P, V, yv, P.cp[j], P.lp[j], sh);
+  if (sh.first == 0) yv[j] = (yv[j] - s) / V[P.lp[j]];
 }
 
 // L^T solve (row j of L^T = column j of L), pull form, unit diagonal.
-__global__ void k_sparse_ltsolve(PlanDev P, const double* vals, int nrhs, double* y, int64_t ylen,
-                                 const int32_t* __restrict__ cols, int begin, int ncols) {
-  const int w = blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
-  if (w >= ncols) return;
-  const int lane = threadIdx.x % kWarp;
+__global__ void __launch_bounds__(256) k_sparse_ltsolve(PlanDev P, const double* vals, int nrhs,
+                                                        double* y, int64_t ylen,
+                                                        const int32_t* __restrict__ cols,
+                                                        int begin, int ncols, int nlong) {
+  const SolveShare sh = solve_share(ncols, nlong);
+  if (sh.i < 0) return;
   const int64_t v = blockIdx.y;
   const double* V = vals + (v / nrhs) * P.blob;
   double* yv = y + v * ylen;
-  const uint32_t j = (uint32_t)cols[begin + w];
-  double s = 0.0;
-  for (uint32_t p = P.lp[j] + 1 + lane; p < P.cp[j + 1]; p += kWarp) s += V[p] * yv[P.ri[p]];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) yv[j] = yv[j] - s;
+  const uint32_t j = (uint32_t)cols[begin + sh.i];
+  const double s = solve_pull(P, V, yv, P.lp[j] + 1, P.cp[j + 1], sh);
+  if (sh.first == 0) yv[j] = yv[j] - s;
 }
 
 // A front in a triangular solve: one CTA per (front, vector) walks the front's columns in
@@ -738,20 +817,54 @@ __global__ void k_border(PlanDev P, const double* vals, int nrhs, double* y, int
 }
 
 // The forward solve's border y_r -= U(r, j) x_j (r < t <= j) in chunks of at most 1024 entries
-// of one tail column, a warp per chunk (grid (ceil(chunks / 8), vectors)), so the long border
-// columns of a mesh's top separator are shared by many warps.
-__global__ void k_border_chunks(PlanDev P, const double* vals, int nrhs, double* y, int64_t ylen) {
-  const int64_t k = (int64_t)blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
-  if (k >= P.nbordck) return;
+// of one tail column, a warp per chunk and up to NV right-hand sides of an instance (grid
+// (ceil(chunks / 8), instances * groups)), so the long border columns of a mesh's top separator
+// are shared by many warps and their entries are loaded once per group.
+template <int NV>
+__global__ void __launch_bounds__(256) k_border_chunks(PlanDev P, const double* vals, int nrhs,
+                                                       double* y, int64_t ylen) {
+  const int64_t c = (int64_t)blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
+  if (c >= P.nbordck) return;
   const int lane = threadIdx.x % kWarp;
-  const int jt = P.bord_ckcol[k];
-  const int64_t v = blockIdx.y;
-  const double* V = vals + (v / nrhs) * P.blob;
-  double* yv = y + v * ylen;
-  const int64_t e0 = P.bord_ck0[k], e1 = min(e0 + 1024, P.bord_ptr[jt + 1]);
-  const double xj = yv[P.t + jt];
-  for (int64_t e = e0 + lane; e < e1; e += kWarp)
-    atomicAdd(yv + P.bord_row[e], -(V[P.bord_slot[e]] * xj));
+  const int jt = P.bord_ckcol[c];
+  const int groups = (nrhs + NV - 1) / NV;
+  const int64_t inst = blockIdx.y / groups;
+  const int k0 = (blockIdx.y % groups) * NV;
+  const int nk = min(NV, nrhs - k0);
+  const double* V = vals + inst * P.blob;
+  double* y0 = y + (inst * nrhs + k0) * ylen;
+  const int64_t e0 = P.bord_ck0[c], e1 = min(e0 + 1024, P.bord_ptr[jt + 1]);
+  double xj[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) xj[k] = k < nk ? y0[k * ylen + P.t + jt] : 0.0;
+  int64_t e = e0 + lane;
+  if (e1 - e0 <= 2 * kWarp) {
+    for (; e < e1; e += kWarp) {
+      const int32_t r = P.bord_row[e];
+      const double m = V[P.bord_slot[e]];
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (k < nk) atomicAdd(y0 + k * ylen + r, -(m * xj[k]));
+    }
+    return;
+  }
+  for (; e < e1; e += kSolveUnroll * kWarp) {
+    int32_t r[kSolveUnroll];
+    double m[kSolveUnroll];
+#pragma unroll
+    for (int u = 0; u < kSolveUnroll; ++u) {
+      const int64_t q = e + u * kWarp;
+      r[u] = q < e1 ? P.bord_row[q] : -1;
+      m[u] = q < e1 ? V[P.bord_slot[q]] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kSolveUnroll; ++u) {
+      if (r[u] < 0) break;
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (k < nk) atomicAdd(y0 + k * ylen + r[u], -(m[u] * xj[k]));
+    }
+  }
 }
 
 // The 64x64 triangle of a front's push solve, by one warp in registers (rows lane and lane + 32),
@@ -1245,35 +1358,45 @@ void launch_solve_permute_out(const PlanDev& P, int count, int nrhs, const doubl
   lc.n++;
 }
 
-#define GLU_SOLVE_LAUNCH(KERNEL)                                                             \
-  k_##KERNEL<<<dim3((ncols + 7) / 8, count * nrhs), 256, 0, s>>>(P, vals, nrhs, y, ylen, cols, \
-                                                                 begin, ncols);              \
-  lc.n++;
-// the push forms take kSolveVecs right-hand sides per warp
-#define GLU_SOLVE_LAUNCH_GROUPED(KERNEL)                                                      \
-  k_##KERNEL<<<dim3((ncols + 7) / 8, count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0,  \
-               s>>>(P, vals, nrhs, y, ylen, cols, begin, ncols);                              \
-  lc.n++;
-
 void launch_sparse_lsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                          int64_t ylen, const int32_t* cols, int begin, int ncols,
+                          int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                           cudaStream_t s, LaunchCounter& lc) {
-  GLU_SOLVE_LAUNCH_GROUPED(sparse_lsolve)
+  const unsigned gx = nlong + (ncols - nlong + 7) / 8;
+  if (nrhs == 1)
+    k_sparse_lsolve<1><<<dim3(gx, count), 256, 0, s>>>(P, vals, nrhs, y, ylen, cols, begin, ncols,
+                                                    nlong);
+  else
+    k_sparse_lsolve<kSolveVecs><<<dim3(gx, count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0, s>>>(
+        P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+  lc.n++;
 }
 void launch_sparse_usolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                          int64_t ylen, const int32_t* cols, int begin, int ncols,
+                          int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                           cudaStream_t s, LaunchCounter& lc) {
-  GLU_SOLVE_LAUNCH_GROUPED(sparse_usolve)
+  const unsigned gx = nlong + (ncols - nlong + 7) / 8;
+  if (nrhs == 1)
+    k_sparse_usolve<1><<<dim3(gx, count), 256, 0, s>>>(P, vals, nrhs, y, ylen, cols, begin, ncols,
+                                                    nlong);
+  else
+    k_sparse_usolve<kSolveVecs><<<dim3(gx, count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0, s>>>(
+        P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+  lc.n++;
 }
 void launch_sparse_utsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                           int64_t ylen, const int32_t* cols, int begin, int ncols,
+                           int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                            cudaStream_t s, LaunchCounter& lc) {
-  GLU_SOLVE_LAUNCH(sparse_utsolve)
+  k_sparse_utsolve<<<dim3(nlong + (ncols - nlong + 7) / 8,
+                      count * nrhs), 256, 0, s>>>(
+      P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+  lc.n++;
 }
 void launch_sparse_ltsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                           int64_t ylen, const int32_t* cols, int begin, int ncols,
+                           int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                            cudaStream_t s, LaunchCounter& lc) {
-  GLU_SOLVE_LAUNCH(sparse_ltsolve)
+  k_sparse_ltsolve<<<dim3(nlong + (ncols - nlong + 7) / 8,
+                      count * nrhs), 256, 0, s>>>(
+      P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+  lc.n++;
 }
 
 void launch_front_solve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
@@ -1320,9 +1443,12 @@ void launch_front_solve(const PlanDev& P, const double* vals, int count, int nrh
 void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                    int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc) {
   if (P.nt == 0) return;
-  if (!transpose && P.nbordck > 0)
-    k_border_chunks<<<dim3((unsigned)((P.nbordck + 7) / 8), count * nrhs), 256, 0, s>>>(
-        P, vals, nrhs, y, ylen);
+  const unsigned gx = (unsigned)((P.nbordck + 7) / 8);
+  if (!transpose && P.nbordck > 0 && nrhs == 1)
+    k_border_chunks<1><<<dim3(gx, count), 256, 0, s>>>(P, vals, nrhs, y, ylen);
+  else if (!transpose && P.nbordck > 0)
+    k_border_chunks<kSolveVecs><<<dim3(gx, count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0,
+                                  s>>>(P, vals, nrhs, y, ylen);
   else
     k_border<<<dim3((P.nt + 7) / 8, count * nrhs), 256, 0, s>>>(P, vals, nrhs, y, ylen, transpose);
   lc.n++;

@@ -128,17 +128,18 @@ void launch_solve_permute_in(const PlanDev& P, int count, int nrhs, const double
                              LaunchCounter& lc);
 void launch_solve_permute_out(const PlanDev& P, int count, int nrhs, const double* y, double* X,
                               int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc);
+// one solve level; its first nlong columns take a CTA each (see kSolveLong, plan_host.h)
 void launch_sparse_lsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                          int64_t ylen, const int32_t* cols, int begin, int ncols,
+                          int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                           cudaStream_t s, LaunchCounter& lc);
 void launch_sparse_usolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                          int64_t ylen, const int32_t* cols, int begin, int ncols,
+                          int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                           cudaStream_t s, LaunchCounter& lc);
 void launch_sparse_utsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                           int64_t ylen, const int32_t* cols, int begin, int ncols,
+                           int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                            cudaStream_t s, LaunchCounter& lc);
 void launch_sparse_ltsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                           int64_t ylen, const int32_t* cols, int begin, int ncols,
+                           int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                            cudaStream_t s, LaunchCounter& lc);
 // fronts fids[0 .. nfronts) of one solve level, every vector (which as in k_front_solve)
 // max_w: the widest of the fronts listed in fids (at least their width)

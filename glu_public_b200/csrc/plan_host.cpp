@@ -658,7 +658,8 @@ int build_host_plan(uint32_t n, uint32_t nnz, const uint32_t* cp, const uint32_t
       for (int32_t x = 0; x < hp.fronts[f].w; ++x) fid[hp.fronts[f].s0 + x] = f;
     }
     auto build = [&](bool lower, std::vector<int32_t>& cols, std::vector<int32_t>& ptr,
-                     std::vector<int32_t>& fr, std::vector<int32_t>& frptr) {
+                     std::vector<int32_t>& fr, std::vector<int32_t>& frptr,
+                     std::vector<int32_t>& nlong) {
       std::vector<int32_t> lev(t, 0), flev(nf, 0);
       auto lv = [&](uint32_t k) { return fid[k] >= 0 ? flev[fid[k]] : lev[k]; };
       int32_t maxl = -1;
@@ -692,12 +693,22 @@ int build_host_plan(uint32_t n, uint32_t nnz, const uint32_t* cp, const uint32_t
       cols.assign(ptr[maxl + 1], 0);
       fr.assign(nf, 0);
       std::vector<int32_t> fc(ptr.begin(), ptr.end() - 1), ff(frptr.begin(), frptr.end() - 1);
+      // a level's long columns first
+      nlong.assign(maxl + 1, 0);
+      auto is_long = [&](uint32_t c) {
+        return (lower ? cp[c + 1] - lp[c] - 1 : lp[c] - cp[c]) >= kSolveLong;
+      };
       for (uint32_t c = 0; c < t; ++c)
-        if (fid[c] < 0) cols[fc[lev[c]]++] = (int32_t)c;
+        if (fid[c] < 0 && is_long(c)) {
+          cols[fc[lev[c]]++] = (int32_t)c;
+          nlong[lev[c]]++;
+        }
+      for (uint32_t c = 0; c < t; ++c)
+        if (fid[c] < 0 && !is_long(c)) cols[fc[lev[c]]++] = (int32_t)c;
       for (int32_t f = 0; f < nf; ++f) fr[ff[flev[f]]++] = f;
     };
-    build(true, hp.lcols, hp.lptr, hp.lfr, hp.lfr_ptr);
-    build(false, hp.ucols, hp.uptr, hp.ufr, hp.ufr_ptr);
+    build(true, hp.lcols, hp.lptr, hp.lfr, hp.lfr_ptr, hp.llong);
+    build(false, hp.ucols, hp.uptr, hp.ufr, hp.ufr_ptr, hp.ulng);
   }
   hp.bord_ptr.assign((size_t)hp.nt + 1, 0);
   hp.bord_row.clear();

@@ -53,6 +53,9 @@ struct FrontLevel {
   std::vector<int32_t> mmax, nmax, tiles4, tiles1;
 };
 
+// Entries from which a column of a sparse solve level gets a CTA instead of a warp.
+constexpr uint32_t kSolveLong = 192;
+
 struct HostPlan {
   uint32_t n = 0, nnz = 0, t = 0, nt = 0, ntp = 0;
   int64_t S = 0, dbase = 0, blob = 0;
@@ -92,6 +95,8 @@ struct HostPlan {
   std::vector<uint8_t> dhasl;
   std::vector<int64_t> pos2slot;
   std::vector<int32_t> lcols, lptr, ucols, uptr;
+  std::vector<int32_t> llong, ulng;           // columns of a solve level (its first ones) whose L
+                                              // / U part has at least kSolveLong entries
   // fronts in the solve schedules: level l runs fronts lfr[lfr_ptr[l] .. lfr_ptr[l+1])
   std::vector<int32_t> lfr, lfr_ptr, ufr, ufr_ptr;
   std::vector<int32_t> fs0, fw;               // first column and width of every front

@@ -1,0 +1,57 @@
+"""Sparse solve levels with columns around the length that gives a column a CTA of its own, against
+the elementwise backward-error bound of substitution."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from glu_public_b200 import glu
+from tests.test_gpu_dense_solve import check_solve
+
+pytestmark = pytest.mark.gpu
+LENGTHS = (1, 31, 33, 64, 65, 128, 191, 192, 193, 500)
+
+
+def long_columns(n, seed):
+    """Columns of the LENGTHS below the diagonal (rows drawn from the last part, so that they do not
+    all fill) and the same lengths above it, random short entries elsewhere; dense [n, n]."""
+    rng = np.random.default_rng(seed)
+    a = np.zeros((n, n))
+    for k, length in enumerate(LENGTHS):
+        a[rng.choice(np.arange(n - 520, n), length, replace=False), 3 + 2 * k] = 1.0
+        a[rng.choice(np.arange(0, 520), length, replace=False), n - 3 - 2 * k] = 1.0
+    short = rng.integers(0, n, (2, 2 * n))
+    a[short[0], short[1]] = 1.0
+    a *= rng.uniform(-1.0, 1.0, a.shape)
+    a[np.arange(n), np.arange(n)] = np.abs(a).sum(0) + np.abs(a).sum(1) + 1.0
+    return a
+
+
+@pytest.mark.parametrize("deterministic", [0, 1])
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("nrhs", [1, 2, 4, 5])
+def test_long_columns(nrhs, transpose, deterministic):
+    import torch
+    n = 1100
+    a = long_columns(n, 7)
+    col, row = np.nonzero(a.T)                # column order
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    # no dense block and no fronts: every column goes through the sparse levels
+    plan = glu.Plan(sym, dense_threshold=2.0, front_min_w=0, deterministic=deterministic)
+    assert plan.stat("nt") == 0
+    idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
+    plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
+    batch = glu.Batch(plan, 2)
+    val = torch.as_tensor(np.stack([sym.val, 2.0 * sym.val]), device="cuda")
+    batch.load_lu_values(val)
+    batch.refactor(0.0)
+    b = torch.as_tensor(np.random.default_rng(1).standard_normal((2, nrhs, n)), device="cuda")
+    x = batch.solve(b, transpose=transpose)
+    cp = sym.sym_c_ptr.astype(np.int64)
+    for i in range(2):
+        lu = np.zeros((n, n))                 # [column, row]
+        lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
+        nl = np.diff(cp) - (sym.l_col_ptr.astype(np.int64) - cp[:-1]) - 1
+        assert nl.max() >= 192 and (nl < 192).any()
+        check_solve(torch, lu, b[i], x[i], transpose)
