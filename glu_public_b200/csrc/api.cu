@@ -13,6 +13,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -423,6 +424,102 @@ int batch_residual_view(glu_batch_t b, const PlanDev** P, int* count, int* devic
 }
 }  // namespace glu
 
+// Releases the batch's captured graph.
+static void drop_graph(glu_batch_s* b) {
+  if (b->exec) cudaGraphExecDestroy(b->exec);
+  if (b->graph) cudaGraphDestroy(b->graph);
+  b->exec = nullptr;
+  b->graph = nullptr;
+}
+
+// Releases everything a batch holds.
+static void batch_free(glu_batch_s* b) {
+  if (!b) return;
+  drop_graph(b);
+  if (b->own_stream) cudaStreamDestroy(b->own_stream);
+  for (int i = 0; i < glu_batch_s::kFrontStreams; ++i) {
+    if (b->fstream[i]) cudaStreamDestroy(b->fstream[i]);
+    if (b->fjoin[i]) cudaEventDestroy(b->fjoin[i]);
+  }
+  if (b->ffork) cudaEventDestroy(b->ffork);
+  if (b->own_vals && b->vals) cudaFree(b->vals);
+  for (void* q : {(void*)b->pert, (void*)b->status, (void*)b->asm_flag, (void*)b->y,
+                  (void*)b->xbuf, (void*)b->gbuf, (void*)b->fbuf, (void*)b->rbuf,
+                  (void*)b->norms, (void*)b->pdesc, (void*)b->pbar})
+    if (q) cudaFree(q);
+  delete b;
+}
+
+// ---- spare batches ----
+// A program that makes a batch per call (the differentiable solve does) spends longer in cudaMalloc
+// and cudaFree than on the device: 16 x n = 4,960 forward and backward, 3.0 ms of kernels, took 8
+// to 20 ms a call, 3.2 ms with them spared.  So the buffers of a plan's last destroyed batch are
+// kept for its next batch of the same count: at most kSpareBytes in all, the oldest given up first,
+// released with the plan, and all of a device's when an allocation of this library fails there.
+static constexpr size_t kSpareBytes = (size_t)1 << 30;
+static std::mutex g_spares_mu;
+static std::vector<glu_batch_s*> g_spares;          // oldest first, at most one per plan
+
+static size_t batch_bytes(const glu_batch_s* b) {
+  const glu::HostPlan& hp = b->plan->hp;
+  const size_t doubles = ((size_t)hp.blob + (size_t)hp.front_area +
+                          2 * (size_t)hp.ntp * hp.hubs_p) * b->count +
+                         (size_t)(b->ylen + 2 * (int64_t)hp.ntp) * b->y_vectors +
+                         ((size_t)hp.n + 4) * b->r_vectors;
+  return sizeof(double) * doubles;
+}
+
+// The plan's spare batch if it has `count` instances (any if 0), no longer spare.
+static glu_batch_s* take_spare(glu_plan_s* p, int count) {
+  std::lock_guard<std::mutex> lock(g_spares_mu);
+  for (auto it = g_spares.begin(); it != g_spares.end(); ++it)
+    if ((*it)->plan == p && (count == 0 || (*it)->count == count)) {
+      glu_batch_s* b = *it;
+      g_spares.erase(it);
+      return b;
+    }
+  return nullptr;
+}
+
+// Frees every spare batch on the device; true if there was one.
+static bool free_spares(int device) {
+  bool any = false;
+  std::lock_guard<std::mutex> lock(g_spares_mu);
+  for (size_t i = g_spares.size(); i-- > 0;)
+    if (g_spares[i]->plan->device == device) {
+      batch_free(g_spares[i]);
+      g_spares.erase(g_spares.begin() + i);
+      any = true;
+    }
+  return any;
+}
+
+// Keeps a destroyed batch's buffers; false if they are not kept.
+static bool keep_spare(glu_batch_s* b) {
+  const size_t bytes = batch_bytes(b);
+  if (!b->own_vals || bytes > kSpareBytes) return false;
+  drop_graph(b);
+  b->loaded = b->factored = false;
+  b->launches = 0;
+  std::lock_guard<std::mutex> lock(g_spares_mu);
+  try {
+    g_spares.push_back(b);
+  } catch (const std::exception&) {
+    return false;
+  }
+  size_t total = 0;
+  for (size_t i = g_spares.size(); i-- > 0;) {      // newest first
+    total += batch_bytes(g_spares[i]);
+    if (g_spares[i] != b && (g_spares[i]->plan == b->plan || total > kSpareBytes)) {
+      total -= batch_bytes(g_spares[i]);
+      glu::DeviceGuard g(g_spares[i]->plan->device);
+      batch_free(g_spares[i]);
+      g_spares.erase(g_spares.begin() + i);
+    }
+  }
+  return true;
+}
+
 extern "C" {
 
 void glu_options_default(glu_options* o) {
@@ -821,6 +918,7 @@ int glu_plan_destroy(glu_plan_t p) {
   if (!p) return GLU_OK;
   {
     glu::DeviceGuard g(p->device);
+    batch_free(take_spare(p, 0));
     for (void* a : p->allocs) cudaFree(a);
   }
   delete p;
@@ -931,12 +1029,7 @@ static int build_persistent(glu_batch_s* b) {
   return GLU_OK;
 }
 
-static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_t* out) {
-  if (int st = check_plan(p)) return st;
-  if (!out || count <= 0 || count > 65535)
-    return set_error(GLU_ARGUMENT_ERROR, "count must be in [1, 65535]");
-  *out = nullptr;
-  glu::DeviceGuard g(p->device);
+static int batch_alloc(glu_plan_t p, int32_t count, double* storage, glu_batch_t* out) {
   glu_batch_s* b = new (std::nothrow) glu_batch_s();
   if (!b) return set_error(GLU_MEMORY_OVERFLOW, "host allocation failed");
   b->plan = p;
@@ -944,8 +1037,6 @@ static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_
   b->ylen = (int64_t)p->hp.n + (int64_t)(p->hp.ntp - p->hp.nt);
   const size_t bytes = sizeof(double) * (size_t)p->hp.blob * count;
   if (storage) {
-    if (reinterpret_cast<uintptr_t>(storage) % 256)
-      return delete b, set_error(GLU_ARGUMENT_ERROR, "storage must be 256-byte aligned");
     b->vals = storage;
   } else {
     if (cudaMalloc(&b->vals, bytes) != cudaSuccess) {
@@ -960,7 +1051,7 @@ static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_
     const size_t fbytes = sizeof(double) * (size_t)p->hp.front_area * count;
     if (cudaMalloc(&b->fbuf, fbytes) != cudaSuccess) {
       cudaGetLastError();
-      glu_batch_destroy(b);
+      batch_free(b);
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes (front buffers) failed", fbytes);
     }
   }
@@ -968,7 +1059,7 @@ static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_
     const size_t gbytes = sizeof(double) * 2 * (size_t)p->P.ntp * p->P.hubs_p * count;
     if (cudaMalloc(&b->gbuf, gbytes) != cudaSuccess) {
       cudaGetLastError();
-      glu_batch_destroy(b);
+      batch_free(b);
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes (hub panels) failed", gbytes);
     }
     cudaMemset(b->gbuf, 0, gbytes);
@@ -977,13 +1068,13 @@ static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_
       cudaMalloc(&b->status, sizeof(int32_t) * count) != cudaSuccess ||
       cudaMalloc(&b->asm_flag, count) != cudaSuccess) {
     cudaGetLastError();
-    glu_batch_destroy(b);
+    batch_free(b);
     return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc failed");
   }
   cudaMemset(b->status, 0, sizeof(int32_t) * count);
   cudaMemset(b->asm_flag, 0, count);
   if (int st = build_persistent(b)) {
-    glu_batch_destroy(b);
+    batch_free(b);
     return st;
   }
   if (!p->hp.fronts.empty()) {
@@ -993,12 +1084,40 @@ static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_
            cudaEventCreateWithFlags(&b->fjoin[i], cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
       cudaGetLastError();
-      glu_batch_destroy(b);
+      batch_free(b);
       return set_error(GLU_MEMORY_OVERFLOW, "front streams / events");
     }
   }
   *out = b;
   return glu::cuda_status("batch create");
+}
+
+static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_t* out) {
+  if (int st = check_plan(p)) return st;
+  if (!out || count <= 0 || count > 65535)
+    return set_error(GLU_ARGUMENT_ERROR, "count must be in [1, 65535]");
+  *out = nullptr;
+  glu::DeviceGuard g(p->device);
+  if (storage && reinterpret_cast<uintptr_t>(storage) % 256)
+    return set_error(GLU_ARGUMENT_ERROR, "storage must be 256-byte aligned");
+  if (!storage) {
+    // the spare batch's buffers may still be in use on some stream: wait for the device once, as
+    // the cudaFree they were spared from would have done
+    if (glu_batch_s* b = take_spare(p, count)) {
+      if (cudaDeviceSynchronize() == cudaSuccess &&
+          cudaMemset(b->status, 0, sizeof(int32_t) * count) == cudaSuccess &&
+          cudaMemset(b->asm_flag, 0, count) == cudaSuccess) {
+        *out = b;
+        return GLU_OK;
+      }
+      cudaGetLastError();
+      batch_free(b);
+    }
+  }
+  int st = batch_alloc(p, count, storage, out);
+  // memory that destroyed batches still hold goes before the call fails
+  if (st == GLU_MEMORY_OVERFLOW && free_spares(p->device)) st = batch_alloc(p, count, storage, out);
+  return st;
 }
 
 int glu_batch_create(glu_plan_t p, int32_t count, glu_batch_t* out) {
@@ -1013,27 +1132,7 @@ int glu_batch_create_external(glu_plan_t p, int32_t count, double* storage_dev, 
 int glu_batch_destroy(glu_batch_t b) {
   if (!b) return GLU_OK;
   glu::DeviceGuard g(b->plan->device);
-  if (b->exec) cudaGraphExecDestroy(b->exec);
-  if (b->graph) cudaGraphDestroy(b->graph);
-  if (b->own_stream) cudaStreamDestroy(b->own_stream);
-  for (int i = 0; i < glu_batch_s::kFrontStreams; ++i) {
-    if (b->fstream[i]) cudaStreamDestroy(b->fstream[i]);
-    if (b->fjoin[i]) cudaEventDestroy(b->fjoin[i]);
-  }
-  if (b->ffork) cudaEventDestroy(b->ffork);
-  if (b->own_vals && b->vals) cudaFree(b->vals);
-  if (b->pert) cudaFree(b->pert);
-  if (b->status) cudaFree(b->status);
-  if (b->asm_flag) cudaFree(b->asm_flag);
-  if (b->y) cudaFree(b->y);
-  if (b->xbuf) cudaFree(b->xbuf);
-  if (b->gbuf) cudaFree(b->gbuf);
-  if (b->fbuf) cudaFree(b->fbuf);
-  if (b->rbuf) cudaFree(b->rbuf);
-  if (b->norms) cudaFree(b->norms);
-  if (b->pdesc) cudaFree(b->pdesc);
-  if (b->pbar) cudaFree(b->pbar);
-  delete b;
+  if (!keep_spare(b)) batch_free(b);
   return GLU_OK;
 }
 
