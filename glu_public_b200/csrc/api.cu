@@ -126,7 +126,7 @@ struct glu_batch_s {
   int64_t r_vectors = 0;
   int64_t ylen = 0;
   int64_t y_vectors = 0;
-  double* xbuf = nullptr;       // solved values of the dense block (2 ntp per vector; trsv.cu),
+  double* xbuf = nullptr;       // solved values of the dense block and the fronts (trsv.cu),
                                 // then the solve's failure word
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -173,7 +173,7 @@ int ensure_workspace(glu_batch_t b, int64_t vectors, cudaStream_t s) {
   b->xbuf = nullptr;
   b->y_vectors = 0;
   if (cudaMalloc(&b->y, sizeof(double) * b->ylen * vectors) != cudaSuccess ||
-      cudaMalloc(&b->xbuf, sizeof(double) * (2 * (size_t)b->plan->P.ntp * vectors + 1)) !=
+      cudaMalloc(&b->xbuf, sizeof(double) * (glu::solve_buffer(b->plan->P) * vectors + 1)) !=
           cudaSuccess) {
     cudaGetLastError();
     return set_error(GLU_MEMORY_OVERFLOW, "solve workspace allocation failed");
@@ -349,37 +349,42 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
   double* y = b->y;
   const int64_t yl = b->ylen;
   const int cnt = b->count;
-  int* serr = reinterpret_cast<int*>(b->xbuf + 2 * (int64_t)P.ntp * b->y_vectors);
+  int* serr = reinterpret_cast<int*>(b->xbuf + glu::solve_buffer(P) * b->y_vectors);
   glu::launch_solve_permute_in(P, cnt, nrhs, B, y, yl, transpose, b->xbuf, serr, s, lc);
   auto dense = [&] {
     glu::launch_dense_solve(P, b->vals, cnt, nrhs, y, yl, transpose != 0, b->xbuf, serr, b->status,
                             b->pwait_ms, s, lc);
   };
   const int nl = (int)hp.lptr.size() - 1, nu = (int)hp.uptr.size() - 1;
-  // one solve level: its single columns, then its fronts (independent of each other)
+  // one level of a phase (which 0: L, 1: U, 2: U^T, 3: L^T): its single columns and its fronts,
+  // which do not depend on each other
   auto lvl = [&](bool L, int l, int which) {
     const std::vector<int32_t>& ptr = L ? hp.lptr : hp.uptr;
-    const std::vector<int32_t>& fptr = L ? hp.lfr_ptr : hp.ufr_ptr;
     const int ncols = ptr[l + 1] - ptr[l];
     const int nlong = (L ? hp.llong : hp.ulng)[l];
-    if (ncols > 0) {
-      const int32_t* cols = L ? pl->d_lcols : pl->d_ucols;
-      if (which == 0) glu::launch_sparse_lsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
-                                                  nlong, s, lc);
-      if (which == 1) glu::launch_sparse_usolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
-                                                  nlong, s, lc);
-      if (which == 2) glu::launch_sparse_utsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
-                                                  nlong, s, lc);
-      if (which == 3) glu::launch_sparse_ltsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols,
-                                                  nlong, s, lc);
-    }
-    const int nf = fptr[l + 1] - fptr[l];
-    if (nf > 0) {
-      const std::vector<int32_t>& fl = L ? hp.lfr : hp.ufr;
-      int max_w = 0;
-      for (int k = fptr[l]; k < fptr[l + 1]; ++k) max_w = std::max(max_w, hp.fw[fl[k]]);
-      glu::launch_front_solve(P, b->vals, cnt, nrhs, y, yl, (L ? P.lfr : P.ufr) + fptr[l], nf,
-                              max_w, which, s, lc);
+    const int32_t* cols = L ? pl->d_lcols : pl->d_ucols;
+    if (!hp.fronts.empty()) {
+      const std::vector<int32_t>& fptr = L ? hp.lflow_ptr : hp.uflow_ptr;
+      const std::vector<int32_t>& eptr =
+          which == 0 ? hp.lext_ptr : which == 1 ? hp.uext_ptr : which == 2 ? hp.udot_ptr : hp.ldot_ptr;
+      const glu::FrontLevelSolve FS{
+          (L ? P.lflow : P.uflow) + 2 * (int64_t)fptr[l], fptr[l + 1] - fptr[l],
+          (L ? hp.lfr_ptr : hp.ufr_ptr)[l + 1] - (L ? hp.lfr_ptr : hp.ufr_ptr)[l],
+          (which == 0 ? P.lext : which == 1 ? P.uext : which == 2 ? P.udot : P.ldot) +
+              4 * (int64_t)eptr[l], eptr[l + 1] - eptr[l]};
+      auto flow = [&] {
+        glu::launch_front_flow(P, b->vals, cnt, nrhs, y, yl, FS, which, b->xbuf, serr, b->status,
+                               b->pwait_ms, s, lc);
+      };
+      if (which == 0) flow();
+      glu::launch_solve_level(P, b->vals, cnt, nrhs, y, yl, which == 1 ? P.ur_rows : cols, ptr[l],
+                              ncols, which == 1 ? hp.ur_long[l] : nlong, FS, which, s, lc);
+      if (which != 0) flow();
+    } else if (ncols > 0) {
+      if (which == 0) glu::launch_sparse_lsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, nlong, s, lc);
+      if (which == 1) glu::launch_sparse_usolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, nlong, s, lc);
+      if (which == 2) glu::launch_sparse_utsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, nlong, s, lc);
+      if (which == 3) glu::launch_sparse_ltsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, nlong, s, lc);
     }
   };
   if (!transpose && hp.deterministic) {
@@ -396,7 +401,8 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
   } else if (!transpose) {
     for (int l = 0; l < nl; ++l) lvl(true, l, 0);
     dense();
-    glu::launch_border(P, b->vals, cnt, nrhs, y, yl, 0, s, lc);
+    // where there are fronts, rows and fronts pull the border with their other entries
+    if (hp.fronts.empty()) glu::launch_border(P, b->vals, cnt, nrhs, y, yl, 0, s, lc);
     for (int l = 0; l < nu; ++l) lvl(false, l, 1);
   } else {
     for (int l = nu - 1; l >= 0; --l) lvl(false, l, 2);
@@ -464,7 +470,7 @@ static size_t batch_bytes(const glu_batch_s* b) {
   const glu::HostPlan& hp = b->plan->hp;
   const size_t doubles = ((size_t)hp.blob + (size_t)hp.front_area +
                           2 * (size_t)hp.ntp * hp.hubs_p) * b->count +
-                         (size_t)(b->ylen + 2 * (int64_t)hp.ntp) * b->y_vectors +
+                         (size_t)(b->ylen + glu::solve_buffer(b->plan->P)) * b->y_vectors +
                          ((size_t)hp.n + 4) * b->r_vectors;
   return sizeof(double) * doubles;
 }
@@ -678,12 +684,17 @@ int glu_plan_create(uint32_t n, uint32_t nnz, const uint32_t* sym_c_ptr,
   }
   if ((st = p->upload(hp.lcols, &lc)) || (st = p->upload(hp.ucols, &uc)) ||
       (st = p->upload(hp.fs0, &P.fs0)) || (st = p->upload(hp.fw, &P.fw)) ||
-      (st = p->upload(hp.lfr, &P.lfr)) || (st = p->upload(hp.ufr, &P.ufr))) {
+      (st = p->upload(hp.lflow, &P.lflow)) || (st = p->upload(hp.uflow, &P.uflow)) ||
+      (st = p->upload(hp.lext, &P.lext)) || (st = p->upload(hp.uext, &P.uext)) ||
+      (st = p->upload(hp.ldot, &P.ldot)) || (st = p->upload(hp.udot, &P.udot)) ||
+      (st = p->upload(hp.fx0, &P.fx0)) || (st = p->upload(hp.uj_ptr, &P.uj_ptr)) ||
+      (st = p->upload(hp.uj_col, &P.uj_col)) || (st = p->upload(hp.uj_slot, &P.uj_slot)) ||
+      (st = p->upload(hp.ur_ptr, &P.ur_ptr)) || (st = p->upload(hp.ur_col, &P.ur_col)) ||
+      (st = p->upload(hp.ur_slot, &P.ur_slot)) || (st = p->upload(hp.ur_rows, &P.ur_rows))) {
     glu_plan_destroy(p);
     return st;
   }
-  P.fw_max = 0;
-  for (int32_t w : hp.fw) P.fw_max = std::max(P.fw_max, w);
+  P.fx_len = hp.fx_len;
   p->d_lcols = const_cast<int32_t*>(lc);
   p->d_ucols = const_cast<int32_t*>(uc);
   *out = p;
@@ -908,7 +919,7 @@ int glu_plan_stat(glu_plan_t p, int i, double* v) {
     case 23: *v = (double)hp.update_depth; break;
     case 24: *v = (double)hp.gemm_variant; break;
     case 25: *v = (double)hp.pull_xcol.size(); break;
-    case 26: *v = (double)p->P.fw_max; break;
+    case 26: *v = hp.fw.empty() ? 0.0 : (double)*std::max_element(hp.fw.begin(), hp.fw.end()); break;
     default: return set_error(GLU_ARGUMENT_ERROR, "unknown statistic %d", i);
   }
   return GLU_OK;

@@ -14,7 +14,6 @@
 //
 // Every kernel takes the instance index from blockIdx.y / blockIdx.z, so one launch covers a
 // whole batch of value sets of the same pattern.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -428,9 +427,10 @@ __global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm,
                              int64_t ylen, int transpose, double* xbuf, int* err) {
   const int64_t v = blockIdx.y;                 // instance * nrhs + rhs
   if (blockIdx.x == 0 && v == 0 && threadIdx.x == 0) *err = 0;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < 2 * (int64_t)P.ntp;
+  const int64_t nx = solve_buffer(P);
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nx;
        k += (int64_t)gridDim.x * blockDim.x)
-    xbuf[v * 2 * P.ntp + k] = __longlong_as_double(kUnsolved);
+    xbuf[v * nx + k] = __longlong_as_double(kUnsolved);
   const double* bv = Bm + v * P.n;
   double* yv = y + v * ylen;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < ylen;
@@ -640,127 +640,159 @@ __global__ void __launch_bounds__(256) k_sparse_ltsolve(PlanDev P, const double*
   if (sh.first == 0) yv[j] = yv[j] - s;
 }
 
-// A front in a triangular solve: one CTA per (front, vector) walks the front's columns in
-// order, so the chain of pivots inside the front costs barriers instead of launches.
-// which: 0 = L push (forward), 1 = U push (backward), 2 = U^T pull (forward), 3 = L^T pull
-// (backward) -- the column forms of the single-column kernels above.
-__global__ void __launch_bounds__(256) k_front_solve(PlanDev P, const double* vals, int nrhs,
+// One level of a phase of the solves of a plan with fronts (WHICH 0: L, 1: U, 2: U^T, 3: L^T), its
+// single columns and the products of its fronts with what lies outside them, up to NV right-hand
+// sides of one instance together (grid.y = instance * groups + group).  CTAs [0, ncb): columns as
+// in the kernels above; U by rows (all entries right of the diagonal pulled), so that the entries
+// above a front's rows need no atomics of their own.  The other CTAs take the pieces ext[..]:
+//   WHICH 0 / 1, 64 rows by up to 256 columns of L(R, S) or U(S, J), whose columns hold the rows
+//   contiguously: y_R -= L(R, S) x_S (after the level's launch_front_flow), y_S -= U(S, J) x_J
+//   (before it), a sum per row in registers and one atomic;
+//   WHICH 2 / 3, a warp per column: y_x -= U(. < s0, x) . y or L(R, x) . y (before it).
+// Bound by the latency of loads on most levels (a few columns and fronts), by HBM on none: the
+// grid of 512 x 512 x 2 nodes with 4 vectors reads 0.59 GB a solve.
+// Measured on that grid, per solve of 4 vectors: 169 L levels 1.38 ms, 169 U levels 1.17 ms and the
+// fronts' own rows (launch_front_flow) 1.55 ms, where pushed columns, one atomic per entry above a
+// front and one CTA or cluster per front took 11.6 ms; 128 x 128 x 2, one vector: 1.28 / 1.63 ms.
+template <int NV, int WHICH>
+__global__ void __launch_bounds__(256) k_solve_level(PlanDev P, const double* vals, int nrhs,
                                                      double* y, int64_t ylen,
-                                                     const int32_t* __restrict__ fids, int which) {
-  __shared__ double red[8];
-  __shared__ double bcast;
-  const int f = fids[blockIdx.x];
-  const int64_t v = blockIdx.y;
-  const double* V = vals + (v / nrhs) * P.blob;
-  double* yv = y + v * ylen;
-  const int s0 = P.fs0[f], w = P.fw[f];
+                                                     const int32_t* __restrict__ cols, int begin,
+                                                     int ncols, int nlong, int ncb,
+                                                     const int4* __restrict__ ext) {
+  __shared__ double xs[256 * NV];
+  __shared__ double red[4 * NV * 64];
+  __shared__ uint32_t bs[256];
+  const int groups = (nrhs + NV - 1) / NV;
+  const int64_t inst = blockIdx.y / groups;
+  const int k0 = (blockIdx.y % groups) * NV;
+  const int nk = min(NV, nrhs - k0);
+  const double* __restrict__ V = vals + inst * P.blob;
+  double* y0 = y + (inst * nrhs + k0) * ylen;
   const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
-  for (int step = 0; step < w; ++step) {
-    const bool fwd = (which == 0 || which == 2);
-    const uint32_t x = (uint32_t)(fwd ? s0 + step : s0 + w - 1 - step);
-    if (which == 0) {
-      __syncthreads();
-      const double yx = yv[x];
-      for (uint32_t p = P.lp[x] + 1 + tid; p < P.cp[x + 1]; p += blockDim.x)
-        atomicAdd(yv + P.ri[p], -(V[p] * yx));
-    } else if (which == 1) {
-      __syncthreads();
-      const double xx = yv[x] / V[P.lp[x]];
-      __syncthreads();
-      if (tid == 0) yv[x] = xx;
-      for (uint32_t p = P.cp[x] + tid; p < P.lp[x]; p += blockDim.x)
-        atomicAdd(yv + P.ri[p], -(V[p] * xx));
-    } else {
-      double sum = 0.0;
-      const uint32_t p0 = which == 2 ? P.cp[x] : P.lp[x] + 1;
-      const uint32_t p1 = which == 2 ? P.lp[x] : P.cp[x + 1];
-      for (uint32_t p = p0 + tid; p < p1; p += blockDim.x) sum += V[p] * yv[P.ri[p]];
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      if (lane == 0) red[warp] = sum;
-      __syncthreads();
-      if (tid == 0) {
-        double t = 0.0;
-        for (int q = 0; q < (int)(blockDim.x / kWarp); ++q) t += red[q];
-        yv[x] = which == 2 ? (yv[x] - t) / V[P.lp[x]] : yv[x] - t;
+  if ((int)blockIdx.x < ncb) {
+    const SolveShare sh = solve_share(ncols, nlong);
+    if (sh.i < 0) return;
+    const uint32_t c = (uint32_t)cols[begin + sh.i];
+    if (WHICH == 0) {
+      double yc[NV];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) yc[k] = k < nk ? y0[k * ylen + c] : 0.0;
+      solve_push(P, V, y0, ylen, nk, yc, P.lp[c] + 1, P.cp[c + 1], sh);
+    } else if (WHICH == 1) {
+      double sum[NV];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sum[k] = 0.0;
+      // the diagonal and the running value are on their way while the row is summed
+      const double d = V[P.lp[c]];
+      const double yc = sh.first < nk ? y0[sh.first * ylen + c] : 0.0;
+      const int64_t e0 = P.ur_ptr[c], e1 = P.ur_ptr[c + 1];
+      int64_t e = e0 + sh.first;
+      if (e1 - e0 <= 2 * sh.step) {
+        for (; e < e1; e += sh.step) {
+          const int32_t j = P.ur_col[e];
+          const double m = V[P.ur_slot[e]];
+#pragma unroll
+          for (int k = 0; k < NV; ++k) sum[k] += m * (k < nk ? y0[k * ylen + j] : 0.0);
+        }
       }
-      __syncthreads();
+      for (; e < e1; e += kSolveUnroll * sh.step) {
+        int32_t j[kSolveUnroll];
+        double m[kSolveUnroll];
+#pragma unroll
+        for (int u = 0; u < kSolveUnroll; ++u) {
+          const int64_t q = e + u * sh.step;
+          j[u] = q < e1 ? P.ur_col[q] : -1;
+          m[u] = q < e1 ? V[P.ur_slot[q]] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < kSolveUnroll; ++u) {
+          if (j[u] < 0) break;
+#pragma unroll
+          for (int k = 0; k < NV; ++k) sum[k] += m[u] * (k < nk ? y0[k * ylen + j[u]] : 0.0);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+        if (sh.cta && lane == 0) red[k * 8 + warp] = sum[k];
+      }
+      if (sh.cta) __syncthreads();
+      if (sh.first < nk) {                     // thread k finishes right-hand side k
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+          if (sh.first == k) t = sum[k];
+        if (sh.cta) {
+          t = 0.0;
+          for (int w = 0; w < 8; ++w) t += red[sh.first * 8 + w];
+        }
+        y0[sh.first * ylen + c] = (yc - t) / d;
+      }
+    } else {
+      const double t = WHICH == 2 ? solve_pull(P, V, y0, P.cp[c], P.lp[c], sh)
+                                  : solve_pull(P, V, y0, P.lp[c] + 1, P.cp[c + 1], sh);
+      if (sh.first == 0) y0[c] = WHICH == 2 ? (y0[c] - t) / V[P.lp[c]] : y0[c] - t;
     }
+    return;
   }
-}
-
-// k_front_solve for the push forms (which 0: L forward, 1: U backward) with the front's own
-// unknowns in shared memory: a step reads the pivot value from shared memory instead of global
-// memory, applies updates to the front's rows there (the rows of one column are distinct, so no
-// atomics) and pushes the rest to global memory with atomics, off the step-to-step chain; each
-// thread's first PF entries of a column (and the pivot) are loaded one step ahead, so the chain
-// from column to column is a barrier and a few shared-memory operations.  Same products and
-// quotients as k_front_solve.
-__global__ void __launch_bounds__(256) k_front_solve_push(PlanDev P, const double* vals, int nrhs,
-                                                          double* y, int64_t ylen,
-                                                          const int32_t* __restrict__ fids,
-                                                          int which) {
-  extern __shared__ double fsm[];
-  const int f = fids[blockIdx.x];
-  const int64_t v = blockIdx.y;
-  const double* __restrict__ V = vals + (v / nrhs) * P.blob;
-  double* yv = y + v * ylen;
-  const int s0 = P.fs0[f], w = P.fw[f];
-  double* ys = fsm;                                          // running values of the front's rows
-  double* xs = fsm + P.fw_max;                               // U: the solved values
-  uint32_t* pb = reinterpret_cast<uint32_t*>(fsm + 2 * P.fw_max);   // entry range per column
-  uint32_t* pe = pb + P.fw_max;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  for (int x = tid; x < w; x += nt) {
-    const uint32_t c = (uint32_t)(s0 + x);
-    ys[x] = yv[c];
-    pb[x] = which == 0 ? P.lp[c] + 1 : P.cp[c];
-    pe[x] = which == 0 ? P.cp[c + 1] : P.lp[c];
+  const int4 it = ext[blockIdx.x - ncb];
+  const int f = it.x, s0 = P.fs0[f], w = P.fw[f];
+  if (WHICH >= 2) {
+    const int x = it.y + warp;
+    if (x >= w) return;
+    const uint32_t d = P.lp[s0 + x];           // rows s0 .. of column s0 + x start at d - x
+    const SolveShare sh{x, lane, kWarp, false};
+    const double t = WHICH == 2 ? solve_pull(P, V, y0, P.cp[s0 + x], d - x, sh)
+                                : solve_pull(P, V, y0, d - x + w, P.cp[s0 + x + 1], sh);
+    if (lane == 0) y0[s0 + x] -= t;
+    return;
   }
-  __syncthreads();
-  constexpr int PF = 4;
-  uint32_t rn[PF];
-  double vn[PF], dn = 1.0;
-  auto prefetch = [&](int step) {                            // entries of the step's column
-    const int x = which == 0 ? step : w - 1 - step;
-    const uint32_t b0 = pb[x], e0 = pe[x];
+  const int r0 = it.y, c0 = it.z;
+  const uint32_t q0 = P.lp[s0] + w;            // rows R in column s0
+  const int64_t j0 = WHICH == 1 ? P.uj_ptr[f] + c0 : 0;
+  const int rows = WHICH == 0 ? (int)(P.cp[s0 + 1] - q0) : w;
+  const int nc = WHICH == 0 ? min(256, w - c0) : (int)min((int64_t)256, P.uj_ptr[f + 1] - j0);
+  if (tid < nc) {
+    const int32_t j = WHICH == 0 ? s0 + c0 + tid : P.uj_col[j0 + tid];
+    bs[tid] = (WHICH == 0 ? P.lp[j] - (c0 + tid) + w : (uint32_t)P.uj_slot[j0 + tid]) + r0;
 #pragma unroll
-    for (int k = 0; k < PF; ++k) {
-      const uint32_t p = b0 + tid + k * nt;
-      rn[k] = p < e0 ? P.ri[p] : 0xffffffffu;
-      vn[k] = p < e0 ? V[p] : 0.0;
-    }
-    dn = which == 1 ? V[e0] : 1.0;                           // U(x, x) sits at lp[c] = pe[x]
-  };
-  prefetch(0);
-  for (int step = 0; step < w; ++step) {
-    const int x = which == 0 ? step : w - 1 - step;
-    uint32_t r[PF];
-    double m[PF];
-#pragma unroll
-    for (int k = 0; k < PF; ++k) {
-      r[k] = rn[k];
-      m[k] = vn[k];
-    }
-    const double d = dn;
-    if (step + 1 < w) prefetch(step + 1);
-    __syncthreads();                                         // the previous step's updates
-    double xv = ys[x];
-    if (which == 1) {
-      xv = xv / d;
-      if (tid == 0) xs[x] = xv;
-    }
-    auto apply = [&](uint32_t rr, double mm) {
-      if (rr >= (uint32_t)s0 && rr < (uint32_t)(s0 + w)) ys[rr - s0] -= mm * xv;
-      else atomicAdd(yv + rr, -(mm * xv));
-    };
-#pragma unroll
-    for (int k = 0; k < PF; ++k)
-      if (r[k] != 0xffffffffu) apply(r[k], m[k]);
-    const uint32_t e0 = pe[x];
-    for (uint32_t p = pb[x] + tid + PF * nt; p < e0; p += nt) apply(P.ri[p], V[p]);
+    for (int k = 0; k < NV; ++k) xs[tid * NV + k] = k < nk ? y0[k * ylen + j] : 0.0;
   }
   __syncthreads();
-  for (int x = tid; x < w; x += nt) yv[s0 + x] = which == 0 ? ys[x] : xs[x];
+  const int r = tid & 63, seg = tid >> 6;
+  double acc[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) acc[k] = 0.0;
+  if (r0 + r < rows) {
+    int i = seg;
+    for (; i + 28 < nc; i += 32) {             // 8 columns of this quarter in flight
+      double m[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) m[u] = V[bs[i + 4 * u] + r];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int k = 0; k < NV; ++k) acc[k] += m[u] * xs[(i + 4 * u) * NV + k];
+    }
+    for (; i < nc; i += 4) {
+      const double m = V[bs[i] + r];
+#pragma unroll
+      for (int k = 0; k < NV; ++k) acc[k] += m * xs[i * NV + k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k) red[(seg * NV + k) * 64 + r] = acc[k];
+  __syncthreads();
+  for (int e = tid; e < 64 * nk; e += 256) {
+    const int row = e % 64, k = e / 64;
+    if (r0 + row >= rows) continue;
+    double t = 0.0;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) t += red[(g * NV + k) * 64 + row];
+    const uint32_t target = WHICH == 0 ? P.ri[q0 + r0 + row] : (uint32_t)(s0 + r0 + row);
+    atomicAdd(y0 + k * ylen + target, -t);
+  }
 }
 
 // Row-wise (pull) forward solves of the deterministic mode, one warp per row; each sum is
@@ -863,285 +895,6 @@ __global__ void __launch_bounds__(256) k_border_chunks(PlanDev P, const double* 
 #pragma unroll
       for (int k = 0; k < NV; ++k)
         if (k < nk) atomicAdd(y0 + k * ylen + r[u], -(m[u] * xj[k]));
-    }
-  }
-}
-
-// The 64x64 triangle of a front's push solve, by one warp in registers (rows lane and lane + 32),
-// the block read from shared memory (Ds[i + 64 j]).  which: 0 = L (unit lower, forward), 1 = U
-// (backward).
-// yb[0 .. 64) must already hold every contribution from outside the block.
-__device__ __forceinline__ void dense_block_solve(int which, const double* __restrict__ Ds,
-                                                  double* yb, int lane, double* xs) {
-  constexpr int TB = 64;
-  double r0 = yb[lane], r1 = yb[lane + 32];
-  if (which == 0) {
-    for (int i = 0; i < TB; ++i) {
-      const double xi = __shfl_sync(0xffffffffu, i < 32 ? r0 : r1, i & 31);
-      const double* col = Ds + i * TB;
-      if (lane > i) r0 -= col[lane] * xi;
-      if (lane + 32 > i) r1 -= col[lane + 32] * xi;
-    }
-  } else {
-    for (int i = TB - 1; i >= 0; --i) {
-      const double* col = Ds + i * TB;
-      if (lane == (i & 31)) {
-        if (i < 32) r0 = r0 / col[i]; else r1 = r1 / col[i];
-      }
-      const double xi = __shfl_sync(0xffffffffu, i < 32 ? r0 : r1, i & 31);
-      if (lane < i) r0 -= col[lane] * xi;
-      if (lane + 32 < i) r1 -= col[lane + 32] * xi;
-    }
-  }
-  yb[lane] = r0;
-  yb[lane + 32] = r1;
-  if (xs) {
-    xs[lane] = r0;
-    xs[lane + 32] = r1;
-  }
-}
-
-// The 64 x 64 diagonal block of a front's columns [xb, xb + 64) (column x's rows s0 + xb ..
-// s0 + xb + 63 start at position pz[x] + xb: a front's diagonal block is dense) copied into D
-// (D[i + 64 j]) with 8-byte asynchronous copies, committed as one group; only for a block that
-// lies inside the front.  dense_block_solve reads only the triangle it needs, so the other
-// triangle's values may stay in D.
-__device__ __forceinline__ void front_stage_async(const double* __restrict__ V,
-                                                  const long long* pz, int xb, double* D, int tid,
-                                                  int nt) {
-  for (int idx = tid; idx < 64 * 64; idx += nt) {
-    const int i = idx % 64, j = idx / 64;
-    const unsigned dst = (unsigned)__cvta_generic_to_shared(D + idx);
-    const double* src = V + pz[xb + j] + xb + i;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src));
-  }
-  asm volatile("cp.async.commit_group;\n" ::);
-}
-
-// The same block when it runs past the front (nb < 64 columns): the triangle's values and the
-// identity on the padding, by plain loads.
-__device__ __forceinline__ void front_stage_edge(const double* __restrict__ V, const long long* pz,
-                                                 int xb, int nb, int which, double* D, int tid,
-                                                 int nt) {
-  for (int idx = tid; idx < 64 * 64; idx += nt) {
-    const int i = idx % 64, j = idx / 64;
-    double val = 0.0;
-    if (i < nb && j < nb) {
-      if (which == 0 ? i > j : i <= j) val = V[pz[xb + j] + xb + i];
-    } else if (i == j) {
-      val = 1.0;                                    // padding: identity
-    }
-    D[idx] = val;
-  }
-}
-
-// A front in the push-form solves (which 0: L forward, 1: U backward), blocked: one CTA per
-// (front, vector).  The front's unknowns y_S stay in shared memory; its columns are taken 64 at a
-// time: the 64 x 64 triangle of the block (a front's diagonal block is dense, so column x's rows
-// s0 .. s1-1 sit contiguously from position lp[x] - (x - s0)) is staged in shared memory and
-// solved by one warp (dense_block_solve), then every thread pushes the block into the front's
-// remaining rows.  After the last block the updates leaving the front go out: for L, the rows R
-// below the front take y_R -= L(R, S) y_S, one sum and one atomic per row (R is the same row list
-// in every column of the front); for U, the entries above row s0 of every column, one atomic
-// each.  The chain from block to block is a triangle and two barriers instead of one barrier
-// per column; each push is the sum of the block's products subtracted at once.
-__global__ void __launch_bounds__(256) k_front_solve_blk(PlanDev P, const double* vals, int nrhs,
-                                                         double* y, int64_t ylen,
-                                                         const int32_t* __restrict__ fids,
-                                                         int which, int tail) {
-  constexpr int TB = 64;
-  extern __shared__ double fsm[];
-  const int f = fids[blockIdx.x];
-  const int s0 = P.fs0[f], w = P.fw[f];
-  const int wpad = (w + TB - 1) / TB * TB;
-  double* Ds = fsm;                                 // [2][TB * TB] the blocks' triangles
-  double* xs = Ds + 2 * TB * TB;                    // [TB] the block's solved values
-  double* ys = xs + TB;                             // [wpad] the front's unknowns
-  long long* pz = reinterpret_cast<long long*>(ys + ((P.fw_max + TB - 1) / TB) * TB);
-  const int64_t v = blockIdx.y;
-  const double* __restrict__ V = vals + (v / nrhs) * P.blob;
-  double* yv = y + v * ylen;
-  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp, nt = blockDim.x;
-  for (int x = tid; x < wpad; x += nt) {
-    ys[x] = x < w ? yv[s0 + x] : 0.0;
-    if (x < w) pz[x] = (long long)P.lp[s0 + x] - x;  // position of row s0 in column s0 + x
-  }
-  __syncthreads();
-  const int nblk = wpad / TB;
-  // block bi's triangle goes to Ds[bi & 1]; the next block's is copied in while this one is
-  // solved and pushed
-  const int xb0 = (which == 0 ? 0 : nblk - 1) * TB;
-  if (xb0 + TB <= w) front_stage_async(V, pz, xb0, Ds, tid, nt);
-  for (int bi = 0; bi < nblk; ++bi) {
-    const int xb = (which == 0 ? bi : nblk - 1 - bi) * TB;
-    const int nb = min(TB, w - xb);
-    double* D = Ds + (bi & 1) * TB * TB;
-    if (nb == TB) asm volatile("cp.async.wait_group 0;\n" ::);
-    else front_stage_edge(V, pz, xb, nb, which, D, tid, nt);
-    __syncthreads();
-    if (bi + 1 < nblk) {
-      const int xn = (which == 0 ? bi + 1 : nblk - 2 - bi) * TB;
-      if (xn + TB <= w) front_stage_async(V, pz, xn, Ds + ((bi + 1) & 1) * TB * TB, tid, nt);
-    }
-    if (warp == 0) dense_block_solve(which, D, ys + xb, lane, xs);
-    __syncthreads();
-    const int lo = which == 0 ? xb + nb : 0, hi = which == 0 ? w : xb;
-    for (int r = lo + tid; r < hi; r += nt) {
-      double sum = 0.0;
-      for (int j = 0; j < nb; ++j) sum += V[pz[xb + j] + r] * xs[j];
-      ys[r] -= sum;
-    }
-    __syncthreads();
-  }
-  for (int x = tid; x < w; x += nt) yv[s0 + x] = ys[x];
-  if (!tail) return;                                // k_front_solve_tail applies the rest
-  if (which == 0) {
-    const int64_t q0 = pz[0] + w;                   // the rows R in column s0
-    const int m = (int)((int64_t)P.cp[s0 + 1] - q0);
-    for (int i = tid; i < m; i += nt) {
-      double sum = 0.0;
-      for (int x = 0; x < w; ++x) sum += V[pz[x] + w + i] * ys[x];
-      atomicAdd(yv + P.ri[q0 + i], -sum);
-    }
-  } else {
-    for (int x = warp; x < w; x += nt / kWarp) {
-      const double xx = ys[x];
-      for (int64_t p = P.cp[s0 + x] + lane; p < pz[x]; p += kWarp)
-        atomicAdd(yv + P.ri[p], -(V[p] * xx));
-    }
-  }
-}
-
-// A wide front in the push-form solves (which 0: L forward, 1: U backward) by a cluster of kFsC
-// CTAs (grid (fronts * kFsC, vectors)): the front's unknowns are dealt out in 64-row blocks,
-// block k to CTA k % kFsC, and every CTA keeps the front's unknowns in its shared memory but
-// updates only its own blocks.  Per 64-column block: the CTA that owns it stages its triangle,
-// solves it with one warp and writes the 64 values into every CTA's xs buffer (distributed shared
-// memory, two buffers in turn); after one cluster barrier every CTA pushes the block into its own
-// rows.  So the push over the rest of the front, which one CTA per front does alone in
-// k_front_solve_blk, is spread over kFsC SMs.  The arithmetic of every unknown is the same as
-// there (same triangle code, each row's sum over the block's columns in the same order).  The
-// rows outside the front are left to k_front_solve_tail.  Every CTA of a cluster walks the same
-// blocks, so all reach every barrier.
-constexpr int kFsC = 8;
-
-__global__ void __cluster_dims__(kFsC, 1, 1) __launch_bounds__(256)
-    k_front_solve_cluster(PlanDev P, const double* vals, int nrhs, double* y, int64_t ylen,
-                          const int32_t* __restrict__ fids, int which) {
-  namespace cg = cooperative_groups;
-  constexpr int TB = 64;
-  extern __shared__ double fsm[];
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank();
-  const int f = fids[blockIdx.x / kFsC];
-  const int s0 = P.fs0[f], w = P.fw[f];
-  const int wpad = (w + TB - 1) / TB * TB;
-  const int fwp = (P.fw_max + TB - 1) / TB * TB;
-  double* Ds = fsm;                                 // [2][TB * TB] the owner's triangles
-  double* xs = Ds + 2 * TB * TB;                    // [2][TB] solved values of a block
-  double* ys = xs + 2 * TB;                         // [fwp] the front's unknowns
-  long long* pz = reinterpret_cast<long long*>(ys + fwp);
-  const int64_t v = blockIdx.y;
-  const double* __restrict__ V = vals + (v / nrhs) * P.blob;
-  double* yv = y + v * ylen;
-  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp, nt = blockDim.x;
-  for (int x = tid; x < wpad; x += nt) {
-    ys[x] = x < w ? yv[s0 + x] : 0.0;
-    if (x < w) pz[x] = (long long)P.lp[s0 + x] - x;  // position of row s0 in column s0 + x
-  }
-  __syncthreads();
-  const int nblk = wpad / TB;
-  // this CTA's blocks kb (kb % kFsC == rank) take Ds[(kb / kFsC) & 1] in turn; the next one's
-  // triangle is copied in while the cluster works on the blocks in between
-  {
-    const int k0 = which == 0 ? rank : nblk - 1 - ((nblk - 1 - rank) % kFsC + kFsC) % kFsC;
-    if (k0 >= 0 && k0 < nblk && (k0 + 1) * TB <= w)
-      front_stage_async(V, pz, k0 * TB, Ds + ((k0 / kFsC) & 1) * TB * TB, tid, nt);
-  }
-  for (int bi = 0; bi < nblk; ++bi) {
-    const int kb = which == 0 ? bi : nblk - 1 - bi;
-    const int xb = kb * TB;
-    const int nb = min(TB, w - xb);
-    double* xbuf = xs + (bi & 1) * TB;
-    if (kb % kFsC == rank) {
-      double* D = Ds + ((kb / kFsC) & 1) * TB * TB;
-      if (nb == TB) asm volatile("cp.async.wait_group 0;\n" ::);
-      else front_stage_edge(V, pz, xb, nb, which, D, tid, nt);
-      __syncthreads();
-      const int kn = which == 0 ? kb + kFsC : kb - kFsC;
-      if (kn >= 0 && kn < nblk && (kn + 1) * TB <= w)
-        front_stage_async(V, pz, kn * TB, Ds + ((kn / kFsC) & 1) * TB * TB, tid, nt);
-      if (warp == 0) {
-        dense_block_solve(which, D, ys + xb, lane, nullptr);
-        __syncwarp();
-        const double a = ys[xb + lane], b = ys[xb + lane + 32];
-        for (int k = 0; k < kFsC; ++k) {
-          double* dst = cl.map_shared_rank(xbuf, k);
-          dst[lane] = a;
-          dst[lane + 32] = b;
-        }
-      }
-    }
-    cl.sync();
-    // this CTA's row blocks in [lo, hi): 64 rows per block, four blocks at a time
-    const int lo = which == 0 ? xb + nb : 0, hi = which == 0 ? w : xb;
-    if (lo < hi) {
-      const int b_lo = lo / TB, b_hi = (hi + TB - 1) / TB;
-      const int first = b_lo + ((rank - b_lo % kFsC) % kFsC + kFsC) % kFsC;
-      for (int bb = first + (tid / TB) * kFsC; bb < b_hi; bb += (nt / TB) * kFsC) {
-        const int r = bb * TB + tid % TB;
-        if (r < lo || r >= hi) continue;
-        double sum = 0.0;
-        for (int j = 0; j < nb; ++j) sum += V[pz[xb + j] + r] * xbuf[j];
-        ys[r] -= sum;
-      }
-    }
-    __syncthreads();
-  }
-  for (int x = tid; x < w; x += nt)
-    if ((x / TB) % kFsC == rank) yv[s0 + x] = ys[x];
-}
-
-// The part of a front's push solve outside the front, after k_front_solve_blk or
-// k_front_solve_cluster has written the front's unknowns x_S: L: y_R -= L(R, S) x_S; U:
-// y_r -= U(r, S) x_S for the rows r < s0 above the front.  One CTA per 64 columns of S (grid
-// (ceil(max w / 64), fronts, vectors)), so a wide front's rows R or its long U columns are spread
-// over many SMs instead of one CTA per front; each CTA adds its 64 columns' share of a row with
-// one atomic.  (Grouping a CTA's work over several vectors was measured slower: fewer CTAs.)
-__global__ void __launch_bounds__(256) k_front_solve_tail(PlanDev P, const double* vals, int nrhs,
-                                                          double* y, int64_t ylen,
-                                                          const int32_t* __restrict__ fids,
-                                                          int which) {
-  constexpr int TC = 64;
-  __shared__ double xs[TC];
-  __shared__ long long pzs[TC];
-  const int f = fids[blockIdx.y];
-  const int s0 = P.fs0[f], w = P.fw[f];
-  const int x0 = blockIdx.x * TC;
-  if (x0 >= w) return;                              // the same for every thread of the CTA
-  const int nx = min(TC, w - x0);
-  const int64_t v = blockIdx.z;
-  const double* __restrict__ V = vals + (v / nrhs) * P.blob;
-  double* yv = y + v * ylen;
-  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp, nt = blockDim.x;
-  if (tid < nx) {
-    xs[tid] = yv[s0 + x0 + tid];
-    pzs[tid] = (long long)P.lp[s0 + x0 + tid] - (x0 + tid);   // row s0 in column s0 + x0 + tid
-  }
-  __syncthreads();
-  if (which == 0) {
-    const int64_t q0 = (int64_t)P.lp[s0] + w;       // the rows R in column s0
-    const int m = (int)((int64_t)P.cp[s0 + 1] - q0);
-    for (int i = tid; i < m; i += nt) {
-      double sum = 0.0;
-      for (int x = 0; x < nx; ++x) sum += V[pzs[x] + w + i] * xs[x];
-      atomicAdd(yv + P.ri[q0 + i], -sum);
-    }
-  } else {
-    for (int x = warp; x < nx; x += nt / kWarp) {
-      const double xx = xs[x];
-      for (int64_t p = P.cp[s0 + x0 + x] + lane; p < pzs[x]; p += kWarp)
-        atomicAdd(yv + P.ri[p], -(V[p] * xx));
     }
   }
 }
@@ -1399,45 +1152,21 @@ void launch_sparse_ltsolve(const PlanDev& P, const double* vals, int count, int 
   lc.n++;
 }
 
-void launch_front_solve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                        int64_t ylen, const int32_t* fids, int nfronts, int max_w, int which,
-                        cudaStream_t s, LaunchCounter& lc) {
-  if (nfronts <= 0) return;
-  const size_t fwp = ((size_t)P.fw_max + 63) / 64 * 64;
-  const size_t smem_blk = sizeof(double) * (2 * 64 * 64 + 64 + fwp) + sizeof(long long) * fwp;
-  if (which <= 1 && smem_blk <= 200 * 1024) {
-    // fronts wider than two blocks leave the rows outside the front to k_front_solve_tail;
-    // a level with a front of at least four blocks solves its fronts by clusters of CTAs
-    const bool split = max_w > 128;
-    const size_t smem_cl = sizeof(double) * (2 * 64 * 64 + 2 * 64 + fwp) + sizeof(long long) * fwp;
-    if (max_w >= 256 && smem_cl <= 200 * 1024) {
-      ensure_smem_limit((const void*)k_front_solve_cluster, smem_cl);
-      k_front_solve_cluster<<<dim3((unsigned)(nfronts * kFsC), (unsigned)(count * nrhs)), 256,
-                              smem_cl, s>>>(P, vals, nrhs, y, ylen, fids, which);
-    } else {
-      ensure_smem_limit((const void*)k_front_solve_blk, smem_blk);
-      k_front_solve_blk<<<dim3((unsigned)nfronts, (unsigned)(count * nrhs)), 256, smem_blk, s>>>(
-          P, vals, nrhs, y, ylen, fids, which, split ? 0 : 1);
-    }
+void launch_solve_level(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                        int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
+                        const FrontLevelSolve& L, int which, cudaStream_t s, LaunchCounter& lc) {
+  const int ncb = nlong + (ncols - nlong + 7) / 8;
+  if (ncb + L.next == 0) return;
+  const int4* ext = reinterpret_cast<const int4*>(L.ext);
+  const auto launch = [&](auto kern, int nv) {
+    kern<<<dim3(ncb + L.next, count * ((nrhs + nv - 1) / nv)), 256, 0, s>>>(
+        P, vals, nrhs, y, ylen, cols, begin, ncols, nlong, ncb, ext);
     lc.n++;
-    if (split) {
-      k_front_solve_tail<<<dim3((unsigned)((max_w + 63) / 64), (unsigned)nfronts,
-                                (unsigned)(count * nrhs)), 256, 0, s>>>(P, vals, nrhs, y, ylen,
-                                                                        fids, which);
-      lc.n++;
-    }
-    return;
-  }
-  const size_t smem = (2 * sizeof(double) + 2 * sizeof(uint32_t)) * (size_t)P.fw_max;
-  if (which <= 1 && smem <= 96 * 1024) {
-    ensure_smem_limit((const void*)k_front_solve_push, smem);
-    k_front_solve_push<<<dim3((unsigned)nfronts, (unsigned)(count * nrhs)), 256, smem, s>>>(
-        P, vals, nrhs, y, ylen, fids, which);
-  } else {
-    k_front_solve<<<dim3((unsigned)nfronts, (unsigned)(count * nrhs)), 256, 0, s>>>(
-        P, vals, nrhs, y, ylen, fids, which);
-  }
-  lc.n++;
+  };
+  if (which == 0) nrhs == 1 ? launch(k_solve_level<1, 0>, 1) : launch(k_solve_level<kSolveVecs, 0>, kSolveVecs);
+  if (which == 1) nrhs == 1 ? launch(k_solve_level<1, 1>, 1) : launch(k_solve_level<kSolveVecs, 1>, kSolveVecs);
+  if (which == 2) launch(k_solve_level<1, 2>, 1);
+  if (which == 3) launch(k_solve_level<1, 3>, 1);
 }
 
 void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, double* y,

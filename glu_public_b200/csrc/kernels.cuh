@@ -141,15 +141,29 @@ void launch_sparse_utsolve(const PlanDev& P, const double* vals, int count, int 
 void launch_sparse_ltsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                            int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                            cudaStream_t s, LaunchCounter& lc);
-// fronts fids[0 .. nfronts) of one solve level, every vector (which as in k_front_solve)
-// max_w: the widest of the fronts listed in fids (at least their width)
-void launch_front_solve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
-                        int64_t ylen, const int32_t* fids, int nfronts, int max_w, int which,
-                        cudaStream_t s, LaunchCounter& lc);
+// the fronts of one solve level: row blocks (two numbers each), fronts, and pieces of the products
+// with what lies outside them (four numbers each; see plan_host.h)
+struct FrontLevelSolve {
+  const int32_t* flow;
+  int nflow, nfronts;
+  const int32_t* ext;
+  int next;
+};
+// the rows of the level's fronts among themselves (which 0: L, 1: U, 2: U^T, 3: L^T), as the dense
+// block's solve (trsv.cu)
+void launch_front_flow(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                       int64_t ylen, const FrontLevelSolve& L, int which, double* xbuf, int* err,
+                       int32_t* status, double budget_ms, cudaStream_t s, LaunchCounter& lc);
+// the level's single columns (which 1: rows) and the outside products of its fronts, one launch
+void launch_solve_level(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                        int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
+                        const FrontLevelSolve& L, int which, cudaStream_t s, LaunchCounter& lc);
+// values a vector has in the solve's buffer of solved values
+__host__ __device__ inline int64_t solve_buffer(const PlanDev& P) { return 2 * ((int64_t)P.ntp + P.fx_len); }
 void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                    int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc);
 // L then U (transpose: U^T then L^T) of the dense block for every vector, one cooperative launch
-// (trsv.cu); xbuf, err: 2 ntp values a vector and the failure word, set up by
+// (trsv.cu); xbuf, err: solve_buffer values a vector and the failure word, set up by
 // launch_solve_permute_in; a wait of more than budget_ms marks the instances GLU_INST_TIMEOUT
 void launch_dense_solve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                         int64_t ylen, bool transpose, double* xbuf, int* err, int32_t* status,

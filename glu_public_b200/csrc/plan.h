@@ -65,9 +65,14 @@ struct PlanDev {
   const uint8_t* fhasl;              // pivot may be perturbed, per padded front pivot
   const int32_t* fs0;                // first column of every front
   const int32_t* fw;                 // width of every front
-  int32_t fw_max;                    // widest front
-  const int32_t* lfr;                // fronts in L-solve level order
-  const int32_t* ufr;                // fronts in U-solve level order
+  // fronts in the solves (see plan_host.h)
+  const int32_t *lflow, *uflow, *lext, *uext, *ldot, *udot;
+  const int64_t* fx0;                // [fronts]
+  int64_t fx_len;
+  const int64_t* uj_ptr;             // [fronts + 1]
+  const int32_t *uj_col, *uj_slot;
+  const int64_t* ur_ptr;             // [t + 1]
+  const int32_t *ur_col, *ur_slot, *ur_rows;
   const FrontGeom* fgeom;            // [fronts]
   const int32_t* fg_aidx;            // gather / write-back index within an instance's front area
   const int32_t* fc_aidx;            // Schur-complement index within an instance's front area

@@ -111,6 +111,95 @@ int32_t column_lanes(int32_t fixed, const uint32_t* cp, const uint32_t* lp,
   return best;
 }
 
+// The solve schedules of a plan with fronts: row blocks and outside products of every level's
+// fronts, and the rows of the single columns (the U solve pulls where there are fronts: every entry
+// above a front's block row is then part of a dense product instead of an atomic of its own).
+void build_front_solves(HostPlan& hp) {
+  constexpr int32_t kRows = 64, kCols = 256;
+  const int32_t nf = (int32_t)hp.fronts.size();
+  const uint32_t n = hp.n, t = hp.t;
+  const uint32_t *cp = hp.cp.data(), *ri = hp.ri.data(), *ci = hp.ci.data(), *dp = hp.dp.data();
+  hp.fx0.assign(nf, 0);
+  hp.fx_len = 0;
+  hp.uj_ptr.assign(nf + 1, 0);
+  hp.uj_col.clear();
+  hp.uj_slot.clear();
+  std::vector<uint8_t> in_front(t, 0);
+  for (int32_t f = 0; f < nf; ++f) {
+    const Front& F = hp.fronts[f];
+    hp.fx0[f] = hp.fx_len;
+    hp.fx_len += F.w;
+    for (int32_t x = 0; x < F.w; ++x) in_front[F.s0 + x] = 1;
+    const uint32_t* J = ci + dp[F.s0 + F.w - 1] + 1;
+    for (int32_t jj = 0; jj < F.q; ++jj) {
+      const uint32_t j = J[jj];
+      const uint32_t* p = std::lower_bound(ri + cp[j], ri + cp[j + 1], (uint32_t)F.s0);
+      hp.uj_col.push_back((int32_t)j);
+      hp.uj_slot.push_back((int32_t)hp.pos2slot[p - ri]);
+    }
+    hp.uj_ptr[f + 1] = (int64_t)hp.uj_col.size();
+  }
+  auto lists = [&](const std::vector<int32_t>& fr, const std::vector<int32_t>& frptr, bool lower,
+                   std::vector<int32_t>& flow, std::vector<int32_t>& flow_ptr,
+                   std::vector<int32_t>& ext, std::vector<int32_t>& ext_ptr,
+                   std::vector<int32_t>& dot, std::vector<int32_t>& dot_ptr) {
+    flow.clear();
+    ext.clear();
+    dot.clear();
+    flow_ptr.assign(1, 0);
+    ext_ptr.assign(1, 0);
+    dot_ptr.assign(1, 0);
+    for (size_t l = 0; l + 1 < frptr.size(); ++l) {
+      int32_t wmax = 0;
+      for (int32_t k = frptr[l]; k < frptr[l + 1]; ++k) wmax = std::max(wmax, hp.fw[fr[k]]);
+      for (int32_t o = 0; o * kRows < wmax; ++o)
+        for (int32_t k = frptr[l]; k < frptr[l + 1]; ++k)
+          if (o * kRows < hp.fw[fr[k]]) {
+            flow.push_back(fr[k]);
+            flow.push_back(o);
+          }
+      for (int32_t k = frptr[l]; k < frptr[l + 1]; ++k) {
+        const Front& F = hp.fronts[fr[k]];
+        const int32_t rows = lower ? F.m : F.w, cols = lower ? F.w : F.q;
+        for (int32_t r = 0; r < rows; r += kRows)
+          for (int32_t c = 0; c < cols; c += kCols)
+            for (int32_t v : {fr[k], r, c, 0}) ext.push_back(v);
+        for (int32_t x = 0; x < F.w; x += 8)
+          for (int32_t v : {fr[k], x, 0, 0}) dot.push_back(v);
+      }
+      flow_ptr.push_back((int32_t)(flow.size() / 2));
+      ext_ptr.push_back((int32_t)(ext.size() / 4));
+      dot_ptr.push_back((int32_t)(dot.size() / 4));
+    }
+  };
+  lists(hp.lfr, hp.lfr_ptr, true, hp.lflow, hp.lflow_ptr, hp.lext, hp.lext_ptr, hp.ldot, hp.ldot_ptr);
+  lists(hp.ufr, hp.ufr_ptr, false, hp.uflow, hp.uflow_ptr, hp.uext, hp.uext_ptr, hp.udot,
+        hp.udot_ptr);
+  // rows of the single columns
+  hp.ur_ptr.assign((size_t)t + 1, 0);
+  for (uint32_t j = 0; j < n; ++j)
+    for (uint32_t p = cp[j]; p < cp[j + 1] && ri[p] < j && ri[p] < t; ++p)
+      if (!in_front[ri[p]]) hp.ur_ptr[ri[p] + 1]++;
+  for (uint32_t r = 0; r < t; ++r) hp.ur_ptr[r + 1] += hp.ur_ptr[r];
+  hp.ur_col.assign(hp.ur_ptr[t], 0);
+  hp.ur_slot.assign(hp.ur_ptr[t], 0);
+  std::vector<int64_t> at(hp.ur_ptr.begin(), hp.ur_ptr.end() - 1);
+  for (uint32_t j = 0; j < n; ++j)
+    for (uint32_t p = cp[j]; p < cp[j + 1] && ri[p] < j && ri[p] < t; ++p)
+      if (!in_front[ri[p]]) {
+        hp.ur_col[at[ri[p]]] = (int32_t)j;
+        hp.ur_slot[at[ri[p]]++] = (int32_t)hp.pos2slot[p];
+      }
+  hp.ur_rows = hp.ucols;
+  hp.ur_long.assign(hp.ulng.size(), 0);
+  for (size_t l = 0; l + 1 < hp.uptr.size(); ++l) {
+    auto mid = std::stable_partition(
+        hp.ur_rows.begin() + hp.uptr[l], hp.ur_rows.begin() + hp.uptr[l + 1],
+        [&](int32_t r) { return hp.ur_ptr[r + 1] - hp.ur_ptr[r] >= (int64_t)kSolveLong; });
+    hp.ur_long[l] = (int32_t)(mid - (hp.ur_rows.begin() + hp.uptr[l]));
+  }
+}
+
 }  // namespace
 
 int build_host_plan(uint32_t n, uint32_t nnz, const uint32_t* cp, const uint32_t* ri,
@@ -710,6 +799,7 @@ int build_host_plan(uint32_t n, uint32_t nnz, const uint32_t* cp, const uint32_t
     build(true, hp.lcols, hp.lptr, hp.lfr, hp.lfr_ptr, hp.llong);
     build(false, hp.ucols, hp.uptr, hp.ufr, hp.ufr_ptr, hp.ulng);
   }
+  if (!hp.fronts.empty()) build_front_solves(hp);
   hp.bord_ptr.assign((size_t)hp.nt + 1, 0);
   hp.bord_row.clear();
   hp.bord_slot.clear();

@@ -100,6 +100,21 @@ struct HostPlan {
   // fronts in the solve schedules: level l runs fronts lfr[lfr_ptr[l] .. lfr_ptr[l+1])
   std::vector<int32_t> lfr, lfr_ptr, ufr, ufr_ptr;
   std::vector<int32_t> fs0, fw;               // first column and width of every front
+  // fronts in the solves (kernels in trsv.cu): the row blocks of a level's fronts {front, order}
+  // of the block in its front's chain, all fronts' first blocks first; and, four numbers each, the
+  // pieces of the products with what lies outside the fronts of a level -- L: {front, first row
+  // of R, first column}; U: {front, first row, first column of J}; transposed: {front, first of 8
+  // columns}
+  std::vector<int32_t> lflow, uflow, lext, uext, ldot, udot;
+  std::vector<int32_t> lflow_ptr, uflow_ptr, lext_ptr, uext_ptr, ldot_ptr, udot_ptr;
+  std::vector<int64_t> fx0;                   // place of a front's values in the solve's buffer
+  int64_t fx_len = 0;                         // columns of all fronts
+  std::vector<int64_t> uj_ptr;                // columns J right of each front: index and slot of
+  std::vector<int32_t> uj_col, uj_slot;       //   the front's first row in each
+  // rows of single columns: entries right of the diagonal, and the rows in U-solve level order,
+  // rows of at least kSolveLong entries first
+  std::vector<int64_t> ur_ptr;
+  std::vector<int32_t> ur_col, ur_slot, ur_rows, ur_long;
   std::vector<int64_t> bord_ptr;
   std::vector<int32_t> bord_row, bord_slot;
   std::vector<int32_t> bord_ckcol;            // chunks of <= 1024 border entries: tail column

@@ -25,6 +25,9 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "glu_b200.h"
 #include "kernels.cuh"
@@ -284,7 +287,8 @@ __device__ bool flow_phase(const double* __restrict__ D, int64_t ld, int nblk, c
   return true;
 }
 
-// Grid: groups of G CTAs; group g takes units g, g + groups, ...  xbuf: 2 ntp values a vector.
+// Grid: groups of G CTAs; group g takes units g, g + groups, ...  xbuf: solve_buffer values a
+// vector, the dense block's first.
 template <int NV, bool TRANS>
 __global__ void __launch_bounds__(256, NV * (TRANS ? 2 : 1) >= 8 ? 1 : 2)
     k_dense_flow(PlanDev P, const double* vals, int count, int nrhs, double* y, int64_t ylen,
@@ -293,7 +297,7 @@ __global__ void __launch_bounds__(256, NV * (TRANS ? 2 : 1) >= 8 ? 1 : 2)
   const int chunks = (nrhs + NV - 1) / NV;
   const int units = count * chunks, groups = gridDim.x / G;
   const int r = blockIdx.x % G, nblk = (int)(P.ntp / kB);
-  const int64_t xl = 2 * (int64_t)P.ntp;
+  const int64_t xl = solve_buffer(P);
   for (int u = blockIdx.x / G; u < units; u += groups) {
     const int inst = u / chunks, v0 = (u % chunks) * NV;
     const int nv = min(NV, nrhs - v0);
@@ -315,17 +319,30 @@ __global__ void __launch_bounds__(256, NV * (TRANS ? 2 : 1) >= 8 ? 1 : 2)
   }
 }
 
+// CTAs of a kernel that fit on the current device at once (cached per kernel and device).
+int flow_capacity(const void* kern, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  int& cap = known[{kern, dev}];
+  if (cap == 0) {
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, smem) != cudaSuccess)
+      cudaGetLastError();
+    cap = std::max(1, per_sm) * sm_count();
+  }
+  return cap;
+}
+
 template <int NV, bool TRANS>
-bool flow_launch(const PlanDev& P, const double* vals, int count, int nrhs, double* y, int64_t ylen,
+void flow_launch(const PlanDev& P, const double* vals, int count, int nrhs, double* y, int64_t ylen,
                  double* xbuf, int* err, int32_t* status, double budget_ms, cudaStream_t s,
                  LaunchCounter& lc) {
   const auto kern = k_dense_flow<NV, TRANS>;
   ensure_smem_limit((const void*)kern, flow_smem<NV>());
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, flow_smem<NV>()) !=
-          cudaSuccess || per_sm < 1)
-    return false;
-  const int cap = per_sm * sm_count(), nblk = (int)(P.ntp / kB);
+  const int cap = flow_capacity((const void*)kern, flow_smem<NV>()), nblk = (int)(P.ntp / kB);
   // the vectors' units share the CTAs that fit on the device: all of a block's rows in flight for
   // a few vectors, down to one CTA walking the blocks of each of many
   const int64_t units = (int64_t)count * ((nrhs + NV - 1) / NV);
@@ -344,7 +361,238 @@ bool flow_launch(const PlanDev& P, const double* vals, int count, int nrhs, doub
   cudaLaunchKernelEx(&cfg, kern, P, vals, count, nrhs, y, ylen, G, xbuf, err, status,
                      (unsigned long long)(budget_ms * 1e6));
   lc.n++;
+}
+
+// ---------------------------------------------------------------------------------------------
+// fronts
+// ---------------------------------------------------------------------------------------------
+
+// Row block `o` (in the order of the phase) of front f for nv vectors: the body of flow_phase with
+// the front's own columns, whose rows lie contiguously in the value slots (row i of column x at
+// lp[s0 + x] - x + i), and bounds for a last block that is not full.
+template <int NV, int WHICH>
+__device__ bool front_block(const PlanDev& P, const double* __restrict__ V, int f, int o, double* y,
+                            int64_t yl, double* xb, int64_t xl, int nv, int* err,
+                            unsigned long long budget_ns, double* sm) {
+  constexpr bool fwd = WHICH == 0 || WHICH == 2;
+  constexpr bool trans = WHICH >= 2;
+  constexpr bool diag = WHICH == 1 || WHICH == 2;
+  constexpr int NX = (kB * NV + 255) / 256;
+  double* Ds = sm;
+  double* xs = Ds + kB * kDs;                 // [2][kB][NV]
+  double* red = xs + 2 * kB * NV;             // [4][NV][kB]
+  double* rc = red + 4 * NV * kB;
+  const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
+  const int vec = warp % NV;
+  const int s0 = P.fs0[f], w = P.fw[f], nblk = (w + kB - 1) / kB;
+  const int b = (fwd ? o : nblk - 1 - o) * kB;
+  const uint32_t* __restrict__ lp = P.lp + s0;
+  auto at = [&](int i, int x) { return V + ((int64_t)lp[x] - x + i); };
+  for (int e = tid; e < kB * kB; e += 256) {
+    const int i = b + e % kB, j = b + e / kB;
+    const bool ok = i < w && j < w;
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(Ds + e % kB + (e / kB) * kDs);
+    const double* src = ok ? at(i, j) : V;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src),
+                 "r"(ok ? 8 : 0));
+  }
+  asm volatile("cp.async.commit_group;\n" ::);
+  double m[16], xn[NX];
+  auto fetch = [&](int k) {
+    const int kb = (fwd ? k : nblk - 1 - k) * kB;
+    if (!trans) {
+      const int i = b + (tid & 63);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        const int x = kb + (tid >> 6) * 16 + q;
+        m[q] = i < w && x < w ? *at(i, x) : 0.0;
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int x = b + warp * 8 + q;
+        m[2 * q] = x < w && kb + lane < w ? *at(kb + lane, x) : 0.0;
+        m[2 * q + 1] = x < w && kb + lane + 32 < w ? *at(kb + lane + 32, x) : 0.0;
+      }
+    }
+  };
+  // the place of value e of solved block k in the front's values, -1 past them
+  auto place = [&](int k, int e) {
+    const int i = (fwd ? k : nblk - 1 - k) * kB + e % kB;
+    return i < w ? i : -1;
+  };
+  auto look = [&](int k) {
+#pragma unroll
+    for (int h = 0; h < NX; ++h) {
+      const int e = tid + h * 256, i = e < kB * NV ? place(k, e) : -1;
+      xn[h] = i >= 0 ? ld_relaxed(xb + (int64_t)min(e / kB, nv - 1) * xl + i) : 0.0;
+    }
+  };
+  if (o > 0) {
+    fetch(0);
+    look(0);
+  }
+  double* yv = y + (int64_t)min(vec, nv - 1) * yl + s0;
+  double y0 = b + lane < w ? yv[b + lane] : 0.0;
+  double y1 = b + lane + 32 < w ? yv[b + lane + 32] : 0.0;
+  double acc[trans ? 8 * NV : NV];
+#pragma unroll
+  for (int i = 0; i < (trans ? 8 * NV : NV); ++i) acc[i] = 0.0;
+  int fail = 0;
+  bool plain = true;
+  auto finish_stage = [&]() {
+    asm volatile("cp.async.wait_group 0;\n" ::);
+    __syncthreads();
+    bool odd = false;
+    if (tid < kB) {
+      if (b + tid >= w) Ds[tid * (kDs + 1)] = 1.0;   // padding: identity
+      const double d = Ds[tid * (kDs + 1)];
+      if (diag) rc[tid] = 1.0 / d;
+      const int ex = (__double2hiint(d) >> 20) & 0x7ff;
+      odd = ex < 64 || ex > 0x7ff - 64;
+    }
+    if (diag) {
+      plain = !__syncthreads_or(odd);
+      if (plain)
+        for (int e = tid; e < kB * kB; e += 256) {
+          const int i = e % kB, j = e / kB, d = trans ? j : i;
+          if (i < j) Ds[i + j * kDs] = quotient_r(Ds[i + j * kDs], Ds[d * (kDs + 1)], rc[d]);
+        }
+    }
+  };
+  for (int k = 0; k < o; ++k) {
+    if (k == o - 1) finish_stage();
+    double* x = xs + (k & 1) * kB * NV;
+#pragma unroll
+    for (int h = 0; h < NX; ++h) {
+      const int e = tid + h * 256;
+      if (e < kB * NV) {
+        const int i = place(k, e);
+        x[(e % kB) * NV + e / kB] =
+            i < 0 ? 0.0
+                  : wait_value(xb + (int64_t)min(e / kB, nv - 1) * xl + i, xn[h], err, budget_ns,
+                               &fail);
+      }
+    }
+    if (__syncthreads_or(fail)) return false;
+    if (k + 1 < o) look(k + 1);
+    if (!trans) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) acc[v] += m[q] * x[((tid >> 6) * 16 + q) * NV + v];
+    } else {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const double x0 = x[lane * NV + v], x1 = x[(lane + 32) * NV + v];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[q * NV + v] += m[2 * q] * x0 + m[2 * q + 1] * x1;
+      }
+    }
+    if (k + 1 < o) fetch(k + 1);
+  }
+  if (o == 0) finish_stage();
+  if (!trans) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) red[((tid >> 6) * NV + v) * kB + (tid & 63)] = acc[v];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8 * NV; ++i) {
+      double t = acc[i];
+      for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+      if (lane == 0) red[(i % NV) * kB + warp * 8 + i / NV] = t;
+    }
+  }
+  __syncthreads();
+  double t0 = 0.0, t1 = 0.0;
+#pragma unroll
+  for (int q = 0; q < (trans ? 1 : 4); ++q) {
+    t0 += red[(q * NV + vec) * kB + lane];
+    t1 += red[(q * NV + vec) * kB + lane + 32];
+  }
+  y0 -= t0;
+  y1 -= t1;
+  if (!diag) {
+    triangle<WHICH, false>(Ds, rc, lane, y0, y1);
+  } else if (plain) {
+    y0 = quotient_r(y0, Ds[lane * (kDs + 1)], rc[lane]);
+    y1 = quotient_r(y1, Ds[(lane + 32) * (kDs + 1)], rc[lane + 32]);
+    triangle<WHICH, false>(Ds, rc, lane, y0, y1);
+  } else {
+    triangle<WHICH, true>(Ds, rc, lane, y0, y1);
+  }
+  if (warp < nv) {
+    double* xo = xb + vec * xl + b;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int i = lane + 32 * h;
+      const double v = h ? y1 : y0;
+      if (b + i < w) {
+        if (o + 1 < nblk) st_relaxed(xo + i, unsolved(v) ? __longlong_as_double(kNaN) : v);
+        yv[b + i] = v;
+      }
+    }
+  }
+  __syncthreads();                            // smem reuse by the next block
   return true;
+}
+
+// The rows of a level's fronts among themselves: items {front, order of the row block}, every
+// front's earlier blocks before its later ones, each for every unit (an instance and up to NV of
+// its right-hand sides).  A CTA takes items in increasing order, and an item waits only for lower
+// ones, so with every CTA resident (a cooperative launch wherever a front has two blocks) the
+// lowest unfinished item can always go on.
+// Bound by latency as the dense block's solve.  Measured, 512 x 512 x 2 nodes, 4 vectors: 11 us per L
+// level and 17 us per U level (wider fronts), where one CTA per front took 30 us a level and a
+// cluster of eight 116 us for the wide ones.
+template <int NV, int WHICH>
+__global__ void __launch_bounds__(256, NV * (WHICH >= 2 ? 2 : 1) >= 8 ? 1 : 2)
+    k_front_flow(PlanDev P, const double* vals, int count, int nrhs, double* y, int64_t ylen,
+                 const int2* __restrict__ items, int nitems, double* xbuf, int* err,
+                 int32_t* status, unsigned long long budget_ns) {
+  extern __shared__ double sm[];
+  const int chunks = (nrhs + NV - 1) / NV;
+  const int64_t units = (int64_t)count * chunks;
+  const int64_t xl = solve_buffer(P);
+  double* xf = xbuf + 2 * (int64_t)P.ntp + (WHICH == 1 || WHICH == 3 ? P.fx_len : 0);
+  for (int64_t it = blockIdx.x; it < nitems * units; it += gridDim.x) {
+    const int2 item = items[it / units];
+    const int u = (int)(it % units), inst = u / chunks, v0 = (u % chunks) * NV;
+    const int64_t vec = (int64_t)inst * nrhs + v0;
+    if (!front_block<NV, WHICH>(P, vals + (int64_t)inst * P.blob, item.x, item.y, y + vec * ylen,
+                                ylen, xf + vec * xl + P.fx0[item.x], xl, min(NV, nrhs - v0), err,
+                                budget_ns, sm)) {
+      if (threadIdx.x == 0) atomicOr(status + inst, GLU_INST_TIMEOUT);
+      return;
+    }
+  }
+}
+
+template <int NV, int WHICH>
+void front_launch(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                  int64_t ylen, const FrontLevelSolve& L, double* xbuf, int* err, int32_t* status,
+                  double budget_ms, cudaStream_t s, LaunchCounter& lc) {
+  const auto kern = k_front_flow<NV, WHICH>;
+  ensure_smem_limit((const void*)kern, flow_smem<NV>());
+  const int64_t total = (int64_t)L.nflow * count * ((nrhs + NV - 1) / NV);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3((unsigned)total);
+  if (L.nflow > L.nfronts) {                  // some front has blocks that wait
+    const int cap = flow_capacity((const void*)kern, flow_smem<NV>());
+    cfg.gridDim = dim3((unsigned)std::min<int64_t>(total, std::max(cap, 1)));
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = flow_smem<NV>();
+  cfg.stream = s;
+  cudaLaunchKernelEx(&cfg, kern, P, vals, count, nrhs, y, ylen,
+                     reinterpret_cast<const int2*>(L.flow), L.nflow, xbuf, err, status,
+                     (unsigned long long)(budget_ms * 1e6));
+  lc.n++;
 }
 
 }  // namespace
@@ -366,6 +614,26 @@ void launch_dense_solve(const PlanDev& P, const double* vals, int count, int nrh
     else GLU_FLOW(4, true);
   }
 #undef GLU_FLOW
+}
+
+void launch_front_flow(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                       int64_t ylen, const FrontLevelSolve& L, int which, double* xbuf, int* err,
+                       int32_t* status, double budget_ms, cudaStream_t s, LaunchCounter& lc) {
+  if (L.nflow == 0) return;
+#define GLU_FRONT(NV, W) \
+  front_launch<NV, W>(P, vals, count, nrhs, y, ylen, L, xbuf, err, status, budget_ms, s, lc)
+#define GLU_FRONT_NV(W)                      \
+  if (nrhs == 1) GLU_FRONT(1, W);            \
+  else if (nrhs == 2) GLU_FRONT(2, W);       \
+  else GLU_FRONT(4, W);
+  switch (which) {
+    case 0: GLU_FRONT_NV(0) break;
+    case 1: GLU_FRONT_NV(1) break;
+    case 2: GLU_FRONT_NV(2) break;
+    default: GLU_FRONT_NV(3) break;
+  }
+#undef GLU_FRONT_NV
+#undef GLU_FRONT
 }
 
 }  // namespace glu
