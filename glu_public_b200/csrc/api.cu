@@ -647,6 +647,7 @@ int glu_plan_create(uint32_t n, uint32_t nnz, const uint32_t* sym_c_ptr,
   std::vector<uint8_t> dh = hp.dhasl;
   if ((st = p->upload(hp.cp, &P.cp)) || (st = p->upload(hp.ri, &P.ri)) ||
       (st = p->upload(hp.lp, &P.lp)) || (st = p->upload(hp.lsplit, &P.lsplit)) ||
+      (st = p->upload(hp.usplit, &P.usplit)) ||
       (st = p->upload(hp.pair_ptr, &P.pair_ptr)) || (st = p->upload(hp.pair_j, &P.pair_j)) ||
       (st = p->upload(hp.pair_uslot, &P.pair_uslot)) ||
       (st = p->upload(hp.pair_moff, &P.pair_moff)) || (st = p->upload(hp.tmap, &P.tmap)) ||

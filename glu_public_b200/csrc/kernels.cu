@@ -140,6 +140,84 @@ __device__ __forceinline__ ColGroup cta_group() {
                   (int)(blockDim.x / kWarp), -1, (int)(threadIdx.x % kWarp), kWarp, 0xffffffffu};
 }
 
+// The pairs (c, j) of one column applied by group w of W groups of `width` lanes (8, 16 or 32;
+// `mask`) of which this is lane `il`: column j of each pair takes -L(:,c) * U(c,j) through the
+// position map (src/numeric.cu:51-89); rows >= t of a tail column j belong to the dense block and
+// are applied afterwards by the hub GEMM and the per-column pull, so a pair with j >= t has only
+// nsplit updates and one with j < t has nL.
+// What bounds this is the latency of dependent loads (pair, then U value and map entry, then the
+// atomic) and, in the columns next to the dense block, a few pairs of thousands of updates among
+// thousands of a dozen.  So fewer long pairs than groups are shared in pieces of 4 * width updates;
+// of the others the lanes fetch the data `width` pairs at a time and the map entries of four pairs are in
+// flight together, with one load of the L value for the four.
+// Measured, sparse levels of one refactorization: n = 20,000 1.13 -> 0.39 ms (a few pairs of 2,860
+// updates in columns of 2,850 pairs), 512 x 512 x 2 nodes 9.4 -> 6.8 ms, 64 x n = 20,000 5.6 -> 3.0 ms;
+// sharing long pairs in pieces wherever there are fewer than groups, not a quarter as many: 128 x 128
+// x 2 nodes 2.15 ms against 1.88.
+__device__ __forceinline__ void apply_pairs(const PlanDev& P, double* __restrict__ V, uint32_t c,
+                                            const double* __restrict__ Lc, uint32_t nL, int64_t w,
+                                            int64_t W, int il, int width, unsigned mask) {
+  const uint32_t nsplit = P.lsplit[c];
+  int64_t q0 = P.pair_ptr[c];
+  const int64_t q1 = P.pair_ptr[c + 1];
+  const int64_t na = P.usplit[c];              // pairs with j < t, the first ones
+  if (4 * na < W && nL > 2 * (uint32_t)width) {  // they would leave most groups without one
+    const uint32_t piece = 4 * width, np = (nL + piece - 1) / piece;
+    for (int64_t e = w; e < na * np; e += W) {
+      const int64_t q = q0 + e / np;
+      const uint32_t k0 = (uint32_t)(e % np) * piece + il;
+      const int32_t* __restrict__ tm = P.tmap + P.pair_moff[q];
+      const double u = V[P.pair_uslot[q]];
+      int32_t t[4];
+      double l[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const uint32_t k = k0 + h * width;
+        t[h] = k < nL ? tm[k] : -1;
+        l[h] = k < nL ? Lc[k] : 0.0;
+      }
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        if (t[h] >= 0) atomicAdd(V + t[h], -(l[h] * u));
+    }
+    q0 += na;
+  }
+  for (int64_t q = q0 + w; q < q1; q += W * width) {
+    const int64_t mine = q + W * il;
+    uint32_t nsp = 0;
+    int64_t mo = 0;
+    double u = 0.0;
+    if (mine < q1) {
+      nsp = (uint32_t)P.pair_j[mine] < P.t ? nL : nsplit;
+      mo = P.pair_moff[mine];
+      u = V[P.pair_uslot[mine]];
+    }
+    const int n = (int)min((int64_t)width, (q1 - q + W - 1) / W);
+    for (int i = 0; i < n; i += 4) {
+      const int32_t* tm[4];
+      uint32_t ns[4], most = 0;
+      double us[4];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {            // lanes past n hold nsp = 0
+        const int src = min(i + h, width - 1);
+        ns[h] = i + h < n ? __shfl_sync(mask, nsp, src, width) : 0u;
+        tm[h] = P.tmap + __shfl_sync(mask, mo, src, width);
+        us[h] = __shfl_sync(mask, u, src, width);
+        most = max(most, ns[h]);
+      }
+      for (uint32_t k = il; k < most; k += width) {
+        const double l = Lc[k];
+        int32_t t[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) t[h] = k < ns[h] ? tm[h][k] : -1;
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (t[h] >= 0) atomicAdd(V + t[h], -(l * us[h]));
+      }
+    }
+  }
+}
+
 // One column c of a sparse level for instance b, by the threads of group g (their warps split the
 // U(c,:) pairs): pivot (perturbed if |d| < pert and the column has an L part,
 // src/numeric.cu:139-140), L(:,c) /= d (src/numeric.cu:37-47), then for every U(c,j) != 0 the
@@ -174,17 +252,7 @@ __device__ __forceinline__ void sparse_column(const PlanDev& P, double* __restri
 
   if (SCALE_ONLY) return;
   const double* __restrict__ Lc = Ls ? Ls : V + l0;
-  const int64_t q1 = P.pair_ptr[c + 1];
-  const uint32_t nsplit = P.lsplit[c];
-  for (int64_t q = P.pair_ptr[c] + g.wig; q < q1; q += g.nwg) {
-    const uint32_t j = (uint32_t)P.pair_j[q];
-    const double u = V[P.pair_uslot[q]];
-    const int32_t* __restrict__ tm = P.tmap + P.pair_moff[q];
-    // rows >= t of a tail column j belong to the dense block: they are applied afterwards by
-    // the hub GEMM and the per-column pull, so only sparse targets are touched here
-    const uint32_t nsp = j < P.t ? nL : nsplit;
-    for (uint32_t k = g.ilane; k < nsp; k += g.istride) atomicAdd(V + tm[k], -(Lc[k] * u));
-  }
+  apply_pairs(P, V, c, Lc, nL, g.wig, g.nwg, g.ilane, g.istride, g.mask);
 }
 
 // Part `part` of `splits` of column c's pairs (c, j), by the whole CTA: L(:,c) = A(:,c) / d is
@@ -202,17 +270,17 @@ __device__ __forceinline__ void sparse_split_part(const PlanDev& P, double* __re
   const double d0 = V[dslot];
   const double d = (pv > 0.0 && nL > 0 && fabs(d0) < pv) ? pv : d0;   // numeric.cu:139-140
   __syncthreads();                             // Ls may still be read by the previous item
-  for (uint32_t k = threadIdx.x; k < nL; k += blockDim.x) Ls[k] = V[l0 + k] / d;
-  __syncthreads();
-  const int64_t q1 = P.pair_ptr[c + 1];
-  const uint32_t nsplit = P.lsplit[c];
-  for (int64_t q = P.pair_ptr[c] + part * nwg + wig; q < q1; q += (int64_t)splits * nwg) {
-    const uint32_t j = (uint32_t)P.pair_j[q];
-    const double u = V[P.pair_uslot[q]];
-    const int32_t* __restrict__ tm = P.tmap + P.pair_moff[q];
-    const uint32_t nsp = j < P.t ? nL : nsplit;
-    for (uint32_t k = lane; k < nsp; k += kWarp) atomicAdd(V + tm[k], -(Ls[k] * u));
+  for (uint32_t k = threadIdx.x; k < nL; k += 4 * blockDim.x) {
+    double a[4];                               // four loads in flight
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      a[h] = k + h * blockDim.x < nL ? V[l0 + k + h * blockDim.x] : 0.0;
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (k + h * blockDim.x < nL) Ls[k + h * blockDim.x] = a[h] / d;
   }
+  __syncthreads();
+  apply_pairs(P, V, c, Ls, nL, part * nwg + wig, (int64_t)splits * nwg, lane, kWarp, 0xffffffffu);
 }
 
 // One launch per sparse level: groups of `wpc` warps share a column (wpc = 1: a warp per

@@ -34,6 +34,7 @@ struct PlanDev {
   const uint32_t* ri;                // sym_r_idx [nnz]
   const uint32_t* lp;                // l_col_ptr [n]
   const uint32_t* lsplit;            // [t] number of L(:,c) rows < t
+  const uint32_t* usplit;            // [t] number of U(c,:) columns < t
   const int64_t* pair_ptr;           // [t+1] range of U(c,:) pairs of column c
   const int32_t* pair_j;             // [npairs] column j of U(c,j)
   const int32_t* pair_uslot;         // [npairs] slot of U(c,j)

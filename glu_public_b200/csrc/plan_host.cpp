@@ -266,11 +266,13 @@ int build_host_plan(uint32_t n, uint32_t nnz, const uint32_t* cp, const uint32_t
 
   // ---- sparse columns: L split, (c, j) pairs and target-slot runs ----
   hp.lsplit.assign(t, 0);
+  hp.usplit.assign(t, 0);
   hp.pair_ptr.assign((size_t)t + 1, 0);
   for (uint32_t c = 0; c < t; ++c) {
     uint32_t k = lp[c] + 1;
     while (k < cp[c + 1] && ri[k] < t) ++k;
     hp.lsplit[c] = k - (lp[c] + 1);
+    hp.usplit[c] = (uint32_t)(std::lower_bound(ci + dp[c] + 1, ci + rp[c + 1], t) - (ci + dp[c] + 1));
     hp.pair_ptr[c + 1] = hp.pair_ptr[c] + (rp[c + 1] - dp[c] - 1);
   }
   const int64_t npairs = hp.pair_ptr[t];

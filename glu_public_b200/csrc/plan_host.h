@@ -66,7 +66,7 @@ struct HostPlan {
   int32_t level_warps = 64;                  // warps per SM the sparse level launches aim for
   int32_t cols_per_warp = 1;                 // columns a warp group takes in turn
   std::vector<uint32_t> cp, ri, lp, rp, ci, dp;
-  std::vector<uint32_t> lsplit;
+  std::vector<uint32_t> lsplit, usplit;
   std::vector<int64_t> pair_ptr;
   std::vector<int32_t> pair_j, pair_uslot;
   std::vector<int64_t> pair_moff;

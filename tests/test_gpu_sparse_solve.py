@@ -7,6 +7,7 @@ import pytest
 
 from glu_public_b200 import glu
 from tests.test_gpu_dense_solve import check_solve
+from tests.test_gpu_dense_steps import check_lu
 
 pytestmark = pytest.mark.gpu
 LENGTHS = (1, 31, 33, 64, 65, 128, 191, 192, 193, 500)
@@ -55,3 +56,33 @@ def test_long_columns(nrhs, transpose, deterministic):
         nl = np.diff(cp) - (sym.l_col_ptr.astype(np.int64) - cp[:-1]) - 1
         assert nl.max() >= 192 and (nl < 192).any()
         check_solve(torch, lu, b[i], x[i], transpose)
+
+
+@pytest.mark.parametrize("options", [{}, dict(sparse_persistent=0), dict(sparse_persistent=0, level_warps_per_sm=0),
+                                     dict(sparse_warps_per_col=1, sparse_col_lanes=8),
+                                     dict(sparse_warps_per_col=1, sparse_col_lanes=16, sparse_persistent=0),
+                                     dict(sparse_warps_per_col=8, sparse_persistent=0),
+                                     dict(sparse_warps_per_col=2, sparse_persistent=0),
+                                     dict(dense_threshold=0.5)])
+def test_long_and_short_pairs(options):
+    """Factors of columns with few long pairs, many short ones and both (pairs of a column shared in
+    pieces or four at a time), |L U - A| <= 4 n u |L| |U|."""
+    import torch
+    n = 1100
+    a = long_columns(n, 3)
+    a[40, 600:] = -0.01                       # long rows of U: many pairs of short columns
+    a[41, 41:90] = 0.02
+    a[500:900, 41] = 0.03                     # few long pairs
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, **{"dense_threshold": 2.0, "front_min_w": 0, **options})
+    batch = glu.Batch(plan, 3)
+    batch.load_lu_values(torch.as_tensor(np.stack([sym.val * s for s in (1.0, 2.0, -1.0)]),
+                                         device="cuda"))
+    batch.refactor(0.0)
+    cp = sym.sym_c_ptr.astype(np.int64)
+    for i, s in enumerate((1.0, 2.0, -1.0)):
+        lu = np.zeros((n, n))                 # [column, row]
+        lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
+        check_lu(torch, lu, np.ascontiguousarray(a.T * s)[None])
