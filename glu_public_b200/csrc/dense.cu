@@ -37,6 +37,7 @@
 #include "glu_b200.h"
 #include "kernels.cuh"
 #include "plan_host.h"
+#include "wait.cuh"
 
 namespace glu {
 
@@ -328,6 +329,7 @@ __device__ __forceinline__ void diag64_body(const DenseView& V, const double* __
 
 __global__ void __launch_bounds__(256) k_dense_diag64(DenseView V, const double* __restrict__ pert,
                                                       int32_t* status, int k) {
+  after_previous();
   diag64_body(V, pert, status, k, blockIdx.x);
 }
 
@@ -342,6 +344,7 @@ __device__ __forceinline__ DenseView front_view(const PlanDev& P, const FrontGeo
 __global__ void __launch_bounds__(256) k_front_diag(PlanDev P, double* F, int64_t fstride, int f0,
                                                   const double* __restrict__ pert,
                                                   int32_t* status, int k) {
+  after_previous();
   const FrontGeom g = P.fgeom[f0 + blockIdx.y];
   if (k >= g.w) return;
   diag64_body(front_view(P, g, F, fstride), pert, status, k, blockIdx.x);
@@ -949,12 +952,14 @@ __device__ __forceinline__ void trsm8_body(const DenseView& V, int k, int mt, in
 constexpr int kTrsm8Smem = (2 * 64 * 68 + 64) * 8;
 
 __global__ void __launch_bounds__(256) k_dense_trsm8(DenseView V, int k, int mt) {
+  after_previous();
   trsm8_body(V, k, mt, blockIdx.x, blockIdx.y);
 }
 
 // The same at pivot k of the fronts of a level: grid (most tiles of a front, fronts * count).
 __global__ void __launch_bounds__(256) k_front_trsm8(PlanDev P, double* F, int64_t fstride, int f0,
                                                      int count, int k) {
+  after_previous();
   const FrontGeom g = P.fgeom[f0 + blockIdx.y / count];
   if (k >= g.w) return;
   const int mt = (g.ld - k - 64) / 64, nt = (g.cols - k - 64) / 64;
@@ -1080,6 +1085,7 @@ constexpr int kStepSmem = 2 * 64 * 68 * 8;
 
 __global__ void __launch_bounds__(256) k_dense_step(DenseView V, const double* __restrict__ pert,
                                                     int32_t* status, int k, int wide) {
+  after_previous();
   step_body(V, pert, status, k, wide, blockIdx.x, blockIdx.y);
 }
 
@@ -1088,6 +1094,7 @@ __global__ void __launch_bounds__(256) k_dense_step(DenseView V, const double* _
 __global__ void __launch_bounds__(256) k_front_step(PlanDev P, double* F, int64_t fstride, int f0,
                                                     int count, const double* __restrict__ pert,
                                                     int32_t* status, int k) {
+  after_previous();
   const FrontGeom g = P.fgeom[f0 + blockIdx.y / count];
   if (k >= g.w) return;
   step_body(front_view(P, g, F, fstride), pert, status, k, 1 << 20, blockIdx.x,
@@ -1100,6 +1107,7 @@ __global__ void __launch_bounds__(256) k_front_step(PlanDev P, double* F, int64_
 __global__ void k_gather(const int32_t* __restrict__ src, const int32_t* __restrict__ dst,
                          int64_t nent, const double* vals, int64_t blob, double* G,
                          int64_t gstride) {
+  after_previous();
   const int64_t b = blockIdx.y;
   const double* V = vals + b * blob;
   double* g = G + b * gstride;
@@ -1199,6 +1207,7 @@ __global__ void __launch_bounds__(256) k_dense_pull(PlanDev P, double* vals,
 // into the column written by k_dense_pull with global atomics: warps take entries in turn,
 // lanes the entry's rows.
 __global__ void __launch_bounds__(256) k_dense_pull_extra(PlanDev P, double* vals) {
+  after_previous();
   const int64_t k = blockIdx.x;
   const int b = blockIdx.y, lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
   double* V = vals + (int64_t)b * P.blob;
@@ -1219,8 +1228,8 @@ void gemm_launch(int M, int N, int K, const double* A, int lda, const double* B,
   using G = Gemm<BM, BN, WM, WN, STAGES, BK>;
   ensure_smem_limit((const void*)k_gemm_sub<BM, BN, WM, WN, STAGES, BK>, G::SMEM);
   dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, count);
-  k_gemm_sub<BM, BN, WM, WN, STAGES, BK><<<grid, G::THREADS, G::SMEM, s>>>(
-      M, N, K, A, lda, B, ldb, C, ldc, sA, sB, sC, FrontGemm{});
+  k_gemm_sub<BM, BN, WM, WN, STAGES, BK><<<grid, G::THREADS, G::SMEM, s>>>(M, N, K, A, lda, B, ldb,
+      C, ldc, sA, sB, sC, FrontGemm{});
 }
 
 template <int BM, int BN, int WM, int WN, int STAGES, bool CPRE, int BK = 32>
@@ -1230,8 +1239,8 @@ void gemm16_launch(int M, int N, int K, const double* A, int lda, const double* 
   using G = Gemm<BM, BN, WM, WN, STAGES, BK>;
   ensure_smem_limit((const void*)k_gemm_sub16<BM, BN, WM, WN, STAGES, CPRE, BK>, G::SMEM);
   dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, count);
-  k_gemm_sub16<BM, BN, WM, WN, STAGES, CPRE, BK><<<grid, G::THREADS, G::SMEM, s>>>(
-      M, N, K, A, lda, B, ldb, C, ldc, sA, sB, sC);
+  k_gemm_sub16<BM, BN, WM, WN, STAGES, CPRE, BK><<<grid, G::THREADS, G::SMEM, s>>>(M, N, K, A, lda,
+      B, ldb, C, ldc, sA, sB, sC);
 }
 
 }  // namespace
@@ -1296,7 +1305,7 @@ int sm_count() {
 void launch_dense_diag(const DenseView& V, int count, const double* pert, int32_t* status, int k,
                        int nb, cudaStream_t s, LaunchCounter& lc) {
   if (nb == 128) k_dense_diag<128><<<count, 256, 0, s>>>(V, pert, status, k);
-  else k_dense_diag64<<<count, 256, kDiagSmem * 8, s>>>(V, pert, status, k);
+  else launch_next(k_dense_diag64, dim3(count), 256, kDiagSmem * 8, s, V, pert, status, k);
   lc.n++;
 }
 
@@ -1319,7 +1328,7 @@ void launch_dense_trsm(const DenseView& V, int count, int k, int nb, cudaStream_
       k_dense_trsm_mma<64, 4><<<dim3(nrt + nct, count), 128, smem4, s>>>(V, k, nrt);
     } else {
       ensure_smem_limit((const void*)k_dense_trsm8, kTrsm8Smem);
-      k_dense_trsm8<<<dim3(nrb + ncb, count), 256, kTrsm8Smem, s>>>(V, k, nrb);
+      launch_next(k_dense_trsm8, dim3(nrb + ncb, count), 256, kTrsm8Smem, s, V, k, nrb);
     }
   }
   lc.n++;
@@ -1381,7 +1390,7 @@ void launch_dense_factor(const DenseView& V, int count, const double* pert, int3
         int64_t c0 = lc.n;
         if (j == 0) launch_dense_diag(V, count, pert, status, c, nb, s, lc);
         if (mt + nt > 0) {
-          k_dense_trsm8<<<dim3(mt + nt, count), 256, kTrsm8Smem, s>>>(V, c, mt);
+          launch_next(k_dense_trsm8, dim3(mt + nt, count), 256, kTrsm8Smem, s, V, c, mt);
           lc.n++;
         }
         mark(2, c0);
@@ -1390,7 +1399,8 @@ void launch_dense_factor(const DenseView& V, int count, const double* pert, int3
         const int gc = std::min(wide, nt), gr = std::min(wide, mt);
         const int tiles = gc * mt + gr * (nt - gc);
         if (tiles > 0) {
-          k_dense_step<<<dim3(tiles, count), 256, kStepSmem, s>>>(V, pert, status, c, wide);
+          launch_next(k_dense_step, dim3(tiles, count), 256, kStepSmem, s, V, pert, status, c,
+                      wide);
           lc.n++;
           mark(6, c0);
         }
@@ -1444,6 +1454,7 @@ __global__ void k_front_pad(double* F, int64_t fstride, int ld, int w, int wp) {
 __global__ void k_front_writeback(const int32_t* __restrict__ slot, const int32_t* __restrict__ idx,
                                   int64_t cnt, double* vals, int64_t blob, const double* F,
                                   int64_t fstride) {
+  after_previous();
   const int64_t b = blockIdx.y;
   double* V = vals + b * blob;
   const double* f = F + b * fstride;
@@ -1457,6 +1468,7 @@ __global__ void k_front_writeback(const int32_t* __restrict__ slot, const int32_
 __global__ void k_front_schur(const int32_t* __restrict__ slot, const int32_t* __restrict__ idx,
                               int64_t cnt, double* vals, int64_t blob, const double* F,
                               int64_t fstride) {
+  after_previous();
   const int64_t b = blockIdx.y;
   double* V = vals + b * blob;
   const double* f = F + b * fstride;
@@ -1478,24 +1490,25 @@ void launch_front(const PlanDev& P, const FrontDev& f, double* vals, int count, 
     k_front_pad<<<dim3(1, count), 64, 0, s>>>(F, fstride, f.ld, f.w, f.wp);
     lc.n++;
   }
-  k_gather<<<dim3(grid(f.g_cnt), count), 256, 0, s>>>(P.fg_slot + f.g_off, P.fg_idx + f.g_off,
-                                                      f.g_cnt, vals, P.blob, F, fstride);
+  launch_next(k_gather, dim3(grid(f.g_cnt), count), 256, 0, s, P.fg_slot + f.g_off,
+              P.fg_idx + f.g_off, f.g_cnt, vals, P.blob, F, fstride);
   lc.n++;
   // 2. its first w pivots with the dense kernels
   DenseView V{F, fstride, f.ld, f.ld, f.wp + f.qp, P.fhasl + f.h_off, f.w};
   launch_dense_factor(V, count, pert, status, f.wp, nb, depth, variant, s, lc,
                       [](int, int64_t) {});
   // 3. factored S columns and U(S, J) back to their slots; Schur complement to the targets
-  k_front_writeback<<<dim3(grid(f.g_cnt), count), 256, 0, s>>>(
-      P.fg_slot + f.g_off, P.fg_idx + f.g_off, f.g_cnt, vals, P.blob, F, fstride);
+  launch_next(k_front_writeback, dim3(grid(f.g_cnt), count), 256, 0, s, P.fg_slot + f.g_off,
+              P.fg_idx + f.g_off, f.g_cnt, vals, P.blob, F, fstride);
   if (f.c_cnt > 0)
-    k_front_schur<<<dim3(grid(f.c_cnt), count), 256, 0, s>>>(
-        P.fc_slot + f.c_off, P.fc_idx + f.c_off, f.c_cnt, vals, P.blob, F, fstride);
+    launch_next(k_front_schur, dim3(grid(f.c_cnt), count), 256, 0, s, P.fc_slot + f.c_off,
+                P.fc_idx + f.c_off, f.c_cnt, vals, P.blob, F, fstride);
   lc.n += f.c_cnt > 0 ? 2 : 1;
 }
 
 // Identity on the padded pivots [w, wp) of every front f0 + blockIdx.x of a level.
 __global__ void k_front_pad_level(PlanDev P, double* F, int64_t fstride, int f0) {
+  after_previous();
   const FrontGeom g = P.fgeom[f0 + blockIdx.x];
   double* f = F + (int64_t)blockIdx.y * fstride + g.foff;
   for (int kk = g.w + threadIdx.x; kk < g.wp; kk += blockDim.x) f[kk + (int64_t)kk * g.ld] = 1.0;
@@ -1515,9 +1528,9 @@ void launch_front_level(const PlanDev& P, const FrontLevel& L, double* vals, int
   const int nf = L.nf, nfc = nf * count;
   // 1. assemble every front [A(S,S) A(S,J); A(R,S) 0] of the level (padded pivots: identity)
   cudaMemset2DAsync(F, sizeof(double) * fstride, 0, sizeof(double) * L.area, count, s);
-  k_front_pad_level<<<dim3(nf, count), 64, 0, s>>>(P, F, fstride, L.f0);
-  k_gather<<<dim3(grid(L.g1 - L.g0), count), 256, 0, s>>>(P.fg_slot + L.g0, P.fg_aidx + L.g0,
-                                                          L.g1 - L.g0, vals, P.blob, F, fstride);
+  launch_next(k_front_pad_level, dim3(nf, count), 64, 0, s, P, F, fstride, L.f0);
+  launch_next(k_gather, dim3(grid(L.g1 - L.g0), count), 256, 0, s, P.fg_slot + L.g0,
+              P.fg_aidx + L.g0, L.g1 - L.g0, vals, P.blob, F, fstride);
   lc.n += 2;
   // 2. their pivots, 64 at a time: diagonal blocks, L21 / U12, trailing update (the same kernels'
   //    bodies as the trailing block's, every front of the level in one launch per stage)
@@ -1534,46 +1547,48 @@ void launch_front_level(const PlanDev& P, const FrontLevel& L, double* vals, int
     if (few) {
       // one launch for L21 / U12 and one for the update with the next diagonal blocks
       if (i == 0) {
-        k_front_diag<<<dim3(count, nf), 256, kDiagSmem * 8, s>>>(P, F, fstride, L.f0, pert, status, k);
+        launch_next(k_front_diag, dim3(count, nf), 256, kDiagSmem * 8, s, P, F, fstride, L.f0, pert,
+                    status, k);
         lc.n++;
       }
       if (L.tiles1[i] > 0) {
-        k_front_trsm8<<<dim3(L.tiles1[i] / 2, nfc), 256, kTrsm8Smem, s>>>(P, F, fstride, L.f0,
-                                                                        count, k);
+        launch_next(k_front_trsm8, dim3(L.tiles1[i] / 2, nfc), 256, kTrsm8Smem, s, P, F, fstride,
+                    L.f0, count, k);
         lc.n++;
       }
       if (L.mmax[i] > 0 && L.nmax[i] > 0) {
-        k_front_step<<<dim3((L.mmax[i] / 64) * (L.nmax[i] / 64), nfc), 256, kStepSmem, s>>>(
-            P, F, fstride, L.f0, count, pert, status, k);
+        launch_next(k_front_step, dim3((L.mmax[i] / 64) * (L.nmax[i] / 64), nfc), 256, kStepSmem, s,
+                    P, F, fstride, L.f0, count, pert, status, k);
         lc.n++;
       }
       continue;
     }
-    k_front_diag<<<dim3(count, nf), 256, kDiagSmem * 8, s>>>(P, F, fstride, L.f0, pert, status, k);
+    launch_next(k_front_diag, dim3(count, nf), 256, kDiagSmem * 8, s, P, F, fstride, L.f0, pert,
+                status, k);
     lc.n++;
     if (L.tiles1[i] > 0) {      // some front has rows below or columns right of this panel
       if ((int64_t)L.tiles4[i] * nfc >= 2 * sm_count())
         k_front_trsm<4><<<dim3(L.tiles4[i], nfc), 128, smem4, s>>>(P, F, fstride, L.f0, count, k);
       else
-        k_front_trsm8<<<dim3(L.tiles1[i] / 2, nfc), 256, kTrsm8Smem, s>>>(P, F, fstride, L.f0,
-                                                                        count, k);
+        launch_next(k_front_trsm8, dim3(L.tiles1[i] / 2, nfc), 256, kTrsm8Smem, s, P, F, fstride,
+                    L.f0, count, k);
       lc.n++;
     }
     if (L.mmax[i] > 0 && L.nmax[i] > 0) {
       const FrontGemm fg{P.fgeom, F, fstride, L.f0, count, k};
       dim3 gg((L.mmax[i] + 63) / 64, (L.nmax[i] + 63) / 64, nfc);
-      k_gemm_sub<64, 64, 32, 32, 2, 16, true><<<gg, G::THREADS, G::SMEM, s>>>(
-          0, 0, 0, nullptr, 0, nullptr, 0, nullptr, 0, 0, 0, 0, fg);
+      k_gemm_sub<64, 64, 32, 32, 2, 16, true><<<gg, G::THREADS, G::SMEM, s>>>(0, 0, 0, nullptr, 0,
+          nullptr, 0, nullptr, 0, 0, 0, 0, fg);
       lc.n++;
     }
   }
   // 3. factored columns and U(S, J) back to their slots; Schur complements to the targets
-  k_front_writeback<<<dim3(grid(L.g1 - L.g0), count), 256, 0, s>>>(
-      P.fg_slot + L.g0, P.fg_aidx + L.g0, L.g1 - L.g0, vals, P.blob, F, fstride);
+  launch_next(k_front_writeback, dim3(grid(L.g1 - L.g0), count), 256, 0, s, P.fg_slot + L.g0,
+              P.fg_aidx + L.g0, L.g1 - L.g0, vals, P.blob, F, fstride);
   lc.n++;
   if (L.c1 > L.c0) {
-    k_front_schur<<<dim3(grid(L.c1 - L.c0), count), 256, 0, s>>>(
-        P.fc_slot + L.c0, P.fc_aidx + L.c0, L.c1 - L.c0, vals, P.blob, F, fstride);
+    launch_next(k_front_schur, dim3(grid(L.c1 - L.c0), count), 256, 0, s, P.fc_slot + L.c0,
+                P.fc_aidx + L.c0, L.c1 - L.c0, vals, P.blob, F, fstride);
     lc.n++;
   }
 }
@@ -1587,10 +1602,10 @@ void launch_hub_update(const PlanDev& P, double* vals, int count, double* gbuf, 
     int64_t g = (n + 255) / 256;
     return (int)(g < 1 ? 1 : (g > 1024 ? 1024 : g));
   };
-  k_gather<<<dim3(grid(P.ngl), count), 256, 0, s>>>(P.gl_src, P.gl_dst, P.ngl, vals, P.blob, gbuf,
-                                                     gstride);
-  k_gather<<<dim3(grid(P.ngu), count), 256, 0, s>>>(P.gu_src, P.gu_dst, P.ngu, vals, P.blob,
-                                                     gbuf + gl, gstride);
+  launch_next(k_gather, dim3(grid(P.ngl), count), 256, 0, s, P.gl_src, P.gl_dst, P.ngl, vals,
+              P.blob, gbuf, gstride);
+  launch_next(k_gather, dim3(grid(P.ngu), count), 256, 0, s, P.gu_src, P.gu_dst, P.ngu, vals,
+              P.blob, gbuf + gl, gstride);
   lc.n += 2;
   launch_gemm_sub((int)P.ntp, (int)P.ntp, (int)P.hubs_p, gbuf, (int)P.ntp, gbuf + gl, (int)P.hubs_p,
                   vals + P.dbase, (int)P.ntp, count, gstride, gstride, P.blob, s, lc, variant);
@@ -1623,7 +1638,7 @@ void dense_pull_launch(const PlanDev& P, double* vals, int count, const uint8_t*
     lc.n++;
   }
   if (split) {
-    k_dense_pull_extra<<<dim3((unsigned)P.npullx, count), 256, 0, s>>>(P, vals);
+    launch_next(k_dense_pull_extra, dim3((unsigned)P.npullx, count), 256, 0, s, P, vals);
     lc.n++;
   }
 }

@@ -52,6 +52,7 @@ __global__ void k_pad_identity(PlanDev P, double* vals, int first) {
 }
 
 __global__ void k_zero_slots(PlanDev P, double* vals, int first) {
+  after_previous();
   double* V = vals + (int64_t)(first + blockIdx.y) * P.blob;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < P.nasm_zero;
        e += (int64_t)gridDim.x * blockDim.x)
@@ -59,6 +60,7 @@ __global__ void k_zero_slots(PlanDev P, double* vals, int first) {
 }
 
 __global__ void k_ingest(PlanDev P, double* vals, int first, const double* __restrict__ a) {
+  after_previous();
   const int b = blockIdx.y;
   double* V = vals + (int64_t)(first + b) * P.blob;
   const double* ab = a + (int64_t)b * P.nnz_a;
@@ -70,6 +72,7 @@ __global__ void k_ingest(PlanDev P, double* vals, int first, const double* __res
 }
 
 __global__ void k_load_lu(PlanDev P, double* vals, int first, const double* __restrict__ val) {
+  after_previous();
   const int b = blockIdx.y;
   double* V = vals + (int64_t)(first + b) * P.blob;
   const double* vb = val + (int64_t)b * P.nnz;
@@ -79,6 +82,7 @@ __global__ void k_load_lu(PlanDev P, double* vals, int first, const double* __re
 }
 
 __global__ void k_export_lu(PlanDev P, const double* vals, int inst, double* __restrict__ val) {
+  after_previous();
   const double* V = vals + (int64_t)inst * P.blob;
   for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < P.nnz;
        p += (int64_t)gridDim.x * blockDim.x)
@@ -106,6 +110,7 @@ __global__ void k_pert_finish(int count, const unsigned long long* norm_bits, do
 }
 
 __global__ void k_fill(int count, double v, double* out) {
+  after_previous();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < count) out[b] = v;
 }
@@ -294,6 +299,7 @@ __global__ void __launch_bounds__(256) k_sparse_level(PlanDev P, double* vals,
                                                       const double* __restrict__ pert,
                                                       int32_t* status, int begin, int ncols,
                                                       int wpc, int cpw, int stage, int lanes) {
+  after_previous();
   extern __shared__ double Lsm[];
   const int b = blockIdx.y;
   const int gsz = wpc == 1 ? lanes : kWarp * wpc;
@@ -321,6 +327,7 @@ __global__ void __launch_bounds__(256) k_sparse_level(PlanDev P, double* vals,
 __global__ void __launch_bounds__(256) k_sparse_scale(PlanDev P, double* vals,
                                                       const double* __restrict__ pert,
                                                       int32_t* status, int begin) {
+  after_previous();
   const int b = blockIdx.y;
   sparse_column<true>(P, vals + (int64_t)b * P.blob, pert[b], status, b,
                       (uint32_t)P.scols[begin + blockIdx.x], cta_group());
@@ -331,6 +338,7 @@ __global__ void __launch_bounds__(256) k_sparse_scale(PlanDev P, double* vals,
 __global__ void __launch_bounds__(256) k_sparse_split(PlanDev P, double* vals,
                                                       const double* __restrict__ pert, int begin,
                                                       int splits) {
+  after_previous();
   extern __shared__ double Ls[];
   const int b = blockIdx.y;
   const int col = blockIdx.x / splits, part = blockIdx.x % splits;
@@ -345,6 +353,7 @@ __global__ void __launch_bounds__(256) k_sparse_split(PlanDev P, double* vals,
 // fixed order.  Grid (ceil(targets / 8), count), targets [t0, t0 + ntargets) of det_tptr.
 __global__ void __launch_bounds__(256) k_sparse_pull(PlanDev P, double* vals, int64_t t0,
                                                      int64_t ntargets) {
+  after_previous();
   const int64_t w = (int64_t)blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
   if (w >= ntargets) return;
   const int lane = threadIdx.x % kWarp;
@@ -493,6 +502,7 @@ __global__ void __launch_bounds__(256) k_sparse_persistent(PlanDev P, double* va
 // Also marks the vector's values of the dense solve unsolved and clears its failure word.
 __global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm, double* y,
                              int64_t ylen, int transpose, double* xbuf, int* err) {
+  after_previous();
   const int64_t v = blockIdx.y;                 // instance * nrhs + rhs
   if (blockIdx.x == 0 && v == 0 && threadIdx.x == 0) *err = 0;
   const int64_t nx = solve_buffer(P);
@@ -519,6 +529,7 @@ __global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm,
 
 __global__ void k_permute_out(PlanDev P, int nrhs, const double* __restrict__ y, double* X,
                               int64_t ylen, int transpose) {
+  after_previous();
   const int64_t v = blockIdx.y;
   const double* yv = y + v * ylen;
   double* xv = X + v * P.n;
@@ -560,17 +571,18 @@ __device__ __forceinline__ SolveShare solve_share(int ncols, int nlong) {
   return SolveShare{i < ncols ? i : -1, (int)(threadIdx.x % kWarp), kWarp, false};
 }
 
-// Entries [p0, p1) of a column pushed into nk vectors: y(ri[p]) -= V[p] xc.
+// Entries [p0, p1) of a column pushed into nk vectors: y(ri[p]) -= V[p] xc; r0 = ri of the thread's
+// first entry.
 template <int NV>
 __device__ __forceinline__ void solve_push(const PlanDev& P, const double* __restrict__ V,
                                            double* y0, int64_t ylen, int nk,
                                            const double (&xc)[NV], uint32_t p0, uint32_t p1,
-                                           const SolveShare& sh) {
+                                           uint32_t r0, const SolveShare& sh) {
   uint32_t p = p0 + sh.first;
   if (p1 - p0 <= 2 * (uint32_t)sh.step) {      // short columns: most of them, in a netlist
-    for (; p < p1; p += sh.step) {
-      const uint32_t r = P.ri[p];
-      const double m = V[p];
+    for (uint32_t q = p; q < p1; q += sh.step) {
+      const uint32_t r = q == p ? r0 : P.ri[q];
+      const double m = V[q];
 #pragma unroll
       for (int k = 0; k < NV; ++k)
         if (k < nk) atomicAdd(y0 + k * ylen + r, -(m * xc[k]));
@@ -604,17 +616,20 @@ __global__ void __launch_bounds__(256) k_sparse_lsolve(PlanDev P, const double* 
                                                        const int32_t* __restrict__ cols, int begin,
                                                        int ncols, int nlong) {
   const SolveShare sh = solve_share(ncols, nlong);
+  const uint32_t c = sh.i < 0 ? 0 : (uint32_t)cols[begin + sh.i];
+  const uint32_t p0 = P.lp[c] + 1, p1 = P.cp[c + 1];
+  const uint32_t r0 = sh.i >= 0 && p0 + sh.first < p1 ? P.ri[p0 + sh.first] : 0;
+  after_previous();
   if (sh.i < 0) return;
   const int groups = (nrhs + NV - 1) / NV;
   const int64_t inst = blockIdx.y / groups;
   const int k0 = (blockIdx.y % groups) * NV;
   const int nk = min(NV, nrhs - k0);
   double* y0 = y + (inst * nrhs + k0) * ylen;
-  const uint32_t c = (uint32_t)cols[begin + sh.i];
   double yc[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) yc[k] = k < nk ? y0[k * ylen + c] : 0.0;
-  solve_push(P, vals + inst * P.blob, y0, ylen, nk, yc, P.lp[c] + 1, P.cp[c + 1], sh);
+  solve_push(P, vals + inst * P.blob, y0, ylen, nk, yc, p0, p1, r0, sh);
 }
 
 // U solve (symbolic.cc:228-236).
@@ -624,6 +639,10 @@ __global__ void __launch_bounds__(256) k_sparse_usolve(PlanDev P, const double* 
                                                        const int32_t* __restrict__ cols, int begin,
                                                        int ncols, int nlong) {
   const SolveShare sh = solve_share(ncols, nlong);
+  const uint32_t c = sh.i < 0 ? 0 : (uint32_t)cols[begin + sh.i];
+  const uint32_t p0 = P.cp[c], p1 = P.lp[c];
+  const uint32_t r0 = sh.i >= 0 && p0 + sh.first < p1 ? P.ri[p0 + sh.first] : 0;
+  after_previous();
   if (sh.i < 0) return;
   const int groups = (nrhs + NV - 1) / NV;
   const int64_t inst = blockIdx.y / groups;
@@ -631,8 +650,7 @@ __global__ void __launch_bounds__(256) k_sparse_usolve(PlanDev P, const double* 
   const int nk = min(NV, nrhs - k0);
   const double* V = vals + inst * P.blob;
   double* y0 = y + (inst * nrhs + k0) * ylen;
-  const uint32_t c = (uint32_t)cols[begin + sh.i];
-  const double d = V[P.lp[c]];
+  const double d = V[p1];
   double xc[NV];
 #pragma unroll
   for (int k = 0; k < NV; ++k) xc[k] = k < nk ? y0[k * ylen + c] / d : 0.0;
@@ -644,7 +662,7 @@ __global__ void __launch_bounds__(256) k_sparse_usolve(PlanDev P, const double* 
       if (sh.first == k) xv = xc[k];
     y0[sh.first * ylen + c] = xv;
   }
-  solve_push(P, V, y0, ylen, nk, xc, P.cp[c], P.lp[c], sh);
+  solve_push(P, V, y0, ylen, nk, xc, p0, p1, r0, sh);
 }
 
 // Sum of V[p] y(ri[p]) over the entries [p0, p1) of a column, in every thread of a warp share, in
@@ -684,12 +702,14 @@ __global__ void __launch_bounds__(256) k_sparse_utsolve(PlanDev P, const double*
                                                         const int32_t* __restrict__ cols,
                                                         int begin, int ncols, int nlong) {
   const SolveShare sh = solve_share(ncols, nlong);
+  const uint32_t j = sh.i < 0 ? 0 : (uint32_t)cols[begin + sh.i];
+  const uint32_t p0 = P.cp[j], p1 = P.lp[j];
+  after_previous();
   if (sh.i < 0) return;
   const int64_t v = blockIdx.y;
   const double* V = vals + (v / nrhs) * P.blob;
   double* yv = y + v * ylen;
-  const uint32_t j = (uint32_t)cols[begin + sh.i];
-  const double s = solve_pull(P, V, yv, P.cp[j], P.lp[j], sh);
+  const double s = solve_pull(P, V, yv, p0, p1, sh);
   if (sh.first == 0) yv[j] = (yv[j] - s) / V[P.lp[j]];
 }
 
@@ -699,12 +719,14 @@ __global__ void __launch_bounds__(256) k_sparse_ltsolve(PlanDev P, const double*
                                                         const int32_t* __restrict__ cols,
                                                         int begin, int ncols, int nlong) {
   const SolveShare sh = solve_share(ncols, nlong);
+  const uint32_t j = sh.i < 0 ? 0 : (uint32_t)cols[begin + sh.i];
+  const uint32_t p0 = P.lp[j] + 1, p1 = P.cp[j + 1];
+  after_previous();
   if (sh.i < 0) return;
   const int64_t v = blockIdx.y;
   const double* V = vals + (v / nrhs) * P.blob;
   double* yv = y + v * ylen;
-  const uint32_t j = (uint32_t)cols[begin + sh.i];
-  const double s = solve_pull(P, V, yv, P.lp[j] + 1, P.cp[j + 1], sh);
+  const double s = solve_pull(P, V, yv, p0, p1, sh);
   if (sh.first == 0) yv[j] = yv[j] - s;
 }
 
@@ -740,21 +762,24 @@ __global__ void __launch_bounds__(256) k_solve_level(PlanDev P, const double* va
   const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
   if ((int)blockIdx.x < ncb) {
     const SolveShare sh = solve_share(ncols, nlong);
+    const uint32_t c = sh.i < 0 ? 0 : (uint32_t)cols[begin + sh.i];
+    const uint32_t dc = P.lp[c], p0 = dc + 1, p1 = P.cp[c + 1];
+    const uint32_t r0 = WHICH == 0 && sh.i >= 0 && p0 + sh.first < p1 ? P.ri[p0 + sh.first] : 0;
+    const int64_t e0 = WHICH == 1 ? P.ur_ptr[c] : 0, e1 = WHICH == 1 ? P.ur_ptr[c + 1] : 0;
+    after_previous();
     if (sh.i < 0) return;
-    const uint32_t c = (uint32_t)cols[begin + sh.i];
     if (WHICH == 0) {
       double yc[NV];
 #pragma unroll
       for (int k = 0; k < NV; ++k) yc[k] = k < nk ? y0[k * ylen + c] : 0.0;
-      solve_push(P, V, y0, ylen, nk, yc, P.lp[c] + 1, P.cp[c + 1], sh);
+      solve_push(P, V, y0, ylen, nk, yc, p0, p1, r0, sh);
     } else if (WHICH == 1) {
       double sum[NV];
 #pragma unroll
       for (int k = 0; k < NV; ++k) sum[k] = 0.0;
       // the diagonal and the running value are on their way while the row is summed
-      const double d = V[P.lp[c]];
+      const double d = V[dc];
       const double yc = sh.first < nk ? y0[sh.first * ylen + c] : 0.0;
-      const int64_t e0 = P.ur_ptr[c], e1 = P.ur_ptr[c + 1];
       int64_t e = e0 + sh.first;
       if (e1 - e0 <= 2 * sh.step) {
         for (; e < e1; e += sh.step) {
@@ -798,14 +823,15 @@ __global__ void __launch_bounds__(256) k_solve_level(PlanDev P, const double* va
         y0[sh.first * ylen + c] = (yc - t) / d;
       }
     } else {
-      const double t = WHICH == 2 ? solve_pull(P, V, y0, P.cp[c], P.lp[c], sh)
-                                  : solve_pull(P, V, y0, P.lp[c] + 1, P.cp[c + 1], sh);
-      if (sh.first == 0) y0[c] = WHICH == 2 ? (y0[c] - t) / V[P.lp[c]] : y0[c] - t;
+      const double t = WHICH == 2 ? solve_pull(P, V, y0, P.cp[c], dc, sh)
+                                  : solve_pull(P, V, y0, p0, p1, sh);
+      if (sh.first == 0) y0[c] = WHICH == 2 ? (y0[c] - t) / V[dc] : y0[c] - t;
     }
     return;
   }
   const int4 it = ext[blockIdx.x - ncb];
   const int f = it.x, s0 = P.fs0[f], w = P.fw[f];
+  after_previous();
   if (WHICH >= 2) {
     const int x = it.y + warp;
     if (x >= w) return;
@@ -873,6 +899,7 @@ __global__ void __launch_bounds__(256) k_rows_solve(PlanDev P, const double* val
                                                     double* y, int64_t ylen,
                                                     const int32_t* __restrict__ rows, int begin,
                                                     int nrows, int which) {
+  after_previous();
   const int w = blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
   if (w >= nrows) return;
   const int lane = threadIdx.x % kWarp;
@@ -897,6 +924,7 @@ __global__ void __launch_bounds__(256) k_rows_solve(PlanDev P, const double* val
 // Border U(r < t, j >= t): push x_j into rows r (solve) or pull w_r into w_j (transpose).
 __global__ void k_border(PlanDev P, const double* vals, int nrhs, double* y, int64_t ylen,
                          int transpose) {
+  after_previous();
   const int jt = blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
   if (jt >= (int)P.nt) return;
   const int lane = threadIdx.x % kWarp;
@@ -923,6 +951,7 @@ __global__ void k_border(PlanDev P, const double* vals, int nrhs, double* y, int
 template <int NV>
 __global__ void __launch_bounds__(256) k_border_chunks(PlanDev P, const double* vals, int nrhs,
                                                        double* y, int64_t ylen) {
+  after_previous();
   const int64_t c = (int64_t)blockIdx.x * (blockDim.x / kWarp) + threadIdx.x / kWarp;
   if (c >= P.nbordck) return;
   const int lane = threadIdx.x % kWarp;
@@ -988,6 +1017,7 @@ __global__ void k_grad(PlanDev P, int nrhs, const double* __restrict__ lambda,
 __global__ void k_residual(PlanDev P, int nrhs, const double* __restrict__ a,
                            const double* __restrict__ X, const double* __restrict__ Bm,
                            double* __restrict__ R, unsigned long long* norms, int transpose) {
+  after_previous();
   residual_rows(P, nrhs, a, X, Bm, R, norms, transpose, blockIdx.y, blockIdx.x, gridDim.x);
 }
 
@@ -997,6 +1027,7 @@ __global__ void k_resid_finish(int64_t nv, const unsigned long long* norms, doub
 }
 
 __global__ void k_axpy(int64_t n, const double* __restrict__ dx, double* __restrict__ x) {
+  after_previous();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     x[i] += dx[i];
@@ -1022,7 +1053,8 @@ void launch_prepare_blob(const PlanDev& P, double* vals, int first, int count, b
       cudaMemset2DAsync(vals + (int64_t)first * P.blob, sizeof(double) * P.blob, 0,
                         sizeof(double) * P.dbase, count, s);
     if (P.nasm_zero > 0) {
-      k_zero_slots<<<dim3(grid1(P.nasm_zero, 256, 256), count), 256, 0, s>>>(P, vals, first);
+      launch_next(k_zero_slots, dim3(grid1(P.nasm_zero, 256, 256), count), 256, 0, s, P, vals,
+                  first);
       lc.n++;
     }
     return;
@@ -1036,26 +1068,26 @@ void launch_prepare_blob(const PlanDev& P, double* vals, int first, int count, b
 
 void launch_ingest(const PlanDev& P, double* vals, int first, int count, const double* a,
                    cudaStream_t s, LaunchCounter& lc) {
-  k_ingest<<<dim3(grid1(P.nnz_a, 256, 1024), count), 256, 0, s>>>(P, vals, first, a);
+  launch_next(k_ingest, dim3(grid1(P.nnz_a, 256, 1024), count), 256, 0, s, P, vals, first, a);
   lc.n++;
 }
 
 void launch_load_lu(const PlanDev& P, double* vals, int first, int count, const double* val,
                     cudaStream_t s, LaunchCounter& lc) {
-  k_load_lu<<<dim3(grid1(P.nnz, 256, 1024), count), 256, 0, s>>>(P, vals, first, val);
+  launch_next(k_load_lu, dim3(grid1(P.nnz, 256, 1024), count), 256, 0, s, P, vals, first, val);
   lc.n++;
 }
 
 void launch_export_lu(const PlanDev& P, const double* vals, int inst, double* val, cudaStream_t s,
                       LaunchCounter& lc) {
-  k_export_lu<<<grid1(P.nnz, 256), 256, 0, s>>>(P, vals, inst, val);
+  launch_next(k_export_lu, dim3(grid1(P.nnz, 256)), 256, 0, s, P, vals, inst, val);
   lc.n++;
 }
 
 void launch_pert(const PlanDev& P, const double* vals, int count, double pert, double* pert_dev,
                  cudaStream_t s, LaunchCounter& lc) {
   if (pert >= 0.0) {
-    k_fill<<<(count + 127) / 128, 128, 0, s>>>(count, pert, pert_dev);
+    launch_next(k_fill, dim3((count + 127) / 128), 128, 0, s, count, pert, pert_dev);
     lc.n++;
     return;
   }
@@ -1086,9 +1118,9 @@ void launch_sparse_level(const PlanDev& P, double* vals, int count, const double
                                  : 2 * (int64_t)sm_count();
   if (wpc > 1 && ctas < target && max_pairs > 16 && max_nl <= kSplitMaxL) {
     int splits = (int)std::min<int64_t>((target + ctas - 1) / ctas, (max_pairs + 7) / 8);
-    k_sparse_split<<<dim3(ncols * splits, count), 256, sizeof(double) * std::max(max_nl, 1), s>>>(
-        P, vals, pert, begin, splits);
-    k_sparse_scale<<<dim3(ncols, count), 256, 0, s>>>(P, vals, pert, status, begin);
+    launch_next(k_sparse_split, dim3(ncols * splits, count), 256, sizeof(double) * std::max(max_nl,
+                1), s, P, vals, pert, begin, splits);
+    launch_next(k_sparse_scale, dim3(ncols, count), 256, 0, s, P, vals, pert, status, begin);
     lc.n += 2;
     return;
   }
@@ -1102,19 +1134,19 @@ void launch_sparse_level(const PlanDev& P, double* vals, int count, const double
   constexpr int kStageMaxL = 3072;
   const bool stage = groups == 1 && max_nl > 0 && max_nl <= kStageMaxL;
   const size_t smem = stage ? sizeof(double) * max_nl : 0;
-  k_sparse_level<<<dim3((ncols + per_cta - 1) / per_cta, count), block, smem, s>>>(
-      P, vals, pert, status, begin, ncols, wpc, std::max(1, cpw), stage ? 1 : 0, lanes);
+  launch_next(k_sparse_level, dim3((ncols + per_cta - 1) / per_cta, count), block, smem, s, P, vals,
+              pert, status, begin, ncols, wpc, std::max(1, cpw), stage ? 1 : 0, lanes);
   lc.n++;
 }
 
 void launch_sparse_level_det(const PlanDev& P, double* vals, int count, const double* pert,
                              int32_t* status, int begin, int ncols, int64_t t0, int64_t t1,
                              cudaStream_t s, LaunchCounter& lc) {
-  k_sparse_scale<<<dim3(ncols, count), 256, 0, s>>>(P, vals, pert, status, begin);
+  launch_next(k_sparse_scale, dim3(ncols, count), 256, 0, s, P, vals, pert, status, begin);
   lc.n++;
   const int64_t nt = t1 - t0;
   if (nt > 0) {
-    k_sparse_pull<<<dim3((unsigned)((nt + 7) / 8), count), 256, 0, s>>>(P, vals, t0, nt);
+    launch_next(k_sparse_pull, dim3((unsigned)((nt + 7) / 8), count), 256, 0, s, P, vals, t0, nt);
     lc.n++;
   }
 }
@@ -1123,8 +1155,8 @@ void launch_rows_solve(const PlanDev& P, const double* vals, int count, int nrhs
                        int64_t ylen, const int32_t* rows, int begin, int nrows, int which,
                        cudaStream_t s, LaunchCounter& lc) {
   if (nrows <= 0) return;
-  k_rows_solve<<<dim3((nrows + 7) / 8, count * nrhs), 256, 0, s>>>(P, vals, nrhs, y, ylen, rows,
-                                                                   begin, nrows, which);
+  launch_next(k_rows_solve, dim3((nrows + 7) / 8, count * nrhs), 256, 0, s, P, vals, nrhs, y, ylen,
+              rows, begin, nrows, which);
   lc.n++;
 }
 
@@ -1167,15 +1199,15 @@ void launch_sparse_persistent(const PlanDev& P, double* vals, int count, const d
 void launch_solve_permute_in(const PlanDev& P, int count, int nrhs, const double* B, double* y,
                              int64_t ylen, int transpose, double* xbuf, int* err, cudaStream_t s,
                              LaunchCounter& lc) {
-  k_permute_in<<<dim3(grid1(ylen, 256, 256), count * nrhs), 256, 0, s>>>(P, nrhs, B, y, ylen,
-                                                                        transpose, xbuf, err);
+  launch_next(k_permute_in, dim3(grid1(ylen, 256, 256), count * nrhs), 256, 0, s, P, nrhs, B, y,
+              ylen, transpose, xbuf, err);
   lc.n++;
 }
 
 void launch_solve_permute_out(const PlanDev& P, int count, int nrhs, const double* y, double* X,
                               int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc) {
-  k_permute_out<<<dim3(grid1(P.n, 256, 256), count * nrhs), 256, 0, s>>>(P, nrhs, y, X, ylen,
-                                                                        transpose);
+  launch_next(k_permute_out, dim3(grid1(P.n, 256, 256), count * nrhs), 256, 0, s, P, nrhs, y, X,
+              ylen, transpose);
   lc.n++;
 }
 
@@ -1184,11 +1216,12 @@ void launch_sparse_lsolve(const PlanDev& P, const double* vals, int count, int n
                           cudaStream_t s, LaunchCounter& lc) {
   const unsigned gx = nlong + (ncols - nlong + 7) / 8;
   if (nrhs == 1)
-    k_sparse_lsolve<1><<<dim3(gx, count), 256, 0, s>>>(P, vals, nrhs, y, ylen, cols, begin, ncols,
-                                                    nlong);
+    launch_next(k_sparse_lsolve<1>, dim3(gx, count), 256, 0, s, P, vals, nrhs, y, ylen, cols, begin,
+                ncols, nlong);
   else
-    k_sparse_lsolve<kSolveVecs><<<dim3(gx, count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0, s>>>(
-        P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+    launch_next(k_sparse_lsolve<kSolveVecs>, dim3(gx,
+                count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0, s, P, vals, nrhs, y, ylen,
+                cols, begin, ncols, nlong);
   lc.n++;
 }
 void launch_sparse_usolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
@@ -1196,27 +1229,26 @@ void launch_sparse_usolve(const PlanDev& P, const double* vals, int count, int n
                           cudaStream_t s, LaunchCounter& lc) {
   const unsigned gx = nlong + (ncols - nlong + 7) / 8;
   if (nrhs == 1)
-    k_sparse_usolve<1><<<dim3(gx, count), 256, 0, s>>>(P, vals, nrhs, y, ylen, cols, begin, ncols,
-                                                    nlong);
+    launch_next(k_sparse_usolve<1>, dim3(gx, count), 256, 0, s, P, vals, nrhs, y, ylen, cols, begin,
+                ncols, nlong);
   else
-    k_sparse_usolve<kSolveVecs><<<dim3(gx, count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0, s>>>(
-        P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+    launch_next(k_sparse_usolve<kSolveVecs>, dim3(gx,
+                count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0, s, P, vals, nrhs, y, ylen,
+                cols, begin, ncols, nlong);
   lc.n++;
 }
 void launch_sparse_utsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                            int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                            cudaStream_t s, LaunchCounter& lc) {
-  k_sparse_utsolve<<<dim3(nlong + (ncols - nlong + 7) / 8,
-                      count * nrhs), 256, 0, s>>>(
-      P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+  launch_next(k_sparse_utsolve, dim3(nlong + (ncols - nlong + 7) / 8, count * nrhs), 256, 0, s, P,
+              vals, nrhs, y, ylen, cols, begin, ncols, nlong);
   lc.n++;
 }
 void launch_sparse_ltsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                            int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                            cudaStream_t s, LaunchCounter& lc) {
-  k_sparse_ltsolve<<<dim3(nlong + (ncols - nlong + 7) / 8,
-                      count * nrhs), 256, 0, s>>>(
-      P, vals, nrhs, y, ylen, cols, begin, ncols, nlong);
+  launch_next(k_sparse_ltsolve, dim3(nlong + (ncols - nlong + 7) / 8, count * nrhs), 256, 0, s, P,
+              vals, nrhs, y, ylen, cols, begin, ncols, nlong);
   lc.n++;
 }
 
@@ -1227,8 +1259,8 @@ void launch_solve_level(const PlanDev& P, const double* vals, int count, int nrh
   if (ncb + L.next == 0) return;
   const int4* ext = reinterpret_cast<const int4*>(L.ext);
   const auto launch = [&](auto kern, int nv) {
-    kern<<<dim3(ncb + L.next, count * ((nrhs + nv - 1) / nv)), 256, 0, s>>>(
-        P, vals, nrhs, y, ylen, cols, begin, ncols, nlong, ncb, ext);
+    launch_next(kern, dim3(ncb + L.next, count * ((nrhs + nv - 1) / nv)), 256, 0, s, P, vals, nrhs,
+                y, ylen, cols, begin, ncols, nlong, ncb, ext);
     lc.n++;
   };
   if (which == 0) nrhs == 1 ? launch(k_solve_level<1, 0>, 1) : launch(k_solve_level<kSolveVecs, 0>, kSolveVecs);
@@ -1242,12 +1274,13 @@ void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, do
   if (P.nt == 0) return;
   const unsigned gx = (unsigned)((P.nbordck + 7) / 8);
   if (!transpose && P.nbordck > 0 && nrhs == 1)
-    k_border_chunks<1><<<dim3(gx, count), 256, 0, s>>>(P, vals, nrhs, y, ylen);
+    launch_next(k_border_chunks<1>, dim3(gx, count), 256, 0, s, P, vals, nrhs, y, ylen);
   else if (!transpose && P.nbordck > 0)
-    k_border_chunks<kSolveVecs><<<dim3(gx, count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0,
-                                  s>>>(P, vals, nrhs, y, ylen);
+    launch_next(k_border_chunks<kSolveVecs>, dim3(gx,
+                count * ((nrhs + kSolveVecs - 1) / kSolveVecs)), 256, 0, s, P, vals, nrhs, y, ylen);
   else
-    k_border<<<dim3((P.nt + 7) / 8, count * nrhs), 256, 0, s>>>(P, vals, nrhs, y, ylen, transpose);
+    launch_next(k_border, dim3((P.nt + 7) / 8, count * nrhs), 256, 0, s, P, vals, nrhs, y, ylen,
+                transpose);
   lc.n++;
 }
 
@@ -1256,8 +1289,8 @@ void launch_residual(const PlanDev& P, int count, int nrhs, const double* a, con
                      int transpose, cudaStream_t s, LaunchCounter& lc) {
   const int64_t nv = (int64_t)count * nrhs;
   cudaMemsetAsync(norms, 0, sizeof(unsigned long long) * 4 * nv, s);
-  k_residual<<<dim3(grid1(P.n, 256, 64), (unsigned)nv), 256, 0, s>>>(P, nrhs, a, X, B, R, norms,
-                                                                    transpose);
+  launch_next(k_residual, dim3(grid1(P.n, 256, 64), (unsigned)nv), 256, 0, s, P, nrhs, a, X, B, R,
+              norms, transpose);
   lc.n++;
   if (resid) {
     k_resid_finish<<<(unsigned)((nv + 127) / 128), 128, 0, s>>>(nv, norms, resid);
@@ -1266,7 +1299,7 @@ void launch_residual(const PlanDev& P, int count, int nrhs, const double* a, con
 }
 
 void launch_axpy(int64_t n, const double* dx, double* x, cudaStream_t s, LaunchCounter& lc) {
-  k_axpy<<<grid1(n, 256, 4096), 256, 0, s>>>(n, dx, x);
+  launch_next(k_axpy, dim3(grid1(n, 256, 4096)), 256, 0, s, n, dx, x);
   lc.n++;
 }
 

@@ -555,6 +555,7 @@ __global__ void __launch_bounds__(256, NV * (WHICH >= 2 ? 2 : 1) >= 8 ? 1 : 2)
   const int64_t units = (int64_t)count * chunks;
   const int64_t xl = solve_buffer(P);
   double* xf = xbuf + 2 * (int64_t)P.ntp + (WHICH == 1 || WHICH == 3 ? P.fx_len : 0);
+  after_previous();
   for (int64_t it = blockIdx.x; it < nitems * units; it += gridDim.x) {
     const int2 item = items[it / units];
     const int u = (int)(it % units), inst = u / chunks, v0 = (u % chunks) * NV;
@@ -578,13 +579,15 @@ void front_launch(const PlanDev& P, const double* vals, int count, int nrhs, dou
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cfg.gridDim = dim3((unsigned)total);
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // as launch_next
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
   if (L.nflow > L.nfronts) {                  // some front has blocks that wait
     const int cap = flow_capacity((const void*)kern, flow_smem<NV>());
     cfg.gridDim = dim3((unsigned)std::min<int64_t>(total, std::max(cap, 1)));
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
   }
   cfg.blockDim = dim3(256);
   cfg.dynamicSmemBytes = flow_smem<NV>();

@@ -22,4 +22,13 @@ __device__ __forceinline__ unsigned long long global_ns() {
 constexpr long long kUnsolved = 0x7ff4a1c35e6b2d97ll;
 constexpr long long kNaN = 0x7ff8000000000000ll;
 
+// First statement of a kernel that launch_next launches (after reads of the plan's arrays at most,
+// which nothing writes): waits until the kernel before it in the stream has finished and its writes
+// are visible, then lets the kernel after it be placed on SMs that become free.  Every CTA passes
+// here before it returns, so kernels finish in stream order.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 }  // namespace glu
