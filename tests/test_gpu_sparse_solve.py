@@ -86,3 +86,30 @@ def test_long_and_short_pairs(options):
         lu = np.zeros((n, n))                 # [column, row]
         lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
         check_lu(torch, lu, np.ascontiguousarray(a.T * s)[None])
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+def test_residual_of_long_rows(transpose):
+    """r = b - op(A) x with rows of 63 to 1,100 entries: within 2 n u |A| |x| of numpy's."""
+    import torch
+    n = 1100
+    a = np.diag(np.linspace(1.0, 2.0, n))
+    for k, length in enumerate((63, 64, 65, 66, 127, 128, 129, 600, n)):
+        a[7 + 40 * k, :length] = np.sin(np.arange(length) + k)
+        a[:length, 11 + 40 * k] = np.cos(np.arange(length) + k)
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym)
+    plan.set_original_pattern(row, col)
+    batch = glu.Batch(plan, 1)
+    rng = np.random.default_rng(0)
+    x, b = rng.standard_normal((2, 1, 1, n))
+    op = a.T if transpose else a
+    val = torch.as_tensor(a[row, col][None], device="cuda")
+    got = batch.residual(val, torch.as_tensor(b, device="cuda"), torch.as_tensor(x, device="cuda"),
+                         transpose=transpose).item()
+    r = np.abs(b[0, 0] - op @ x[0, 0]).max()
+    den = np.abs(op).sum(1).max() * np.abs(x).max() + np.abs(b).max()
+    slack = 2 * n * 2.0 ** -53 * (np.abs(op) @ np.abs(x[0, 0])).max() / den
+    assert abs(got - r / den) <= slack + 4 * n * 2.0 ** -53 * r / den
