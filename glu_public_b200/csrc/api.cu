@@ -387,7 +387,28 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
       if (which == 3) glu::launch_sparse_ltsolve(P, b->vals, cnt, nrhs, y, yl, cols, ptr[l], ncols, nlong, s, lc);
     }
   };
-  if (!transpose && hp.deterministic) {
+  // the sparse columns as a dataflow: one launch for each of L, U (or their transposes), with the
+  // part of U right of t (L below t in the transposed solve) pulled beforehand by all rows at once
+  auto flow = [&](int which) {
+    glu::launch_sparse_flow(P, b->vals, cnt, nrhs, y, yl, which == 0 || which == 3 ? pl->d_lcols
+                            : pl->d_ucols, which, b->xbuf, serr, b->status, b->pwait_ms, s, lc);
+  };
+  if (hp.fronts.empty() && glu::sparse_solve_flows(P, cnt, nrhs)) {
+    if (!transpose) {
+      flow(0);
+      dense();
+      glu::launch_outer_rows(P, b->vals, cnt, nrhs, y, yl, (int)hp.br_rows.size(), hp.br_long, 1, s,
+                             lc);
+      flow(1);
+    } else {
+      flow(2);
+      glu::launch_border(P, b->vals, cnt, nrhs, y, yl, 1, s, lc);
+      dense();
+      glu::launch_outer_rows(P, b->vals, cnt, nrhs, y, yl, (int)hp.lc_cols.size(), hp.lc_long, 3, s,
+                             lc);
+      flow(3);
+    }
+  } else if (!transpose && hp.deterministic) {
     // row-wise (pull) solves: every entry of y is written by one warp, sums in a fixed order
     for (int l = 0; l < nl; ++l)
       glu::launch_rows_solve(P, b->vals, cnt, nrhs, y, yl, pl->d_lcols, hp.lptr[l],
@@ -691,11 +712,14 @@ int glu_plan_create(uint32_t n, uint32_t nnz, const uint32_t* sym_c_ptr,
       (st = p->upload(hp.fx0, &P.fx0)) || (st = p->upload(hp.uj_ptr, &P.uj_ptr)) ||
       (st = p->upload(hp.uj_col, &P.uj_col)) || (st = p->upload(hp.uj_slot, &P.uj_slot)) ||
       (st = p->upload(hp.ur_ptr, &P.ur_ptr)) || (st = p->upload(hp.ur_col, &P.ur_col)) ||
-      (st = p->upload(hp.ur_slot, &P.ur_slot)) || (st = p->upload(hp.ur_rows, &P.ur_rows))) {
+      (st = p->upload(hp.ur_slot, &P.ur_slot)) || (st = p->upload(hp.ur_rows, &P.ur_rows)) ||
+      (st = p->upload(hp.lr_ptr, &P.lr_ptr)) || (st = p->upload(hp.lr_col, &P.lr_col)) ||
+      (st = p->upload(hp.lr_slot, &P.lr_slot)) || (st = p->upload(hp.ur_split, &P.ur_split)) ||
+      (st = p->upload(hp.br_rows, &P.br_rows)) || (st = p->upload(hp.lc_cols, &P.lc_cols))) {
     glu_plan_destroy(p);
     return st;
   }
-  P.fx_len = hp.fx_len;
+  P.fx_len = hp.fronts.empty() ? hp.t : hp.fx_len;
   p->d_lcols = const_cast<int32_t*>(lc);
   p->d_ucols = const_cast<int32_t*>(uc);
   *out = p;

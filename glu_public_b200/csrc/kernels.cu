@@ -889,6 +889,63 @@ __global__ void __launch_bounds__(256) k_solve_level(PlanDev P, const double* va
   }
 }
 
+// Sums of solved values from the dense block taken off sparse rows (WHICH 1: the entries of U right
+// of t) or columns (3: the entries of L below t), up to NV right-hand sides of one instance
+// together; the long ones take a CTA.  No atomics, the same order of additions in every run.
+template <int NV, int WHICH>
+__global__ void __launch_bounds__(256) k_outer_rows(PlanDev P, const double* vals, int nrhs,
+                                                    double* y, int64_t ylen, int nrows, int nlong) {
+  __shared__ double red[NV * 8];
+  const SolveShare sh = solve_share(nrows, nlong);
+  const int32_t c = sh.i < 0 ? 0 : (WHICH == 1 ? P.br_rows : P.lc_cols)[sh.i];
+  const int64_t e0 = WHICH == 1 ? P.ur_ptr[c] + P.ur_split[c] : (int64_t)P.lp[c] + 1 + P.lsplit[c];
+  const int64_t e1 = WHICH == 1 ? P.ur_ptr[c + 1] : (int64_t)P.cp[c + 1];
+  after_previous();
+  if (sh.i < 0) return;
+  const int groups = (nrhs + NV - 1) / NV;
+  const int64_t inst = blockIdx.y / groups;
+  const int k0 = (blockIdx.y % groups) * NV;
+  const int nk = min(NV, nrhs - k0);
+  const double* __restrict__ V = vals + inst * P.blob;
+  double* y0 = y + (inst * nrhs + k0) * ylen;
+  double sum[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) sum[k] = 0.0;
+  for (int64_t e = e0 + sh.first; e < e1; e += kSolveUnroll * sh.step) {
+    int32_t j[kSolveUnroll];
+    double m[kSolveUnroll];
+#pragma unroll
+    for (int u = 0; u < kSolveUnroll; ++u) {
+      const int64_t q = e + u * sh.step;
+      j[u] = q < e1 ? (WHICH == 1 ? P.ur_col[q] : (int32_t)P.ri[q]) : -1;
+      m[u] = q < e1 ? (WHICH == 1 ? V[P.ur_slot[q]] : V[q]) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < kSolveUnroll; ++u) {
+      if (j[u] < 0) break;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) sum[k] += m[u] * (k < nk ? y0[k * ylen + j[u]] : 0.0);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    for (int o = 16; o > 0; o >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+    if (sh.cta && threadIdx.x % kWarp == 0) red[k * 8 + threadIdx.x / kWarp] = sum[k];
+  }
+  if (sh.cta) __syncthreads();
+  if (sh.first < nk) {
+    double t = 0.0;
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (sh.first == k) t = sum[k];
+    if (sh.cta) {
+      t = 0.0;
+      for (int w = 0; w < 8; ++w) t += red[sh.first * 8 + w];
+    }
+    y0[sh.first * ylen + c] -= t;
+  }
+}
+
 // Row-wise (pull) forward solves of the deterministic mode, one warp per row; each sum is
 // formed lane by lane over the row's entries and reduced by shuffles, in a fixed order.
 // which 0 (L, unit diagonal): y_r -= sum L(r, c) y_c over the row's entries with c < min(r, t);
@@ -1267,6 +1324,22 @@ void launch_solve_level(const PlanDev& P, const double* vals, int count, int nrh
   if (which == 1) nrhs == 1 ? launch(k_solve_level<1, 1>, 1) : launch(k_solve_level<kSolveVecs, 1>, kSolveVecs);
   if (which == 2) launch(k_solve_level<1, 2>, 1);
   if (which == 3) launch(k_solve_level<1, 3>, 1);
+}
+
+void launch_outer_rows(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                       int64_t ylen, int nrows, int nlong, int which, cudaStream_t s,
+                       LaunchCounter& lc) {
+  if (nrows == 0) return;
+  const unsigned gx = nlong + (nrows - nlong + 7) / 8;
+  const auto launch = [&](auto kern, int nv) {
+    launch_next(kern, dim3(gx, count * ((nrhs + nv - 1) / nv)), 256, 0, s, P, vals, nrhs, y, ylen,
+                nrows, nlong);
+    lc.n++;
+  };
+  if (which == 1 && nrhs == 1) launch(k_outer_rows<1, 1>, 1);
+  else if (which == 1) launch(k_outer_rows<kSolveVecs, 1>, kSolveVecs);
+  else if (nrhs == 1) launch(k_outer_rows<1, 3>, 1);
+  else launch(k_outer_rows<kSolveVecs, 3>, kSolveVecs);
 }
 
 void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, double* y,

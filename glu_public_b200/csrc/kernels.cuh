@@ -179,6 +179,18 @@ void launch_front_flow(const PlanDev& P, const double* vals, int count, int nrhs
 void launch_solve_level(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                         int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                         const FrontLevelSolve& L, int which, cudaStream_t s, LaunchCounter& lc);
+// plans without fronts: whether the sparse columns are solved as a dataflow, one launch per phase
+bool sparse_solve_flows(const PlanDev& P, int count, int nrhs);
+// one such phase (which 0: L, with the rows t .. n of L21; 1: U; 2: U^T; 3: L^T), `items` the sparse
+// columns in the levels' order (trsv.cu)
+void launch_sparse_flow(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                        int64_t ylen, const int32_t* items, int which, double* xbuf, int* err,
+                        int32_t* status, double budget_ms, cudaStream_t s, LaunchCounter& lc);
+// which 1: y_r -= U(r, j) x_j over the columns j >= t of the rows br_rows; which 3: y_c -= L(i, c)
+// x_i over the rows i >= t of the columns lc_cols; the first nlong of the nrows take a CTA each
+void launch_outer_rows(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
+                       int64_t ylen, int nrows, int nlong, int which, cudaStream_t s,
+                       LaunchCounter& lc);
 // values a vector has in the solve's buffer of solved values
 __host__ __device__ inline int64_t solve_buffer(const PlanDev& P) { return 2 * ((int64_t)P.ntp + P.fx_len); }
 void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, double* y,

@@ -74,6 +74,8 @@ struct PlanDev {
   const int32_t *uj_col, *uj_slot;
   const int64_t* ur_ptr;             // [t + 1]
   const int32_t *ur_col, *ur_slot, *ur_rows;
+  const int64_t* lr_ptr;             // [n + 1]
+  const int32_t *lr_col, *lr_slot, *ur_split, *br_rows, *lc_cols;
   const FrontGeom* fgeom;            // [fronts]
   const int32_t* fg_aidx;            // gather / write-back index within an instance's front area
   const int32_t* fc_aidx;            // Schur-complement index within an instance's front area

@@ -111,6 +111,62 @@ int32_t column_lanes(int32_t fixed, const uint32_t* cp, const uint32_t* lp,
   return best;
 }
 
+// Entries right of the diagonal of every row r < t that is in no front.
+void build_u_rows(HostPlan& hp, const std::vector<uint8_t>& in_front) {
+  const uint32_t n = hp.n, t = hp.t;
+  const uint32_t *cp = hp.cp.data(), *ri = hp.ri.data();
+  hp.ur_ptr.assign((size_t)t + 1, 0);
+  for (uint32_t j = 0; j < n; ++j)
+    for (uint32_t p = cp[j]; p < cp[j + 1] && ri[p] < j && ri[p] < t; ++p)
+      if (!in_front[ri[p]]) hp.ur_ptr[ri[p] + 1]++;
+  for (uint32_t r = 0; r < t; ++r) hp.ur_ptr[r + 1] += hp.ur_ptr[r];
+  hp.ur_col.assign(hp.ur_ptr[t], 0);
+  hp.ur_slot.assign(hp.ur_ptr[t], 0);
+  std::vector<int64_t> at(hp.ur_ptr.begin(), hp.ur_ptr.end() - 1);
+  for (uint32_t j = 0; j < n; ++j)
+    for (uint32_t p = cp[j]; p < cp[j + 1] && ri[p] < j && ri[p] < t; ++p)
+      if (!in_front[ri[p]]) {
+        hp.ur_col[at[ri[p]]] = (int32_t)j;
+        hp.ur_slot[at[ri[p]]++] = (int32_t)hp.pos2slot[p];
+      }
+}
+
+// The lists of the sparse solves as a dataflow (plans without fronts).
+void build_flow_solves(HostPlan& hp) {
+  const uint32_t n = hp.n, t = hp.t;
+  const uint32_t *cp = hp.cp.data(), *ri = hp.ri.data(), *lp = hp.lp.data();
+  build_u_rows(hp, std::vector<uint8_t>(t, 0));
+  hp.ur_split.assign(t, 0);
+  hp.br_rows.clear();
+  hp.lc_cols.clear();
+  auto border = [&](int32_t r) { return hp.ur_ptr[r + 1] - hp.ur_ptr[r] - hp.ur_split[r]; };
+  auto below = [&](int32_t c) { return (int64_t)cp[c + 1] - lp[c] - 1 - hp.lsplit[c]; };
+  for (uint32_t r = 0; r < t; ++r) {
+    const auto b = hp.ur_col.begin() + hp.ur_ptr[r], e = hp.ur_col.begin() + hp.ur_ptr[r + 1];
+    hp.ur_split[r] = (int32_t)(std::lower_bound(b, e, (int32_t)t) - b);
+    if (border((int32_t)r) > 0) hp.br_rows.push_back((int32_t)r);
+    if (below((int32_t)r) > 0) hp.lc_cols.push_back((int32_t)r);
+  }
+  hp.br_long = (int32_t)(std::stable_partition(hp.br_rows.begin(), hp.br_rows.end(), [&](int32_t r) {
+                           return border(r) >= (int64_t)kSolveLong;
+                         }) - hp.br_rows.begin());
+  hp.lc_long = (int32_t)(std::stable_partition(hp.lc_cols.begin(), hp.lc_cols.end(), [&](int32_t c) {
+                           return below(c) >= (int64_t)kSolveLong;
+                         }) - hp.lc_cols.begin());
+  hp.lr_ptr.assign((size_t)n + 1, 0);
+  for (uint32_t c = 0; c < t; ++c)
+    for (uint32_t p = lp[c] + 1; p < cp[c + 1]; ++p) hp.lr_ptr[ri[p] + 1]++;
+  for (uint32_t r = 0; r < n; ++r) hp.lr_ptr[r + 1] += hp.lr_ptr[r];
+  hp.lr_col.assign(hp.lr_ptr[n], 0);
+  hp.lr_slot.assign(hp.lr_ptr[n], 0);
+  std::vector<int64_t> at(hp.lr_ptr.begin(), hp.lr_ptr.end() - 1);
+  for (uint32_t c = 0; c < t; ++c)
+    for (uint32_t p = lp[c] + 1; p < cp[c + 1]; ++p) {
+      hp.lr_col[at[ri[p]]] = (int32_t)c;
+      hp.lr_slot[at[ri[p]]++] = (int32_t)hp.pos2slot[p];
+    }
+}
+
 // The solve schedules of a plan with fronts: row blocks and outside products of every level's
 // fronts, and the rows of the single columns (the U solve pulls where there are fronts: every entry
 // above a front's block row is then part of a dense product instead of an atomic of its own).
@@ -175,21 +231,7 @@ void build_front_solves(HostPlan& hp) {
   lists(hp.lfr, hp.lfr_ptr, true, hp.lflow, hp.lflow_ptr, hp.lext, hp.lext_ptr, hp.ldot, hp.ldot_ptr);
   lists(hp.ufr, hp.ufr_ptr, false, hp.uflow, hp.uflow_ptr, hp.uext, hp.uext_ptr, hp.udot,
         hp.udot_ptr);
-  // rows of the single columns
-  hp.ur_ptr.assign((size_t)t + 1, 0);
-  for (uint32_t j = 0; j < n; ++j)
-    for (uint32_t p = cp[j]; p < cp[j + 1] && ri[p] < j && ri[p] < t; ++p)
-      if (!in_front[ri[p]]) hp.ur_ptr[ri[p] + 1]++;
-  for (uint32_t r = 0; r < t; ++r) hp.ur_ptr[r + 1] += hp.ur_ptr[r];
-  hp.ur_col.assign(hp.ur_ptr[t], 0);
-  hp.ur_slot.assign(hp.ur_ptr[t], 0);
-  std::vector<int64_t> at(hp.ur_ptr.begin(), hp.ur_ptr.end() - 1);
-  for (uint32_t j = 0; j < n; ++j)
-    for (uint32_t p = cp[j]; p < cp[j + 1] && ri[p] < j && ri[p] < t; ++p)
-      if (!in_front[ri[p]]) {
-        hp.ur_col[at[ri[p]]] = (int32_t)j;
-        hp.ur_slot[at[ri[p]]++] = (int32_t)hp.pos2slot[p];
-      }
+  build_u_rows(hp, in_front);
   hp.ur_rows = hp.ucols;
   hp.ur_long.assign(hp.ulng.size(), 0);
   for (size_t l = 0; l + 1 < hp.uptr.size(); ++l) {
@@ -802,6 +844,7 @@ int build_host_plan(uint32_t n, uint32_t nnz, const uint32_t* cp, const uint32_t
     build(false, hp.ucols, hp.uptr, hp.ufr, hp.ufr_ptr, hp.ulng);
   }
   if (!hp.fronts.empty()) build_front_solves(hp);
+  else build_flow_solves(hp);
   hp.bord_ptr.assign((size_t)hp.nt + 1, 0);
   hp.bord_row.clear();
   hp.bord_slot.clear();

@@ -115,6 +115,13 @@ struct HostPlan {
   // rows of at least kSolveLong entries first
   std::vector<int64_t> ur_ptr;
   std::vector<int32_t> ur_col, ur_slot, ur_rows, ur_long;
+  // plans without fronts, whose sparse solves may run as a dataflow (trsv.cu): entries of each row
+  // left of min(row, t); of each row's entries right of the diagonal, the number left of t; the
+  // rows with entries right of t and the columns with entries below it, those of at least
+  // kSolveLong first
+  std::vector<int64_t> lr_ptr;
+  std::vector<int32_t> lr_col, lr_slot, ur_split, br_rows, lc_cols;
+  int32_t br_long = 0, lc_long = 0;
   std::vector<int64_t> bord_ptr;
   std::vector<int32_t> bord_row, bord_slot;
   std::vector<int32_t> bord_ckcol;            // chunks of <= 1024 border entries: tail column

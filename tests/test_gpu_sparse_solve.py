@@ -30,8 +30,8 @@ def long_columns(n, seed):
 
 @pytest.mark.parametrize("deterministic", [0, 1])
 @pytest.mark.parametrize("transpose", [False, True])
-@pytest.mark.parametrize("nrhs", [1, 2, 4, 5])
-def test_long_columns(nrhs, transpose, deterministic):
+@pytest.mark.parametrize("nrhs,count", [(1, 2), (2, 2), (4, 2), (5, 2), (1, 200), (5, 100)])
+def test_long_columns(nrhs, count, transpose, deterministic):
     import torch
     n = 1100
     a = long_columns(n, 7)
@@ -43,19 +43,49 @@ def test_long_columns(nrhs, transpose, deterministic):
     assert plan.stat("nt") == 0
     idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
     plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
-    batch = glu.Batch(plan, 2)
-    val = torch.as_tensor(np.stack([sym.val, 2.0 * sym.val]), device="cuda")
-    batch.load_lu_values(val)
+    batch = glu.Batch(plan, count)            # more than 200,000 rows in all: a launch per level
+    scale = torch.linspace(1.0, 2.0, count, dtype=torch.float64, device="cuda")
+    batch.load_lu_values(scale[:, None] * torch.as_tensor(sym.val, device="cuda"))
     batch.refactor(0.0)
-    b = torch.as_tensor(np.random.default_rng(1).standard_normal((2, nrhs, n)), device="cuda")
+    b = torch.as_tensor(np.random.default_rng(1).standard_normal((count, nrhs, n)), device="cuda")
     x = batch.solve(b, transpose=transpose)
     cp = sym.sym_c_ptr.astype(np.int64)
-    for i in range(2):
+    for i in (0, count - 1):
         lu = np.zeros((n, n))                 # [column, row]
         lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
         nl = np.diff(cp) - (sym.l_col_ptr.astype(np.int64) - cp[:-1]) - 1
         assert nl.max() >= 192 and (nl < 192).any()
         check_solve(torch, lu, b[i], x[i], transpose)
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("nrhs,count", [(1, 1), (3, 2), (1, 250)])
+def test_sparse_columns_beside_a_dense_block(nrhs, count, transpose):
+    """L21 and the part of U above the dense block, with rows and columns of more and of fewer entries
+    than give them a CTA."""
+    import torch
+    n = 1100
+    a = long_columns(n, 5)
+    a[n - 260:, n - 260:] += 0.01             # a dense block; row 50 and column 51 reach all of it
+    a[50, n - 260:] = 0.02
+    a[n - 260:, 51] = 0.03
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, front_min_w=0)
+    assert 200 <= plan.stat("nt") < n
+    idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
+    plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
+    batch = glu.Batch(plan, count)
+    batch.load_lu_values(torch.as_tensor(sym.val, device="cuda").repeat(count, 1))
+    batch.refactor(0.0)
+    b = torch.as_tensor(np.random.default_rng(1).standard_normal((count, nrhs, n)), device="cuda")
+    x = batch.solve(b, transpose=transpose)
+    assert not batch.status().any()
+    cp = sym.sym_c_ptr.astype(np.int64)
+    lu = np.zeros((n, n))
+    lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(count - 1).cpu().numpy()
+    check_solve(torch, lu, b[count - 1], x[count - 1], transpose)
 
 
 @pytest.mark.parametrize("options", [{}, dict(sparse_persistent=0), dict(sparse_persistent=0, level_warps_per_sm=0),
