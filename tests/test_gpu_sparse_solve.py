@@ -143,3 +143,39 @@ def test_residual_of_long_rows(transpose):
     den = np.abs(op).sum(1).max() * np.abs(x).max() + np.abs(b).max()
     slack = 2 * n * 2.0 ** -53 * (np.abs(op) @ np.abs(x[0, 0])).max() / den
     assert abs(got - r / den) <= slack + 4 * n * 2.0 ** -53 * r / den
+
+
+@pytest.mark.parametrize("count", [2, 24])
+def test_assembly_of_the_dense_block(count):
+    """Columns of the dense block built from the entries and the sparse columns' products, a CTA each
+    (count 2) or a warp each (24), beside instances loaded in the filled-pattern order:
+    |L U - A| <= 4 n u |L| |U|."""
+    import torch
+    n, tail = 1100, 300
+    rng = np.random.default_rng(9)
+    a = np.zeros((n, n))
+    a[n - tail:, n - tail:] = rng.uniform(-1.0, 1.0, (tail, tail))
+    for c in range(0, n - tail, 7):           # 1 to 100 rows of L21, up to 40 columns of U12 each
+        a[rng.choice(np.arange(n - tail, n), 1 + c % 100, replace=False), c] = 0.1
+        a[c, rng.choice(np.arange(n - tail, n), 1 + c % 40, replace=False)] = -0.2
+    a[np.arange(n), np.arange(n)] = np.abs(a).sum(0) + np.abs(a).sum(1) + 1.0
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, front_min_w=0, hub_min_frac=0.9)
+    nt = plan.stat("nt")
+    assert 200 <= nt < n and 0 < plan.stat("pull_entries") <= 64 * nt
+    assert (plan.stat("ntp") * count >= 32 * 148) == (count == 24)
+    plan.set_ingest(sym.positions(row.astype(np.uint32), ap))
+    batch = glu.Batch(plan, count)
+    scale = np.linspace(1.0, 2.0, count)
+    val = torch.as_tensor(scale[:, None] * a[row, col][None], device="cuda")
+    batch.load_values(val)
+    lu1 = torch.as_tensor(scale[1] * sym.val[None], device="cuda")
+    batch.load_lu_values(lu1, first=1)
+    batch.refactor(0.0)
+    cp = sym.sym_c_ptr.astype(np.int64)
+    for i in (0, 1, count - 1):
+        lu = np.zeros((n, n))                 # [column, row]
+        lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
+        check_lu(torch, lu, np.ascontiguousarray(a.T * scale[i])[None])
