@@ -3,9 +3,9 @@
 //
 // Launch structure of one refactorization (replaces the host loop of LUonDevice,
 // src/numeric.cu:423-596, which launches 1..3*width kernels per level and synchronizes the
-// device after every level): one kernel per sparse level, then two kernels per dense panel,
-// all enqueued on the caller's stream with no host synchronization, so the whole sequence can
-// be captured once in a CUDA graph and replayed.
+// device after every level): one kernel per sparse level (runs of narrow levels in one), then two
+// to four kernels per dense panel, all enqueued on the caller's stream with no host
+// synchronization, so the whole sequence can be captured once in a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
 #include <algorithm>

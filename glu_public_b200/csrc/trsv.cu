@@ -121,6 +121,12 @@ __device__ __forceinline__ double wait_value(const double* p, double v, int* err
   return v;
 }
 
+// The end of a CTA whose wait gave up: its own copies have landed before it returns.
+__device__ __forceinline__ bool gave_up() {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  return false;
+}
+
 // One phase (WHICH as in triangle) of a unit (an instance's nv vectors) for CTA r of G.  rhs: the
 // block's right-hand side, to be waited for if `wait_rhs`; xb: the solved values (vectors xl
 // apart), also written to yd (vectors yl apart) if not null.  Returns false if a wait gave up.
@@ -217,7 +223,7 @@ __device__ bool flow_phase(const double* __restrict__ D, int64_t ld, int nblk, c
         if (e < kB * NV)
           x[(e % kB) * NV + e / kB] = wait_value(xaddr(k, e), xn[h], err, budget_ns, &fail);
       }
-      if (__syncthreads_or(fail)) return false;
+      if (__syncthreads_or(fail)) return gave_up();
       if (k + 1 < o) {
 #pragma unroll
         for (int h = 0; h < NX; ++h)
@@ -254,7 +260,7 @@ __device__ bool flow_phase(const double* __restrict__ D, int64_t ld, int nblk, c
       y0 = wait_value(ry, y0, err, budget_ns, &fail);
       y1 = wait_value(ry + 32, y1, err, budget_ns, &fail);
     }
-    if (__syncthreads_or(fail)) return false;  // sums, triangle and reciprocals are there too
+    if (__syncthreads_or(fail)) return gave_up();  // sums, triangle and reciprocals are there too
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
     for (int q = 0; q < (trans ? 1 : 4); ++q) {
@@ -474,7 +480,7 @@ __device__ bool front_block(const PlanDev& P, const double* __restrict__ V, int 
                                &fail);
       }
     }
-    if (__syncthreads_or(fail)) return false;
+    if (__syncthreads_or(fail)) return gave_up();
     if (k + 1 < o) look(k + 1);
     if (!trans) {
 #pragma unroll

@@ -91,15 +91,17 @@ typedef struct glu_options {
   int32_t update_depth;       /* dense panels per trailing update: each group of this many panels
                                  is factored left-looking inside the group, then the rest of the
                                  block takes one update with K = update_depth * panel, so it is
-                                 read and written once per group (1, 2, 4 or 8; default 8) */
+                                 read and written once per group (1, 2, 4 or 8; default 8); a
+                                 few small blocks are updated whole after every panel instead */
   int32_t sparse_persistent;  /* runs of at least this many consecutive narrow sparse levels
                                  (at most two columns of the batch per SM) without
                                  fronts are factored by ONE cooperative launch that walks the
                                  levels with device-side barriers instead of one launch per
                                  level (0 = never; default 2) */
-  double level_wait_ms;       /* bound of every device-side wait of that launch: a barrier not
-                                 reached within it marks the instances GLU_INST_TIMEOUT and the
-                                 launch returns (default 1000) */
+  double level_wait_ms;       /* bound of every device-side wait, of that launch and of the
+                                 solves (whose rows wait for the values they need within one
+                                 launch): one that lasts longer marks the instances
+                                 GLU_INST_TIMEOUT and the launch returns (default 1000) */
   int32_t wide_level_cols;    /* a level of at least this many columns is "wide" (default 592 =
                                  4 x 148 SMs); with sparse_warps_per_col = 0 wide levels get one
                                  warp per column, narrow levels a CTA per column ... */
