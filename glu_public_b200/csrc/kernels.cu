@@ -158,7 +158,9 @@ __device__ __forceinline__ ColGroup cta_group() {
 // Measured, sparse levels of one refactorization: n = 20,000 1.13 -> 0.39 ms (a few pairs of 2,860
 // updates in columns of 2,850 pairs), 512 x 512 x 2 nodes 9.4 -> 6.8 ms, 64 x n = 20,000 5.6 -> 3.0 ms;
 // sharing long pairs in pieces wherever there are fewer than groups, not a quarter as many: 128 x 128
-// x 2 nodes 2.15 ms against 1.88.
+// x 2 nodes 2.15 ms against 1.88.  Without a dense block, where a column has up to a thousand pairs
+// of a thousand updates: 64 x n = 2,000 8.5 -> 6.1 ms, one n = 4,960 17.2 -> 17.3, four of them 15.9 ->
+// 16.8 (the row loop unrolled by two: 6.95, 19.5 and 16.7).
 __device__ __forceinline__ void apply_pairs(const PlanDev& P, double* __restrict__ V, uint32_t c,
                                             const double* __restrict__ Lc, uint32_t nL, int64_t w,
                                             int64_t W, int il, int width, unsigned mask) {
