@@ -37,6 +37,7 @@
 #include "glu_b200.h"
 #include "kernels.cuh"
 #include "plan_host.h"
+#include "quotient.cuh"
 #include "wait.cuh"
 
 namespace glu {
@@ -128,20 +129,6 @@ __global__ void __launch_bounds__(256) k_dense_diag(DenseView V,
   for (int i = 0; i < R; ++i)
 #pragma unroll
     for (int j = 0; j < R; ++j) D[(tx + 16 * i) + (int64_t)(ty + 16 * j) * ld] = a[i][j];
-}
-
-__device__ __forceinline__ bool finite_bits(double x) {
-  return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
-}
-
-// x / d from r = 1 / d with one FMA correction (Markstein's division: q = x r, e = x - q d,
-// q + e r; Muller et al., Handbook of Floating-Point Arithmetic, 2nd ed., sec. 4.7): within an ulp
-// of x / d, three dependent operations, and no slow path for the zeros a padded or nearly dense
-// block is full of.  An infinite or NaN first quotient (zero pivot, overflow) is returned as it is.
-__device__ __forceinline__ double quotient(double x, double d, double r) {
-  const double q = x * r;
-  const double e = fma(fma(-q, d, x), r, q);
-  return finite_bits(q) ? e : q;
 }
 
 __device__ __forceinline__ void dmma884(double& d0, double& d1, double a, double b) {
@@ -259,7 +246,7 @@ __device__ __forceinline__ void diag64_tile(double* __restrict__ T, int s, int r
 constexpr int kDiagSmem = 64 * kDiagSt + 2 * 64 + 8;   // doubles: T, Ub, Lb, rcp
 
 template <bool PERT>
-__device__ __forceinline__ void diag64_steps(double* T, double pv,
+__device__ __forceinline__ bool diag64_steps(double* T, double pv,
                                              const uint8_t* __restrict__ hasl, int32_t* status,
                                              int b, int np) {
   const int lane = threadIdx.x % kWarp, warp = threadIdx.x / kWarp;
@@ -269,6 +256,7 @@ __device__ __forceinline__ void diag64_steps(double* T, double pv,
   double* rcp = Lb + 64;
   unsigned hm = 0;
   if (PERT) hm = __ballot_sync(0xffffffffu, lane < 8 && hasl[warp * 8 + (lane & 7)] != 0);
+  bool odd = false;
 #pragma unroll 1
   for (int s = 0; s < np; ++s) {
     if (warp == s) diag64_block<PERT>(T, Ub, Lb, rcp, s, lane, pv, hm, status, b);
@@ -280,6 +268,7 @@ __device__ __forceinline__ void diag64_steps(double* T, double pv,
         const int i = e % 8, j = e / 8;
         T[s * 8 * (kDiagSt + 1) + i + j * kDiagSt] = i > j ? Lb[j * 8 + i] : Ub[i * 8 + j];
       }
+      odd = !plain_divisor(Ub[(lane & 7) * 9]);
     }
     __syncthreads();
     if (warp == s + 1) {
@@ -291,14 +280,53 @@ __device__ __forceinline__ void diag64_steps(double* T, double pv,
       for (int r = s + 1; r < 8; ++r) diag64_tile(T, s, r, warp, g, t);
     }
   }
+  return !__syncthreads_or(odd);
+}
+
+// The same factorization of the first nv pivots with true divisions, column by column, for blocks
+// with a pivot whose reciprocal does not stand for it; A (leading dimension ld) is the block.
+__device__ __noinline__ void diag64_divide(double* T, const double* A, int64_t ld, double pv,
+                                           const uint8_t* hasl, int32_t* status, int b, int nv) {
+  for (int e = threadIdx.x; e < 64 * 64; e += 256)
+    T[e % 64 + (e / 64) * kDiagSt] = A[e % 64 + (int64_t)(e / 64) * ld];
+  for (int c = 0; c < nv; ++c) {
+    double* P = T + c * (kDiagSt + 1);
+    __syncthreads();
+    if (threadIdx.x == 0 && pv > 0.0 && hasl[c] && fabs(*P) < pv) {
+      *P = pv;
+      atomicOr(status + b, GLU_INST_PERTURBED);
+    }
+    __syncthreads();
+    for (int i = 1 + threadIdx.x; i < 64 - c; i += 256) P[i] /= *P;
+    __syncthreads();
+    for (int e = threadIdx.x; e < 64 * (63 - c); e += 256) {
+      const int i = e % 64, j = 1 + e / 64;
+      if (i > 0 && i < 64 - c) P[i + j * kDiagSt] -= P[i] * P[j * kDiagSt];
+    }
+  }
   __syncthreads();
 }
 
-__device__ __forceinline__ void diag64(double* T, double pv, const uint8_t* __restrict__ hasl,
-                                       int32_t* status, int b, int nv) {
+// The first n quotients and updates of a row with true divisions: x_c /= U(c, c), then
+// x_j -= x_c U(c, j), x_c = X[c sx], U(c, j) = U[c + j ld].
+__device__ __noinline__ void row_divide(double* X, int64_t sx, const double* U, int ld, int n) {
+#pragma unroll 1
+  for (int c = 0; c < n; ++c) {
+    const double x = X[c * sx] / U[c * (ld + 1)];
+    X[c * sx] = x;
+#pragma unroll 1
+    for (int j = c + 1; j < n; ++j) X[j * sx] -= x * U[c + j * ld];
+  }
+}
+
+// A: where the block lies (leading dimension ld), unchanged so far, read only if it is done over.
+__device__ __forceinline__ void diag64(double* T, const double* A, int64_t ld, double pv,
+                                       const uint8_t* __restrict__ hasl, int32_t* status, int b,
+                                       int nv) {
   const int np = min(8, (nv + 7) / 8);
-  if (pv > 0.0) diag64_steps<true>(T, pv, hasl, status, b, np);
-  else diag64_steps<false>(T, pv, hasl, status, b, np);
+  const bool plain = pv > 0.0 ? diag64_steps<true>(T, pv, hasl, status, b, np)
+                              : diag64_steps<false>(T, pv, hasl, status, b, np);
+  if (!plain) diag64_divide(T, A, ld, pv, hasl, status, b, nv);
   if (threadIdx.x < nv) {
     const double d = T[threadIdx.x * (kDiagSt + 1)];
     if (d == 0.0) atomicOr(status + b, GLU_INST_ZERO_PIVOT);
@@ -319,7 +347,7 @@ __device__ __forceinline__ void diag64_body(const DenseView& V, const double* __
     T[e % 64 + (e / 64) * kDiagSt] = D[e % 64 + (int64_t)(e / 64) * ld];
   }
   __syncthreads();
-  diag64(T, pert[b], V.hasl + k, status, b, min(64, V.nvalid - k));
+  diag64(T, D, ld, pert[b], V.hasl + k, status, b, min(64, V.nvalid - k));
 #pragma unroll
   for (int q = 0; q < 16; ++q) {
     const int e = threadIdx.x + q * 256;
@@ -777,10 +805,21 @@ __device__ __forceinline__ void trsm_mma_body(const DenseView& V, int k, int nrt
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
+  bool odd = false;
   if (lower)
-    for (int c = tid; c < NB; c += WARPS * 32) R[c] = 1.0 / T[c * (TS + 1)];
-  __syncthreads();
+    for (int c = tid; c < NB; c += WARPS * 32) {
+      const double d = T[c * (TS + 1)];
+      R[c] = 1.0 / d;
+      odd |= !plain_divisor(d);
+    }
+  odd = __syncthreads_or(odd);
   if (first >= extent) return;
+  if (odd) {
+    if (first + lane < extent)
+      row_divide(D + (int64_t)(k + NB + first + lane) + (int64_t)k * ld, ld, T, TS,
+                 min(NB, V.nvalid - k));
+    return;
+  }
   __syncwarp();
   const int nblk = min(NBLK, (V.nvalid - k + 7) / 8);   // blocks past it: padding, stay zero
 #pragma unroll 1
@@ -900,9 +939,18 @@ __device__ __forceinline__ void trsm8_body(const DenseView& V, int k, int mt, in
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
+  bool odd = false;
   if (lower) {
-    if (tid < 64) R[tid] = 1.0 / T[tid * (ST + 1)];
-    __syncthreads();
+    if (tid < 64) {
+      const double d = T[tid * (ST + 1)];
+      R[tid] = 1.0 / d;
+      odd = !plain_divisor(d);
+    }
+    odd = __syncthreads_or(odd);
+  }
+  if (odd) {
+    if (tid < 64) row_divide(Xg + tid, ld, T, ST, min(64, V.nvalid - k));
+    return;
   }
   const int xr = lower ? 1 : ST, xc = lower ? ST : 1;   // X(r, c) = X[r * xr + c * xc]
   const int sk = lower ? 1 : ST, sn = lower ? ST : 1;   // B operand: T(kk, n) = T[kk * sk + n * sn]
@@ -1052,17 +1100,15 @@ __device__ __forceinline__ void step_body(const DenseView& V, const double* __re
   cp_async_wait<0>();
   __syncthreads();
   if (kv > 48) steps(3);
-  if (ti > 0 || tj > 0 || k + 64 >= V.nvalid) {
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
+  for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-      for (int ni = 0; ni < 2; ++ni)
+    for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-          C[(wm + mi * 8) + (int64_t)(wn + ni * 8 + (lane & 3) * 2 + e) * ld] =
-              neg(acc[mi][ni][e]);
-    return;
-  }
+      for (int e = 0; e < 2; ++e)
+        C[(wm + mi * 8) + (int64_t)(wn + ni * 8 + (lane & 3) * 2 + e) * ld] =
+            neg(acc[mi][ni][e]);
+  if (ti > 0 || tj > 0 || k + 64 >= V.nvalid) return;
   // the next panel's diagonal block, in shared memory
   __syncthreads();                            // every warp is done with As and Bs
 #pragma unroll
@@ -1073,7 +1119,7 @@ __device__ __forceinline__ void step_body(const DenseView& V, const double* __re
       for (int e = 0; e < 2; ++e)
         As[(wn + ni * 8 + (lane & 3) * 2 + e) * ST + wm + mi * 8] = neg(acc[mi][ni][e]);
   __syncthreads();
-  diag64(As, pert[b], V.hasl + k + 64, status, b, min(64, V.nvalid - k - 64));
+  diag64(As, C, ld, pert[b], V.hasl + k + 64, status, b, min(64, V.nvalid - k - 64));
 #pragma unroll
   for (int q = 0; q < 16; ++q) {
     const int e = tid + q * 256;

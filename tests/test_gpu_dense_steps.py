@@ -80,3 +80,52 @@ def test_bad_and_perturbed_pivots_of_a_panel(pivot):
     assert lu[pivot, pivot] == 1e-3 and not lu[pivot, pivot + 1:].any()
     a[1, pivot, pivot] = 1e-3
     check_lu(torch, lu[None], a[1:2])
+
+
+def lone_pivot(n, count, k, value, below):
+    """`matrices` with pivot k of `value`: nothing left of it or above it, `below` under it."""
+    a = matrices(n, count, 11)
+    a[:, :k, k] = 0.0
+    a[:, k, :k] = 0.0
+    a[:, k, k] = value
+    a[:, k, k + 1:] = below(n - k - 1)
+    return a
+
+
+@pytest.mark.parametrize("n,count,pivot", [(40, 1, 0), (64, 2, 9), (64, 1, 37), (130, 1, 3), (130, 2, 70),
+                                           (129, 401, 20)])
+def test_pivot_without_a_finite_reciprocal(n, count, pivot):
+    """1 / d overflows for a pivot below 2^-1024; the quotients with it, of the block and of the rows
+    below, are ordinary numbers: |L(i, k) - a / d| <= u |a / d| and |L U - A| <= 4 n u |L| |U|, each
+    plus a subnormal's rounding."""
+    import torch
+    d = 3e-310
+    rng = np.random.default_rng(0)
+    a = lone_pivot(n, count, pivot, d, lambda m: rng.uniform(-1.0, 1.0, m) * d)
+    batch = glu.Batch(glu.Plan(dense_symbolic(n), dense_min=1), count)
+    batch.load_lu_values(torch.as_tensor(a.reshape(count, -1), device="cuda"))
+    batch.refactor(0.0)
+    assert not batch.status().any()
+    lu = batch.get_lu(count - 1).cpu().numpy().reshape(n, n)
+    want = a[-1, pivot, pivot + 1:] / d
+    assert (np.abs(lu[pivot, pivot + 1:] - want) <= 2 * U * np.abs(want)).all()
+    m = torch.as_tensor(lu, device="cuda").T
+    lo, up = torch.tril(m, -1) + torch.eye(n, dtype=m.dtype, device=m.device), torch.triu(m)
+    err = (lo @ up - torch.as_tensor(a[-1], device="cuda").T).abs()
+    assert bool((err <= 4 * n * U * (lo.abs() @ up.abs()) + 2 * n * 2.0 ** -1074).all())
+
+
+@pytest.mark.parametrize("n,pivot", [(40, 0), (64, 37), (130, 3), (130, 70)])
+def test_infinite_pivot(n, pivot):
+    """Quotients with an infinite pivot are zero, so the other pivots' factors are those of the matrix
+    without its row and column; the instance is flagged."""
+    import torch
+    a = lone_pivot(n, 1, pivot, np.inf, lambda m: np.linspace(1.0, 2.0, m))
+    batch = glu.Batch(glu.Plan(dense_symbolic(n), dense_min=1), 1)
+    batch.load_lu_values(torch.as_tensor(a.reshape(1, -1), device="cuda"))
+    batch.refactor(0.0)
+    assert batch.status()[0] == 2
+    lu = batch.get_lu(0).cpu().numpy().reshape(n, n)
+    assert not lu[pivot, pivot + 1:].any()
+    rest = np.delete(np.arange(n), pivot)
+    check_lu(torch, lu[np.ix_(rest, rest)][None], a[:, rest][:, :, rest])
