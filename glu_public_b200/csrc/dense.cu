@@ -284,11 +284,18 @@ __device__ __forceinline__ bool diag64_steps(double* T, double pv,
 }
 
 // The same factorization of the first nv pivots with true divisions, column by column, for blocks
-// with a pivot whose reciprocal does not stand for it; A (leading dimension ld) is the block.
-__device__ __noinline__ void diag64_divide(double* T, const double* A, int64_t ld, double pv,
+// with a pivot whose reciprocal does not stand for it.  The block is made again from what lies in
+// memory: C less the product of the kv columns at A with the kv rows at B (leading dimensions ld).
+__device__ __noinline__ void diag64_divide(double* T, const double* C, const double* A,
+                                           const double* B, int kv, int64_t ld, double pv,
                                            const uint8_t* hasl, int32_t* status, int b, int nv) {
-  for (int e = threadIdx.x; e < 64 * 64; e += 256)
-    T[e % 64 + (e / 64) * kDiagSt] = A[e % 64 + (int64_t)(e / 64) * ld];
+  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
+    const int i = e % 64;
+    const int64_t j = e / 64;
+    double x = -C[i + j * ld];
+    for (int q = 0; q < kv; ++q) x += A[i + q * ld] * B[q + j * ld];
+    T[i + j * kDiagSt] = -x;
+  }
   for (int c = 0; c < nv; ++c) {
     double* P = T + c * (kDiagSt + 1);
     __syncthreads();
@@ -297,8 +304,9 @@ __device__ __noinline__ void diag64_divide(double* T, const double* A, int64_t l
       atomicOr(status + b, GLU_INST_PERTURBED);
     }
     __syncthreads();
-    for (int i = 1 + threadIdx.x; i < 64 - c; i += 256) P[i] /= *P;
+    if (const int i = 1 + threadIdx.x; i < 64 - c) P[i] /= *P;
     __syncthreads();
+#pragma unroll 1
     for (int e = threadIdx.x; e < 64 * (63 - c); e += 256) {
       const int i = e % 64, j = 1 + e / 64;
       if (i > 0 && i < 64 - c) P[i + j * kDiagSt] -= P[i] * P[j * kDiagSt];
@@ -319,14 +327,15 @@ __device__ __noinline__ void row_divide(double* X, int64_t sx, const double* U, 
   }
 }
 
-// A: where the block lies (leading dimension ld), unchanged so far, read only if it is done over.
-__device__ __forceinline__ void diag64(double* T, const double* A, int64_t ld, double pv,
+// C, A, B, kv, ld: what the block T was made from (see diag64_divide).
+__device__ __forceinline__ void diag64(double* T, const double* C, const double* A,
+                                       const double* B, int kv, int64_t ld, double pv,
                                        const uint8_t* __restrict__ hasl, int32_t* status, int b,
                                        int nv) {
   const int np = min(8, (nv + 7) / 8);
   const bool plain = pv > 0.0 ? diag64_steps<true>(T, pv, hasl, status, b, np)
                               : diag64_steps<false>(T, pv, hasl, status, b, np);
-  if (!plain) diag64_divide(T, A, ld, pv, hasl, status, b, nv);
+  if (!plain) diag64_divide(T, C, A, B, kv, ld, pv, hasl, status, b, nv);
   if (threadIdx.x < nv) {
     const double d = T[threadIdx.x * (kDiagSt + 1)];
     if (d == 0.0) atomicOr(status + b, GLU_INST_ZERO_PIVOT);
@@ -347,7 +356,7 @@ __device__ __forceinline__ void diag64_body(const DenseView& V, const double* __
     T[e % 64 + (e / 64) * kDiagSt] = D[e % 64 + (int64_t)(e / 64) * ld];
   }
   __syncthreads();
-  diag64(T, D, ld, pert[b], V.hasl + k, status, b, min(64, V.nvalid - k));
+  diag64(T, D, D, D, 0, ld, pert[b], V.hasl + k, status, b, min(64, V.nvalid - k));
 #pragma unroll
   for (int q = 0; q < 16; ++q) {
     const int e = threadIdx.x + q * 256;
@@ -948,10 +957,6 @@ __device__ __forceinline__ void trsm8_body(const DenseView& V, int k, int mt, in
     }
     odd = __syncthreads_or(odd);
   }
-  if (odd) {
-    if (tid < 64) row_divide(Xg + tid, ld, T, ST, min(64, V.nvalid - k));
-    return;
-  }
   const int xr = lower ? 1 : ST, xc = lower ? ST : 1;   // X(r, c) = X[r * xr + c * xc]
   const int sk = lower ? 1 : ST, sn = lower ? ST : 1;   // B operand: T(kk, n) = T[kk * sk + n * sn]
   double* __restrict__ Xw = X + warp * 8 * xr;          // the warp's 8 rows
@@ -989,6 +994,10 @@ __device__ __forceinline__ void trsm8_body(const DenseView& V, int k, int mt, in
       for (int j = 0; j < 8; ++j) Xw[lane * xr + (c0 + j) * xc] = x[j];
     }
     __syncwarp();
+  }
+  if (odd) {
+    if (tid < 64) row_divide(Xg + tid, ld, T, ST, min(64, V.nvalid - k));
+    return;
   }
   __syncthreads();
   for (int idx = tid; idx < 64 * 64; idx += 256) {
@@ -1100,15 +1109,17 @@ __device__ __forceinline__ void step_body(const DenseView& V, const double* __re
   cp_async_wait<0>();
   __syncthreads();
   if (kv > 48) steps(3);
+  if (ti > 0 || tj > 0 || k + 64 >= V.nvalid) {
 #pragma unroll
-  for (int mi = 0; mi < 4; ++mi)
+    for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-    for (int ni = 0; ni < 2; ++ni)
+      for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
-        C[(wm + mi * 8) + (int64_t)(wn + ni * 8 + (lane & 3) * 2 + e) * ld] =
-            neg(acc[mi][ni][e]);
-  if (ti > 0 || tj > 0 || k + 64 >= V.nvalid) return;
+        for (int e = 0; e < 2; ++e)
+          C[(wm + mi * 8) + (int64_t)(wn + ni * 8 + (lane & 3) * 2 + e) * ld] =
+              neg(acc[mi][ni][e]);
+    return;
+  }
   // the next panel's diagonal block, in shared memory
   __syncthreads();                            // every warp is done with As and Bs
 #pragma unroll
@@ -1119,7 +1130,7 @@ __device__ __forceinline__ void step_body(const DenseView& V, const double* __re
       for (int e = 0; e < 2; ++e)
         As[(wn + ni * 8 + (lane & 3) * 2 + e) * ST + wm + mi * 8] = neg(acc[mi][ni][e]);
   __syncthreads();
-  diag64(As, C, ld, pert[b], V.hasl + k + 64, status, b, min(64, V.nvalid - k - 64));
+  diag64(As, C, A, B, kv, ld, pert[b], V.hasl + k + 64, status, b, min(64, V.nvalid - k - 64));
 #pragma unroll
   for (int q = 0; q < 16; ++q) {
     const int e = tid + q * 256;
