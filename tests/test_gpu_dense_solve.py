@@ -78,6 +78,71 @@ def test_pivots_at_the_edge_of_the_exponent_range(transpose):
     np.testing.assert_allclose(xs[1], xs[0], rtol=8 * n * U * cond, atol=0)
 
 
+# (diagonal, entry, x of the entry's column, right-hand side, solution) of a row with one entry
+EXTREME = {
+    "quotient_overflows": (2.0 ** -900, 2.0 ** 200, 0.0, 2.0 ** -899, 2.0),
+    "cancels_before_the_division": (2.0 ** -900, 2.0 ** 200, 1.0, 2.0 ** 200, 0.0),
+    "quotient_underflows": (2.0 ** 900, 2.0 ** -200, 2.0 ** 150, 0.0, -2.0 ** -950),
+    "reciprocal_overflows": (3e-310, 2.0 ** -3, 0.0, 6e-310, 2.0),
+    "infinite": (np.inf, 1.0, 1.0, 3.0, 0.0),
+}
+
+
+@pytest.mark.parametrize("case", EXTREME)
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("front", [False, True])
+@pytest.mark.parametrize("k,j", [(10, 50), (70, 100), (129, 139)])
+def test_rows_of_extreme_exponents(case, transpose, front, k, j):
+    """A row of U whose division by its diagonal overflows or underflows, or has no reciprocal, beside
+    ordinary rows and beside a right-hand side of NaN: the row's solution is exact, the others'
+    within 8 n u cond."""
+    import torch
+    n = 140
+    d, entry, xj, bk, xk = EXTREME[case]
+    a = matrices(n, 1, 3)[0]
+    m = np.where(np.arange(n)[:, None] <= np.arange(n)[None, :], a.T, 0.0)   # upper, row, column
+    if transpose:
+        k, j = j, k                           # row k of U^T: column k of U
+    for p in (k, j):
+        m[p, :] = m[:, p] = 0.0
+    m[j, j] = 1.0
+    rest = np.delete(np.arange(n), [k, j])
+    cond = np.abs(m).sum() / np.abs(np.diag(m))[rest].min()
+    m[(j, k) if transpose else (k, j)] = entry
+    m[k, k] = d
+    rng = np.random.default_rng(2)
+    b = rng.standard_normal((1, 3, n))
+    b[0, :, k], b[0, :, j] = bk, xj
+    b[0, 1] = np.nan
+    sub = (m.T if transpose else m)[np.ix_(rest, rest)]
+    want = np.linalg.solve(sub, b[0][:, rest].T).T
+    size = n + 30 if front else n             # the rows and columns of a front and some outside it
+    full = np.eye(size)
+    full[:n, :n] = m
+    if front:
+        pattern = np.eye(size)
+        pattern[:n, :n] = pattern[[n + 9, n + 19], :n] = pattern[:n, [n + 4, n + 14]] = 1.0
+        col, row = np.nonzero(pattern.T)
+        sym = glu.SymbolicMatrix(size).analyze(
+            row.astype(np.uint32), np.searchsorted(col, np.arange(size + 1)).astype(np.uint32))
+        plan = glu.Plan(sym, dense_threshold=2.0, front_min_flops=1.0)
+        idx, one = np.arange(size, dtype=np.uint32), np.ones(size)
+        plan.set_solve_maps(glu.NicsluArrays(size, idx, idx, idx, idx, one, one, 0))
+        assert plan.stat("front_w_max") == n
+    else:
+        plan = plan_for(n)
+    batch = glu.Batch(plan, 1)
+    col = np.repeat(np.arange(size), np.diff(plan.sym.sym_c_ptr.astype(np.int64)))
+    batch.load_lu_values(torch.as_tensor(full[plan.sym.sym_r_idx, col][None], device="cuda"))
+    batch.refactor(0.0)
+    b = np.concatenate([b, np.zeros((1, 3, size - n))], 2)
+    x = batch.solve(torch.as_tensor(b, device="cuda"), transpose=transpose)[0].cpu().numpy()
+    for v in (0, 2):
+        assert x[v, k] == xk and x[v, j] == xj
+        np.testing.assert_allclose(x[v, rest], want[v], rtol=8 * n * U * cond, atol=0)
+    assert np.isnan(x[1, :n]).all()
+
+
 def test_waits_of_the_dense_solve_are_bounded():
     """With a bound of a nanosecond a wait gives up: the instances are flagged, the launch ends and
     the context stays usable."""
