@@ -625,7 +625,11 @@ __global__ void __launch_bounds__(256, NV * (WHICH >= 2 ? 2 : 1) >= 8 ? 1 : 2)
     if (!front_block<NV, WHICH>(P, vals + (int64_t)inst * P.blob, item.x, item.y, y + vec * ylen,
                                 ylen, xf + vec * xl + P.fx0[item.x], xl, min(NV, nrhs - v0), err,
                                 budget_ns, sm)) {
-      if (threadIdx.x == 0) atomicOr(status + inst, GLU_INST_TIMEOUT);
+      // a wait gave up: this item and the CTA's later ones are void, and the last block of a front
+      // has nobody waiting for it who would notice
+      if (threadIdx.x == 0)
+        for (; it < nitems * units; it += gridDim.x)
+          atomicOr(status + (int)(it % units) / chunks, GLU_INST_TIMEOUT);
       return;
     }
   }

@@ -70,3 +70,42 @@ def test_front_solves(nrhs, transpose, dense_threshold):
         lu = np.zeros((n, n))                 # [column, row]
         lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
         check_solve(torch, lu, b[i], x[i], transpose)
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("count", [24, 40, 57])
+def test_instances_behind_a_wait_that_gave_up(count, transpose):
+    """A front of eleven row blocks in more instances than the GPU takes at once, with a bound of a
+    nanosecond: the first instance's diagonals are at the bottom of the exponent range, so that its
+    blocks take long and the waits for them give up.  Whatever a CTA that gave up had left to do
+    belongs to other instances too: each is flagged or right."""
+    import torch
+    w, n = 700, 760
+    rng = np.random.default_rng(4)
+    a = np.eye(n)
+    a[:w, :w] = a[720:740, :w] = a[:w, 710:730] = 1.0
+    a *= rng.uniform(-1.0, 1.0, a.shape)
+    a[np.arange(n), np.arange(n)] = np.abs(a).sum(0) + np.abs(a).sum(1) + 1.0
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, dense_threshold=2.0, front_min_flops=1.0, level_wait_ms=1e-6)
+    assert plan.stat("front_w_max") == w
+    idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
+    plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
+    batch = glu.Batch(plan, count)
+    scale = np.ones(count)
+    scale[0] = 2.0 ** -990
+    b = torch.as_tensor(rng.standard_normal((count, 1, n)), device="cuda")
+    b[0] *= 2.0 ** -990
+    batch.load_lu_values(torch.as_tensor(scale[:, None] * sym.val[None], device="cuda"))
+    batch.refactor(0.0)
+    x = batch.solve(b, transpose=transpose)
+    flagged = batch.status() & 8
+    assert flagged[0]
+    cp = sym.sym_c_ptr.astype(np.int64)
+    col = np.repeat(np.arange(n), np.diff(cp))
+    for i in np.flatnonzero(flagged == 0):
+        lu = np.zeros((n, n))                 # [column, row]
+        lu[col, sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
+        check_solve(torch, lu, b[i], x[i], transpose)
