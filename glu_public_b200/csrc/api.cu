@@ -317,7 +317,8 @@ int ensure_refine_workspace(glu_batch_t b, int64_t vectors, cudaStream_t s) {
   return GLU_OK;
 }
 
-int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose, cudaStream_t s);
+int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose, bool fresh,
+             cudaStream_t s);
 
 // `steps` rounds of iterative refinement on the ORIGINAL matrix: r = b - op(A) x, solve
 // op(A) d = r with the factors, x += d.  resid (may be null): final relative residuals.
@@ -329,7 +330,7 @@ int do_refine(glu_batch_t b, int nrhs, const double* a, const double* B, double*
   glu::LaunchCounter lc;
   for (int it = 0; it < steps; ++it) {
     glu::launch_residual(P, b->count, nrhs, a, X, B, b->rbuf, b->norms, nullptr, transpose, s, lc);
-    if ((st = do_solve(b, nrhs, b->rbuf, b->rbuf, transpose, s))) return st;
+    if ((st = do_solve(b, nrhs, b->rbuf, b->rbuf, transpose, false, s))) return st;
     lc.n += b->launches;
     glu::launch_axpy((int64_t)b->count * nrhs * P.n, b->rbuf, X, s, lc);
   }
@@ -339,7 +340,9 @@ int do_refine(glu_batch_t b, int nrhs, const double* a, const double* B, double*
   return glu::cuda_status("refine");
 }
 
-int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose, cudaStream_t s) {
+// fresh: a solve of its own, which clears the mark of an earlier one whose waits gave up
+int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose, bool fresh,
+             cudaStream_t s) {
   glu_plan_s* pl = b->plan;
   const glu::PlanDev& P = pl->P;
   const glu::HostPlan& hp = pl->hp;
@@ -350,7 +353,8 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
   const int64_t yl = b->ylen;
   const int cnt = b->count;
   int* serr = reinterpret_cast<int*>(b->xbuf + glu::solve_buffer(P) * b->y_vectors);
-  glu::launch_solve_permute_in(P, cnt, nrhs, B, y, yl, transpose, b->xbuf, serr, s, lc);
+  glu::launch_solve_permute_in(P, cnt, nrhs, B, y, yl, transpose, b->xbuf, serr, b->status, fresh, s,
+                               lc);
   auto dense = [&] {
     glu::launch_dense_solve(P, b->vals, cnt, nrhs, y, yl, transpose != 0, b->xbuf, serr, b->status,
                             b->pwait_ms, s, lc);
@@ -431,7 +435,7 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
     dense();
     for (int l = nl - 1; l >= 0; --l) lvl(true, l, 3);
   }
-  glu::launch_solve_permute_out(P, cnt, nrhs, y, X, yl, transpose, s, lc);
+  glu::launch_solve_permute_out(P, cnt, nrhs, y, X, yl, transpose, b->status, s, lc);
   b->launches = lc.n;
   return glu::cuda_status("solve launch");
 }
@@ -1350,6 +1354,8 @@ int glu_batch_status(glu_batch_t b, int32_t* flags, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   cudaMemcpyAsync(flags, b->status, sizeof(int32_t) * b->count, cudaMemcpyDeviceToHost, s);
   cudaStreamSynchronize(s);
+  for (int i = 0; i < b->count; ++i)
+    if (flags[i] & glu::kSolveGaveUp) flags[i] = (flags[i] & ~glu::kSolveGaveUp) | GLU_INST_TIMEOUT;
   return glu::cuda_status("status");
 }
 
@@ -1361,7 +1367,7 @@ int glu_solve(glu_batch_t b, int32_t nrhs, const double* B_dev, double* X_dev, i
   if (!b->plan->has_solve) return set_error(GLU_NOT_READY, "no solve maps (glu_plan_set_solve_maps)");
   if (!b->factored) return set_error(GLU_NOT_READY, "solve before refactor");
   glu::DeviceGuard g(b->plan->device);
-  return do_solve(b, nrhs, B_dev, X_dev, transpose, (cudaStream_t)stream);
+  return do_solve(b, nrhs, B_dev, X_dev, transpose, true, (cudaStream_t)stream);
 }
 
 int glu_residual(glu_batch_t b, int32_t nrhs, const double* a_dev, const double* B_dev,
@@ -1459,7 +1465,7 @@ int glu_graph_capture(glu_batch_t b, const double* a_dev, int32_t nrhs, const do
   int st = do_refactor(b, pert, s);
   int64_t total = lc.n + b->launches;
   if (st == GLU_OK && nrhs > 0) {
-    st = do_solve(b, nrhs, B_dev, X_dev, 0, s);
+    st = do_solve(b, nrhs, B_dev, X_dev, 0, true, s);
     total += b->launches;
   }
   if (st == GLU_OK && refine_steps > 0) {
@@ -1598,7 +1604,7 @@ int glu_group_capture(int32_t nbatch, const glu_batch_t* batches, const double* 
     st = do_refactor(b, pert, bs);
     total += lc.n + b->launches;
     if (st == GLU_OK && nrhs[i] > 0) {
-      st = do_solve(b, nrhs[i], B_dev[i], X_dev[i], 0, bs);
+      st = do_solve(b, nrhs[i], B_dev[i], X_dev[i], 0, true, bs);
       total += b->launches;
     }
     if (st == GLU_OK && nrhs[i] > 0 && refine_steps > 0) {

@@ -501,12 +501,17 @@ __global__ void __launch_bounds__(256) k_sparse_persistent(PlanDev P, double* va
 // solves
 // ---------------------------------------------------------------------------------------------
 
-// Also marks the vector's values of the dense solve unsolved and clears its failure word.
+// Also marks the vector's values of the dataflow solves unsolved and clears their failure word and,
+// if `fresh`, the instances' kSolveGaveUp.
 __global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm, double* y,
-                             int64_t ylen, int transpose, double* xbuf, int* err) {
+                             int64_t ylen, int transpose, double* xbuf, int* err, int32_t* status,
+                             int fresh) {
   after_previous();
   const int64_t v = blockIdx.y;                 // instance * nrhs + rhs
-  if (blockIdx.x == 0 && v == 0 && threadIdx.x == 0) *err = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (v == 0) *err = 0;
+    if (fresh && v % nrhs == 0) atomicAnd(status + v / nrhs, ~kSolveGaveUp);
+  }
   const int64_t nx = solve_buffer(P);
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nx;
        k += (int64_t)gridDim.x * blockDim.x)
@@ -530,11 +535,17 @@ __global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm,
 }
 
 __global__ void k_permute_out(PlanDev P, int nrhs, const double* __restrict__ y, double* X,
-                              int64_t ylen, int transpose) {
+                              int64_t ylen, int transpose, const int32_t* status) {
   after_previous();
   const int64_t v = blockIdx.y;
   const double* yv = y + v * ylen;
   double* xv = X + v * P.n;
+  if (*(const volatile int32_t*)(status + v / nrhs) & kSolveGaveUp) {   // not a solution
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < P.n;
+         k += (int64_t)gridDim.x * blockDim.x)
+      xv[k] = __longlong_as_double(kNaN);
+    return;
+  }
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < P.n;
        k += (int64_t)gridDim.x * blockDim.x) {
     if (!transpose) {            // symbolic.cc:238-245
@@ -1256,17 +1267,18 @@ void launch_sparse_persistent(const PlanDev& P, double* vals, int count, const d
 }
 
 void launch_solve_permute_in(const PlanDev& P, int count, int nrhs, const double* B, double* y,
-                             int64_t ylen, int transpose, double* xbuf, int* err, cudaStream_t s,
-                             LaunchCounter& lc) {
+                             int64_t ylen, int transpose, double* xbuf, int* err, int32_t* status,
+                             bool fresh, cudaStream_t s, LaunchCounter& lc) {
   launch_next(k_permute_in, dim3(grid1(ylen, 256, 256), count * nrhs), 256, 0, s, P, nrhs, B, y,
-              ylen, transpose, xbuf, err);
+              ylen, transpose, xbuf, err, status, fresh ? 1 : 0);
   lc.n++;
 }
 
 void launch_solve_permute_out(const PlanDev& P, int count, int nrhs, const double* y, double* X,
-                              int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc) {
+                              int64_t ylen, int transpose, const int32_t* status, cudaStream_t s,
+                              LaunchCounter& lc) {
   launch_next(k_permute_out, dim3(grid1(P.n, 256, 256), count * nrhs), 256, 0, s, P, nrhs, y, X,
-              ylen, transpose);
+              ylen, transpose, status);
   lc.n++;
 }
 

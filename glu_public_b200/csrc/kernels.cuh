@@ -143,12 +143,19 @@ void launch_gemm_sub(int M, int N, int K, const double* A, int lda, const double
                      double* C, int ldc, int count, int64_t strideA, int64_t strideB,
                      int64_t strideC, cudaStream_t s, LaunchCounter& lc, int variant);
 
+// An instance's status bit (not one of the interface's; glu_batch_status reports it as
+// GLU_INST_TIMEOUT): a wait of the solve gave up.
+constexpr int32_t kSolveGaveUp = 1 << 8;
+
 // solves; y: [count][nrhs][ylen] workspace, ylen = n + (ntp - nt)
+// fresh: clears kSolveGaveUp first (a solve of its own, not one of a refinement)
 void launch_solve_permute_in(const PlanDev& P, int count, int nrhs, const double* B, double* y,
-                             int64_t ylen, int transpose, double* xbuf, int* err, cudaStream_t s,
-                             LaunchCounter& lc);
+                             int64_t ylen, int transpose, double* xbuf, int* err, int32_t* status,
+                             bool fresh, cudaStream_t s, LaunchCounter& lc);
+// the vectors of an instance with kSolveGaveUp are NaN
 void launch_solve_permute_out(const PlanDev& P, int count, int nrhs, const double* y, double* X,
-                              int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc);
+                              int64_t ylen, int transpose, const int32_t* status, cudaStream_t s,
+                              LaunchCounter& lc);
 // one solve level; its first nlong columns take a CTA each (see kSolveLong, plan_host.h)
 void launch_sparse_lsolve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                           int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
@@ -197,7 +204,7 @@ void launch_border(const PlanDev& P, const double* vals, int count, int nrhs, do
                    int64_t ylen, int transpose, cudaStream_t s, LaunchCounter& lc);
 // L then U (transpose: U^T then L^T) of the dense block for every vector, one cooperative launch
 // (trsv.cu); xbuf, err: solve_buffer values a vector and the failure word, set up by
-// launch_solve_permute_in; a wait of more than budget_ms marks the instances GLU_INST_TIMEOUT
+// launch_solve_permute_in; a wait of more than budget_ms marks the instances kSolveGaveUp
 void launch_dense_solve(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                         int64_t ylen, bool transpose, double* xbuf, int* err, int32_t* status,
                         double budget_ms, cudaStream_t s, LaunchCounter& lc);

@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(256, NV * (TRANS ? 2 : 1) >= 8 ? 1 : 2)
                                       budget_ns, sm);
     if (!ok) {                                // a wait gave up: this unit and the rest are void
       if (threadIdx.x == 0)
-        for (int w = u; w < units; w += groups) atomicOr(status + w / chunks, GLU_INST_TIMEOUT);
+        for (int w = u; w < units; w += groups) atomicOr(status + w / chunks, kSolveGaveUp);
       return;
     }
   }
@@ -629,7 +629,7 @@ __global__ void __launch_bounds__(256, NV * (WHICH >= 2 ? 2 : 1) >= 8 ? 1 : 2)
       // has nobody waiting for it who would notice
       if (threadIdx.x == 0)
         for (; it < nitems * units; it += gridDim.x)
-          atomicOr(status + (int)(it % units) / chunks, GLU_INST_TIMEOUT);
+          atomicOr(status + (int)(it % units) / chunks, kSolveGaveUp);
       return;
     }
   }
@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(256) k_sparse_flow(PlanDev P, const double* va
       }
       if (__any_sync(0xffffffffu, fail)) {    // a wait gave up: this unit and the rest are void
         if (lane == 0)
-          for (int w = u; w < units; w += groups) atomicOr(status + w / chunks, GLU_INST_TIMEOUT);
+          for (int w = u; w < units; w += groups) atomicOr(status + w / chunks, kSolveGaveUp);
         return;
       }
       double s = 0.0;

@@ -49,7 +49,7 @@ extern "C" {
 #define GLU_INST_ZERO_PIVOT   1
 #define GLU_INST_NAN_PIVOT    2
 #define GLU_INST_PERTURBED    4
-#define GLU_INST_TIMEOUT      8
+#define GLU_INST_TIMEOUT      8   /* until the next glu_refactor, or, set by a solve, glu_solve */
 
 typedef struct glu_symbolic_s* glu_symbolic_t;
 typedef struct glu_plan_s* glu_plan_t;
@@ -101,7 +101,8 @@ typedef struct glu_options {
   double level_wait_ms;       /* bound of every device-side wait, of that launch and of the
                                  solves (whose rows wait for the values they need within one
                                  launch): one that lasts longer marks the instances
-                                 GLU_INST_TIMEOUT and the launch returns (default 1000) */
+                                 GLU_INST_TIMEOUT and the launch returns (default 1000);
+                                 what a marked instance gets from the solve is NaN */
   int32_t wide_level_cols;    /* a level of at least this many columns is "wide" (default 592 =
                                  4 x 148 SMs); with sparse_warps_per_col = 0 wide levels get one
                                  warp per column, narrow levels a CTA per column ... */
@@ -256,7 +257,8 @@ int glu_batch_status(glu_batch_t b, int32_t* flags, void* stream);
 
 /* Solves A_i X_i = B_i for every instance i with nrhs right-hand sides (Symbolic_Matrix::solve
  * semantics).  B_dev, X_dev: [count][nrhs][n] doubles (column-major per instance).
- * transpose != 0 solves A_i^T X_i = B_i (the adjoint).  X may alias B. */
+ * transpose != 0 solves A_i^T X_i = B_i (the adjoint).  X may alias B.  An instance for which a
+ * device-side wait gave up (level_wait_ms) gets NaN and GLU_INST_TIMEOUT until the next glu_solve. */
 int glu_solve(glu_batch_t b, int32_t nrhs, const double* B_dev, double* X_dev, int transpose,
               void* stream);
 

@@ -162,3 +162,27 @@ def test_waits_of_the_dense_solve_are_bounded():
     x = good.solve(b)
     assert not good.status().any()
     check_solve(torch, good.get_lu(0).cpu().numpy(), b[0], x[0], False)
+
+
+def test_a_solve_that_gave_up_is_no_solution():
+    """Its vectors are NaN, also after a refinement; the flag goes with the next solve, whose waits
+    (none: a CTA per group of right-hand sides) are met."""
+    import torch
+    n = 700
+    a = matrices(n, 1, 2)
+    plan = plan_for(n, level_wait_ms=1e-6)
+    col = np.repeat(np.arange(n), n)
+    plan.set_original_pattern(np.tile(np.arange(n), n), col)
+    batch = glu.Batch(plan, 1)
+    val = torch.as_tensor(a.reshape(1, -1), device="cuda")
+    batch.load_lu_values(val)
+    batch.refactor(0.0)
+    b = torch.as_tensor(np.random.default_rng(0).standard_normal((1, 800, n)), device="cuda")
+    one = b[:, :1].contiguous()
+    x = batch.solve(one)
+    assert batch.status()[0] == 8 and bool(x.isnan().all())
+    batch.refine(val, one, x)
+    assert batch.status()[0] == 8 and bool(x.isnan().all())
+    x = batch.solve(b)
+    assert batch.status()[0] == 0
+    check_solve(torch, batch.get_lu(0).cpu().numpy(), b[0], x[0], False)
