@@ -57,7 +57,7 @@ __device__ __forceinline__ void pivot_flags(int32_t* status, int b, double d, bo
 // ---------------------------------------------------------------------------------------------
 template <int NB>
 __global__ void __launch_bounds__(256) k_dense_diag(DenseView V,
-                                                    const double* __restrict__ pert,
+                                                    const double* pert,
                                                     int32_t* status, int k) {
   constexpr int R = NB / 16;
   __shared__ double srow[2][NB];
@@ -344,7 +344,7 @@ __device__ __forceinline__ void diag64(double* T, const double* C, const double*
 }
 
 // The diagonal block at pivot k of instance b (256 threads).
-__device__ __forceinline__ void diag64_body(const DenseView& V, const double* __restrict__ pert,
+__device__ __forceinline__ void diag64_body(const DenseView& V, const double* pert,
                                             int32_t* status, int k, int b) {
   extern __shared__ double sm[];
   double* T = sm;
@@ -364,7 +364,7 @@ __device__ __forceinline__ void diag64_body(const DenseView& V, const double* __
   }
 }
 
-__global__ void __launch_bounds__(256) k_dense_diag64(DenseView V, const double* __restrict__ pert,
+__global__ void __launch_bounds__(256) k_dense_diag64(DenseView V, const double* pert,
                                                       int32_t* status, int k) {
   after_previous();
   diag64_body(V, pert, status, k, blockIdx.x);
@@ -379,7 +379,7 @@ __device__ __forceinline__ DenseView front_view(const PlanDev& P, const FrontGeo
 // Diagonal block at pivot k of every front f0 + blockIdx.y of a level (grid (count, fronts)) that
 // still has a pivot there; the same body as k_dense_diag64.
 __global__ void __launch_bounds__(256) k_front_diag(PlanDev P, double* F, int64_t fstride, int f0,
-                                                  const double* __restrict__ pert,
+                                                  const double* pert,
                                                   int32_t* status, int k) {
   after_previous();
   const FrontGeom g = P.fgeom[f0 + blockIdx.y];
@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(256) k_front_trsm8(PlanDev P, double* F, int64
 // Bound by the diagonal block's latency: 14 us with it and 4.4 us without on a 448 x 448 block, where
 // the launches it stands for took 26 (diagonal block) + 2 x 24 us (in-group products of up to 7
 // panels); n = 4,960 refactorization, panels and products: 1.27 -> 0.59 ms.
-__device__ __forceinline__ void step_body(const DenseView& V, const double* __restrict__ pert,
+__device__ __forceinline__ void step_body(const DenseView& V, const double* pert,
                                           int32_t* status, int k, int wide, int idx, int b) {
   constexpr int ST = 68;
   extern __shared__ double sm[];
@@ -1057,8 +1057,8 @@ __device__ __forceinline__ void step_body(const DenseView& V, const double* __re
   const int64_t ld = V.ld;
   double* __restrict__ D = V.base + (int64_t)b * V.stride;
   const int m0 = k + 64 + ti * 64, n0 = k + 64 + tj * 64;
-  const double* __restrict__ A = D + m0 + (int64_t)k * ld;
-  const double* __restrict__ B = D + k + (int64_t)n0 * ld;
+  const double* A = D + m0 + (int64_t)k * ld;
+  const double* B = D + k + (int64_t)n0 * ld;
   double* __restrict__ C = D + m0 + (int64_t)n0 * ld;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {               // 16 pivots per copy group
@@ -1140,7 +1140,7 @@ __device__ __forceinline__ void step_body(const DenseView& V, const double* __re
 
 constexpr int kStepSmem = 2 * 64 * 68 * 8;
 
-__global__ void __launch_bounds__(256) k_dense_step(DenseView V, const double* __restrict__ pert,
+__global__ void __launch_bounds__(256) k_dense_step(DenseView V, const double* pert,
                                                     int32_t* status, int k, int wide) {
   after_previous();
   step_body(V, pert, status, k, wide, blockIdx.x, blockIdx.y);
@@ -1149,7 +1149,7 @@ __global__ void __launch_bounds__(256) k_dense_step(DenseView V, const double* _
 // The same at pivot k of the fronts of a level, the whole trailing block of each: grid (most
 // tiles of a front, fronts * count).
 __global__ void __launch_bounds__(256) k_front_step(PlanDev P, double* F, int64_t fstride, int f0,
-                                                    int count, const double* __restrict__ pert,
+                                                    int count, const double* pert,
                                                     int32_t* status, int k) {
   after_previous();
   const FrontGeom g = P.fgeom[f0 + blockIdx.y / count];

@@ -59,7 +59,7 @@ __global__ void k_zero_slots(PlanDev P, double* vals, int first) {
     V[P.asm_zero[e]] = 0.0;
 }
 
-__global__ void k_ingest(PlanDev P, double* vals, int first, const double* __restrict__ a) {
+__global__ void k_ingest(PlanDev P, double* vals, int first, const double* a) {
   after_previous();
   const int b = blockIdx.y;
   double* V = vals + (int64_t)(first + b) * P.blob;
@@ -71,7 +71,7 @@ __global__ void k_ingest(PlanDev P, double* vals, int first, const double* __res
   }
 }
 
-__global__ void k_load_lu(PlanDev P, double* vals, int first, const double* __restrict__ val) {
+__global__ void k_load_lu(PlanDev P, double* vals, int first, const double* val) {
   after_previous();
   const int b = blockIdx.y;
   double* V = vals + (int64_t)(first + b) * P.blob;
@@ -298,7 +298,7 @@ __device__ __forceinline__ void sparse_split_part(const PlanDev& P, double* __re
 // in dynamic shared memory (the launch sizes it for the level's longest L part) and every warp's
 // updates read it from there.
 __global__ void __launch_bounds__(256) k_sparse_level(PlanDev P, double* vals,
-                                                      const double* __restrict__ pert,
+                                                      const double* pert,
                                                       int32_t* status, int begin, int ncols,
                                                       int wpc, int cpw, int stage, int lanes) {
   after_previous();
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(256) k_sparse_level(PlanDev P, double* vals,
 // Pivot and scaling of a level's columns (a CTA per column): after k_sparse_split, and in the
 // deterministic mode before k_sparse_pull.
 __global__ void __launch_bounds__(256) k_sparse_scale(PlanDev P, double* vals,
-                                                      const double* __restrict__ pert,
+                                                      const double* pert,
                                                       int32_t* status, int begin) {
   after_previous();
   const int b = blockIdx.y;
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(256) k_sparse_scale(PlanDev P, double* vals,
 // A narrow level's columns with their updates split over `splits` CTAs each (grid
 // (ncols * splits, count)); k_sparse_scale scales the columns afterwards.
 __global__ void __launch_bounds__(256) k_sparse_split(PlanDev P, double* vals,
-                                                      const double* __restrict__ pert, int begin,
+                                                      const double* pert, int begin,
                                                       int splits) {
   after_previous();
   extern __shared__ double Ls[];
@@ -424,7 +424,7 @@ __device__ bool group_barrier(unsigned* ctr, int* err, unsigned target,
 // instances GLU_INST_TIMEOUT, *err becomes non-zero, and every CTA returns.  `extra` arrivals are
 // added to every barrier target (0 in use; a test sets 1 to make the first barrier unreachable).
 __global__ void __launch_bounds__(256) k_sparse_persistent(PlanDev P, double* vals,
-                                                           const double* __restrict__ pert,
+                                                           const double* pert,
                                                            int32_t* status,
                                                            const int4* __restrict__ desc,
                                                            int nlev, int count, unsigned* bar,
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(256) k_sparse_persistent(PlanDev P, double* va
 
 // Also marks the vector's values of the dataflow solves unsolved and clears their failure word and,
 // if `fresh`, the instances' kSolveGaveUp.
-__global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm, double* y,
+__global__ void k_permute_in(PlanDev P, int nrhs, const double* Bm, double* y,
                              int64_t ylen, int transpose, double* xbuf, int* err, int32_t* status,
                              int fresh) {
   after_previous();
@@ -534,7 +534,7 @@ __global__ void k_permute_in(PlanDev P, int nrhs, const double* __restrict__ Bm,
   }
 }
 
-__global__ void k_permute_out(PlanDev P, int nrhs, const double* __restrict__ y, double* X,
+__global__ void k_permute_out(PlanDev P, int nrhs, const double* y, double* X,
                               int64_t ylen, int transpose, const int32_t* status) {
   after_previous();
   const int64_t v = blockIdx.y;
@@ -1084,9 +1084,9 @@ __global__ void k_grad(PlanDev P, int nrhs, const double* __restrict__ lambda,
 // r = b - A x (or b - A^T x) for every (instance, rhs) vector on the ORIGINAL matrix, and the
 // infinity norms ||r||, ||x||, ||b||, ||A|| of each vector (as non-negative double bits) for
 // ||r|| / (||A|| ||x|| + ||b||), the acceptance test of the solves.  Grid (chunks, vectors).
-__global__ void k_residual(PlanDev P, int nrhs, const double* __restrict__ a,
-                           const double* __restrict__ X, const double* __restrict__ Bm,
-                           double* __restrict__ R, unsigned long long* norms, int transpose) {
+__global__ void k_residual(PlanDev P, int nrhs, const double* a,
+                           const double* X, const double* Bm,
+                           double* R, unsigned long long* norms, int transpose) {
   after_previous();
   residual_rows(P, nrhs, a, X, Bm, R, norms, transpose, blockIdx.y, blockIdx.x, gridDim.x);
 }
@@ -1096,7 +1096,7 @@ __global__ void k_resid_finish(int64_t nv, const unsigned long long* norms, doub
   if (v < nv) out[v] = residual_ratio(norms + 4 * v);
 }
 
-__global__ void k_axpy(int64_t n, const double* __restrict__ dx, double* __restrict__ x) {
+__global__ void k_axpy(int64_t n, const double* dx, double* x) {
   after_previous();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)

@@ -18,10 +18,10 @@ namespace glu {
 // atomicMax on their bit patterns (non-negative doubles order like their bits).  A NaN residual
 // counts as infinite.  The whole warp must call this (it reduces with shuffles).
 __device__ __forceinline__ void residual_rows(const PlanDev& P, int nrhs,
-                                              const double* __restrict__ a,
-                                              const double* __restrict__ X,
-                                              const double* __restrict__ Bm,
-                                              double* __restrict__ R, unsigned long long* norms,
+                                              const double* a,
+                                              const double* X,
+                                              const double* Bm,
+                                              double* R, unsigned long long* norms,
                                               int transpose, int64_t v, int64_t chunk,
                                               int64_t nchunks) {
   const int64_t inst = v / nrhs;

@@ -26,6 +26,10 @@ constexpr long long kNaN = 0x7ff8000000000000ll;
 // which nothing writes): waits until the kernel before it in the stream has finished and its writes
 // are visible, then lets the kernel after it be placed on SMs that become free.  Every CTA passes
 // here before it returns, so kernels finish in stream order.
+// Such a kernel is resident while the one before it writes, so const __restrict__, which lets the
+// compiler load through the read-only path and at any place in the kernel, is for the plan's
+// arrays only: not for what the kernel before it in the stream, or the caller's, may have written
+// (right-hand sides, solutions, matrix values as loaded, perturbations).
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
