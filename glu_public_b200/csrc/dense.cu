@@ -1148,7 +1148,9 @@ __global__ void __launch_bounds__(256) k_dense_step(DenseView V, const double* p
 
 // The same at pivot k of the fronts of a level, the whole trailing block of each: grid (most
 // tiles of a front, fronts * count).
-__global__ void __launch_bounds__(256) k_front_step(PlanDev P, double* F, int64_t fstride, int f0,
+// Two CTAs on an SM: left to itself the compiler takes 80 registers and spills around the call of
+// diag64_divide (512 x 512 x 2 nodes: 27.9 ms a pass against 27.7).
+__global__ void __launch_bounds__(256, 2) k_front_step(PlanDev P, double* F, int64_t fstride, int f0,
                                                     int count, const double* pert,
                                                     int32_t* status, int k) {
   after_previous();
