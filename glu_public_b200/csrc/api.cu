@@ -63,6 +63,28 @@ int cuda_status(const char* what) {
 }
 
 }  // namespace
+
+static bool free_spares(int device);
+
+// cudaMalloc on the current device; where it finds no memory, what destroyed batches still hold on
+// the device is given back first.
+static bool device_alloc(void** p, size_t bytes, int device) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaSuccess) return true;
+  cudaGetLastError();                         // reported here, not by the caller's launch check
+  if (e == cudaErrorMemoryAllocation && free_spares(device)) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+  }
+  *p = nullptr;
+  return false;
+}
+
+template <class T>
+static bool device_alloc(T** p, size_t bytes, int device) {
+  return device_alloc(reinterpret_cast<void**>(p), bytes, device);
+}
+
 }  // namespace glu
 
 struct glu_plan_s {
@@ -85,11 +107,9 @@ struct glu_plan_s {
     *out = nullptr;
     if (v.empty()) return GLU_OK;
     void* p = nullptr;
-    if (cudaMalloc(&p, sizeof(T) * v.size()) != cudaSuccess) {
-      cudaGetLastError();
+    if (!glu::device_alloc(&p, sizeof(T) * v.size(), device))
       return glu::set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes failed",
                             sizeof(T) * v.size());
-    }
     allocs.push_back(p);
     dev_bytes += sizeof(T) * v.size();
     if (cudaMemcpy(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -172,12 +192,11 @@ int ensure_workspace(glu_batch_t b, int64_t vectors, cudaStream_t s) {
   b->y = nullptr;
   b->xbuf = nullptr;
   b->y_vectors = 0;
-  if (cudaMalloc(&b->y, sizeof(double) * b->ylen * vectors) != cudaSuccess ||
-      cudaMalloc(&b->xbuf, sizeof(double) * (glu::solve_buffer(b->plan->P) * vectors + 1)) !=
-          cudaSuccess) {
-    cudaGetLastError();
+  const int dev = b->plan->device;
+  if (!glu::device_alloc(&b->y, sizeof(double) * b->ylen * vectors, dev) ||
+      !glu::device_alloc(&b->xbuf,
+                         sizeof(double) * (glu::solve_buffer(b->plan->P) * vectors + 1), dev))
     return set_error(GLU_MEMORY_OVERFLOW, "solve workspace allocation failed");
-  }
   b->y_vectors = vectors;
   return GLU_OK;
 }
@@ -308,11 +327,10 @@ int ensure_refine_workspace(glu_batch_t b, int64_t vectors, cudaStream_t s) {
   b->rbuf = nullptr;
   b->norms = nullptr;
   b->r_vectors = 0;
-  if (cudaMalloc(&b->rbuf, sizeof(double) * b->plan->hp.n * vectors) != cudaSuccess ||
-      cudaMalloc(&b->norms, sizeof(unsigned long long) * 4 * vectors) != cudaSuccess) {
-    cudaGetLastError();
+  const int dev = b->plan->device;
+  if (!glu::device_alloc(&b->rbuf, sizeof(double) * b->plan->hp.n * vectors, dev) ||
+      !glu::device_alloc(&b->norms, sizeof(unsigned long long) * 4 * vectors, dev))
     return set_error(GLU_MEMORY_OVERFLOW, "refinement workspace allocation failed");
-  }
   b->r_vectors = vectors;
   return GLU_OK;
 }
@@ -486,7 +504,8 @@ static void batch_free(glu_batch_s* b) {
 // and cudaFree than on the device: 16 x n = 4,960 forward and backward, 3.0 ms of kernels, took 8
 // to 20 ms a call, 3.2 ms with them spared.  So the buffers of a plan's last destroyed batch are
 // kept for its next batch of the same count: at most kSpareBytes in all, the oldest given up first,
-// released with the plan, and all of a device's when an allocation of this library fails there.
+// released with the plan, and all of a device's when an allocation of this library finds no memory
+// there (device_alloc).
 static constexpr size_t kSpareBytes = (size_t)1 << 30;
 static std::mutex g_spares_mu;
 static std::vector<glu_batch_s*> g_spares;          // oldest first, at most one per plan
@@ -512,8 +531,8 @@ static glu_batch_s* take_spare(glu_plan_s* p, int count) {
   return nullptr;
 }
 
-// Frees every spare batch on the device; true if there was one.
-static bool free_spares(int device) {
+// Frees every spare batch on the device (the current one); true if there was one.
+static bool glu::free_spares(int device) {
   bool any = false;
   std::lock_guard<std::mutex> lock(g_spares_mu);
   for (size_t i = g_spares.size(); i-- > 0;)
@@ -1058,11 +1077,10 @@ static int build_persistent(glu_batch_s* b) {
   }
   if (b->pruns.empty()) return GLU_OK;
   b->pgroups = max_groups;
-  if (cudaMalloc(&b->pdesc, sizeof(int4) * desc.size()) != cudaSuccess ||
-      cudaMalloc(&b->pbar, sizeof(unsigned) * (max_groups + 1)) != cudaSuccess) {
-    cudaGetLastError();
+  const int dev = b->plan->device;
+  if (!glu::device_alloc(&b->pdesc, sizeof(int4) * desc.size(), dev) ||
+      !glu::device_alloc(&b->pbar, sizeof(unsigned) * (max_groups + 1), dev))
     return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of the level-run descriptors failed");
-  }
   if (cudaMemcpy(b->pdesc, desc.data(), sizeof(int4) * desc.size(), cudaMemcpyHostToDevice) !=
       cudaSuccess)
     return glu::cuda_status("level-run descriptors");
@@ -1079,8 +1097,7 @@ static int batch_alloc(glu_plan_t p, int32_t count, double* storage, glu_batch_t
   if (storage) {
     b->vals = storage;
   } else {
-    if (cudaMalloc(&b->vals, bytes) != cudaSuccess) {
-      cudaGetLastError();
+    if (!glu::device_alloc(&b->vals, bytes, p->device)) {
       delete b;
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes for %d instances failed",
                        bytes, count);
@@ -1089,25 +1106,22 @@ static int batch_alloc(glu_plan_t p, int32_t count, double* storage, glu_batch_t
   }
   if (p->hp.front_area > 0) {
     const size_t fbytes = sizeof(double) * (size_t)p->hp.front_area * count;
-    if (cudaMalloc(&b->fbuf, fbytes) != cudaSuccess) {
-      cudaGetLastError();
+    if (!glu::device_alloc(&b->fbuf, fbytes, p->device)) {
       batch_free(b);
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes (front buffers) failed", fbytes);
     }
   }
   if (p->P.hubs_p > 0) {
     const size_t gbytes = sizeof(double) * 2 * (size_t)p->P.ntp * p->P.hubs_p * count;
-    if (cudaMalloc(&b->gbuf, gbytes) != cudaSuccess) {
-      cudaGetLastError();
+    if (!glu::device_alloc(&b->gbuf, gbytes, p->device)) {
       batch_free(b);
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes (hub panels) failed", gbytes);
     }
     cudaMemset(b->gbuf, 0, gbytes);
   }
-  if (cudaMalloc(&b->pert, sizeof(double) * count) != cudaSuccess ||
-      cudaMalloc(&b->status, sizeof(int32_t) * count) != cudaSuccess ||
-      cudaMalloc(&b->asm_flag, count) != cudaSuccess) {
-    cudaGetLastError();
+  if (!glu::device_alloc(&b->pert, sizeof(double) * count, p->device) ||
+      !glu::device_alloc(&b->status, sizeof(int32_t) * count, p->device) ||
+      !glu::device_alloc(&b->asm_flag, count, p->device)) {
     batch_free(b);
     return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc failed");
   }
@@ -1154,10 +1168,7 @@ static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_
       batch_free(b);
     }
   }
-  int st = batch_alloc(p, count, storage, out);
-  // memory that destroyed batches still hold goes before the call fails
-  if (st == GLU_MEMORY_OVERFLOW && free_spares(p->device)) st = batch_alloc(p, count, storage, out);
-  return st;
+  return batch_alloc(p, count, storage, out);
 }
 
 int glu_batch_create(glu_plan_t p, int32_t count, glu_batch_t* out) {

@@ -8,7 +8,7 @@ import pytest
 
 from glu_public_b200 import glu
 from tests.test_gpu_dense_solve import check_solve, plan_for
-from tests.test_gpu_dense_steps import check_lu, matrices
+from tests.test_gpu_dense_steps import check_lu, dense_symbolic, matrices
 
 pytestmark = pytest.mark.gpu
 
@@ -60,3 +60,45 @@ def test_memory_is_given_back_with_the_plan():
     del plan
     gc.collect()
     assert torch.cuda.mem_get_info()[0] >= free0
+
+
+@pytest.mark.parametrize("call", ["solve", "refine", "plan", "batch"])
+def test_memory_is_given_back_when_an_allocation_needs_it(call):
+    """With little but a destroyed batch's memory left on the device, every allocation of the library
+    finds it: solve and refinement workspaces, plans, batches."""
+    import torch
+    n = 2000
+    plan, other = plan_for(n), plan_for(n)
+    col = np.repeat(np.arange(n), n)
+    other.set_original_pattern(np.tile(np.arange(n), n), col)
+    val = torch.as_tensor(matrices(n, 1, 0).reshape(1, -1), device="cuda")
+    batch = glu.Batch(other, 1)
+    batch.load_lu_values(val)
+    batch.refactor(0.0)
+    b = torch.ones((1, 6000, n), dtype=torch.float64, device="cuda")
+    few = b[:, :9].contiguous()               # the kernels are on the device before it is full
+    batch.refine(val, few, batch.solve(few))
+    torch.cuda.synchronize()
+    spare = glu.Batch(plan, 16)               # 512 MB
+    if call == "refine":
+        x = batch.solve(b)
+    before = torch.cuda.mem_get_info()[0]
+    del spare
+    assert torch.cuda.mem_get_info()[0] < before + (256 << 20)    # kept
+    x = torch.empty_like(b)
+    leave = {"solve": 160, "refine": 64, "plan": 64, "batch": 64}[call] << 20
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda")
+    assert torch.cuda.mem_get_info()[0] <= leave
+    try:
+        if call == "solve":
+            batch.solve(b, out=x)             # 290 MB
+        elif call == "refine":
+            batch.refine(val, b, x)           # 96 MB
+        elif call == "plan":
+            glu.Plan(dense_symbolic(2800), dense_min=1)   # over 90 MB
+        else:
+            glu.Batch(other, 4)               # 128 MB
+        torch.cuda.synchronize()
+    finally:
+        del rest
+        torch.cuda.empty_cache()
