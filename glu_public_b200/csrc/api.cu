@@ -169,6 +169,16 @@ struct glu_batch_s {
   int pgroups = 0;
   int pextra = 0;               // test hook: arrivals added to every barrier target
   double pwait_ms = 1000.0;     // bound of every wait of the cooperative launches
+  // the end of the last work on each stream the batch was used on, for the next owner of its buffers
+  // to wait for; `untracked`: its work is in a graph, which may be launched anywhere, or on more
+  // streams than this
+  struct Use {
+    unsigned long long stream;  // cudaStreamGetId: a later stream of the same handle is another
+    cudaEvent_t done;
+  };
+  std::vector<Use> uses;
+  size_t nuses = 0;             // of the events made, those in use
+  bool untracked = false;
 };
 
 namespace {
@@ -473,6 +483,47 @@ int batch_residual_view(glu_batch_t b, const PlanDev** P, int* count, int* devic
 }
 }  // namespace glu
 
+// Notes that the call has put work of the batch on stream s.
+static void note_use(glu_batch_s* b, cudaStream_t s) {
+  constexpr size_t kMaxUses = 4;
+  if (b->untracked || !b->own_vals) return;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  bool ok = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
+            cudaStreamGetId(s, &id) == cudaSuccess;
+  size_t i = 0;
+  while (ok && i < b->nuses && b->uses[i].stream != id) ++i;
+  if (ok && i == b->uses.size()) {
+    cudaEvent_t e = nullptr;
+    ok = i < kMaxUses && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    if (ok) b->uses.push_back({id, e});
+  }
+  if (ok) {
+    b->uses[i].stream = id;
+    b->nuses = std::max(b->nuses, i + 1);
+    ok = cudaEventRecord(b->uses[i].done, s) == cudaSuccess;
+  }
+  if (!ok) {
+    cudaGetLastError();
+    b->untracked = true;
+  }
+}
+
+// Clears what a new batch has cleared, once the work noted on its buffers is done; waits for that
+// and for nothing else (other streams may be capturing, or busy), on a stream of the batch's own.
+static bool batch_clear(glu_batch_s* b, size_t gbytes) {
+  if (!b->own_stream &&
+      cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking) != cudaSuccess)
+    return false;
+  for (size_t i = 0; i < b->nuses; ++i)
+    if (cudaStreamWaitEvent(b->own_stream, b->uses[i].done, 0) != cudaSuccess) return false;
+  b->nuses = 0;
+  return (gbytes == 0 || cudaMemsetAsync(b->gbuf, 0, gbytes, b->own_stream) == cudaSuccess) &&
+         cudaMemsetAsync(b->status, 0, sizeof(int32_t) * b->count, b->own_stream) == cudaSuccess &&
+         cudaMemsetAsync(b->asm_flag, 0, b->count, b->own_stream) == cudaSuccess &&
+         cudaStreamSynchronize(b->own_stream) == cudaSuccess;
+}
+
 // Releases the batch's captured graph.
 static void drop_graph(glu_batch_s* b) {
   if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -486,6 +537,7 @@ static void batch_free(glu_batch_s* b) {
   if (!b) return;
   drop_graph(b);
   if (b->own_stream) cudaStreamDestroy(b->own_stream);
+  for (const glu_batch_s::Use& u : b->uses) cudaEventDestroy(u.done);
   for (int i = 0; i < glu_batch_s::kFrontStreams; ++i) {
     if (b->fstream[i]) cudaStreamDestroy(b->fstream[i]);
     if (b->fjoin[i]) cudaEventDestroy(b->fjoin[i]);
@@ -547,8 +599,7 @@ static bool glu::free_spares(int device) {
 // Keeps a destroyed batch's buffers; false if they are not kept.
 static bool keep_spare(glu_batch_s* b) {
   const size_t bytes = batch_bytes(b);
-  if (!b->own_vals || bytes > kSpareBytes) return false;
-  drop_graph(b);
+  if (!b->own_vals || b->untracked || bytes > kSpareBytes) return false;
   b->loaded = b->factored = false;
   b->launches = 0;
   std::lock_guard<std::mutex> lock(g_spares_mu);
@@ -1111,13 +1162,13 @@ static int batch_alloc(glu_plan_t p, int32_t count, double* storage, glu_batch_t
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes (front buffers) failed", fbytes);
     }
   }
+  size_t gbytes = 0;
   if (p->P.hubs_p > 0) {
-    const size_t gbytes = sizeof(double) * 2 * (size_t)p->P.ntp * p->P.hubs_p * count;
+    gbytes = sizeof(double) * 2 * (size_t)p->P.ntp * p->P.hubs_p * count;
     if (!glu::device_alloc(&b->gbuf, gbytes, p->device)) {
       batch_free(b);
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes (hub panels) failed", gbytes);
     }
-    cudaMemset(b->gbuf, 0, gbytes);
   }
   if (!glu::device_alloc(&b->pert, sizeof(double) * count, p->device) ||
       !glu::device_alloc(&b->status, sizeof(int32_t) * count, p->device) ||
@@ -1125,8 +1176,11 @@ static int batch_alloc(glu_plan_t p, int32_t count, double* storage, glu_batch_t
     batch_free(b);
     return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc failed");
   }
-  cudaMemset(b->status, 0, sizeof(int32_t) * count);
-  cudaMemset(b->asm_flag, 0, count);
+  if (!batch_clear(b, gbytes)) {
+    const int st = glu::cuda_status("batch create");
+    batch_free(b);
+    return st ? st : set_error(GLU_CUDA_ERROR, "batch create");
+  }
   if (int st = build_persistent(b)) {
     batch_free(b);
     return st;
@@ -1155,12 +1209,8 @@ static int batch_create(glu_plan_t p, int32_t count, double* storage, glu_batch_
   if (storage && reinterpret_cast<uintptr_t>(storage) % 256)
     return set_error(GLU_ARGUMENT_ERROR, "storage must be 256-byte aligned");
   if (!storage) {
-    // the spare batch's buffers may still be in use on some stream: wait for the device once, as
-    // the cudaFree they were spared from would have done
     if (glu_batch_s* b = take_spare(p, count)) {
-      if (cudaDeviceSynchronize() == cudaSuccess &&
-          cudaMemset(b->status, 0, sizeof(int32_t) * count) == cudaSuccess &&
-          cudaMemset(b->asm_flag, 0, count) == cudaSuccess) {
+      if (batch_clear(b, 0)) {
         *out = b;
         return GLU_OK;
       }
@@ -1200,6 +1250,7 @@ int glu_load_values(glu_batch_t b, int32_t first, int32_t count, const double* a
   glu::launch_prepare_blob(b->plan->P, b->vals, first, count, asm_ok, s, lc);
   glu::launch_ingest(b->plan->P, b->vals, first, count, a_dev, s, lc);
   cudaMemsetAsync(b->asm_flag + first, asm_ok ? 1 : 0, count, s);
+  note_use(b, s);
   b->loaded = true;
   b->factored = false;
   return glu::cuda_status("load values");
@@ -1216,6 +1267,7 @@ int glu_load_lu_values(glu_batch_t b, int32_t first, int32_t count, const double
   glu::launch_prepare_blob(b->plan->P, b->vals, first, count, false, s, lc);
   glu::launch_load_lu(b->plan->P, b->vals, first, count, val_dev, s, lc);
   cudaMemsetAsync(b->asm_flag + first, 0, count, s);
+  note_use(b, s);
   b->loaded = true;
   b->factored = false;
   return glu::cuda_status("load LU values");
@@ -1225,7 +1277,9 @@ int glu_refactor(glu_batch_t b, double pert, void* stream) {
   if (!b) return set_error(GLU_ARGUMENT_ERROR, "null batch");
   if (!b->loaded) return set_error(GLU_NOT_READY, "no values loaded");
   glu::DeviceGuard g(b->plan->device);
-  return do_refactor(b, pert, (cudaStream_t)stream);
+  const int st = do_refactor(b, pert, (cudaStream_t)stream);
+  note_use(b, (cudaStream_t)stream);
+  return st;
 }
 
 int glu_refactor_timed(glu_batch_t b, double pert, void* stream, double* phase_ms,
@@ -1241,6 +1295,7 @@ int glu_refactor_timed(glu_batch_t b, double pert, void* stream, double* phase_m
   PhaseTimer tm;
   tm.s = s;
   int st = do_refactor(b, pert, s, &tm, phase_launches);
+  note_use(b, s);
   if (st) return st;
   if (cudaStreamSynchronize(s) != cudaSuccess) return glu::cuda_status("refactor");
   for (size_t i = 1; i < tm.ev.size(); ++i) {
@@ -1260,6 +1315,7 @@ int glu_debug_refactor_unreachable_barrier(glu_batch_t b, double wait_ms, void* 
   b->pextra = 1;
   b->pwait_ms = wait_ms;
   int st = do_refactor(b, 0.0, s);
+  note_use(b, s);
   b->pextra = 0;
   b->pwait_ms = saved;
   if (st) return st;
@@ -1378,7 +1434,9 @@ int glu_solve(glu_batch_t b, int32_t nrhs, const double* B_dev, double* X_dev, i
   if (!b->plan->has_solve) return set_error(GLU_NOT_READY, "no solve maps (glu_plan_set_solve_maps)");
   if (!b->factored) return set_error(GLU_NOT_READY, "solve before refactor");
   glu::DeviceGuard g(b->plan->device);
-  return do_solve(b, nrhs, B_dev, X_dev, transpose, true, (cudaStream_t)stream);
+  const int st = do_solve(b, nrhs, B_dev, X_dev, transpose, true, (cudaStream_t)stream);
+  note_use(b, (cudaStream_t)stream);
+  return st;
 }
 
 int glu_residual(glu_batch_t b, int32_t nrhs, const double* a_dev, const double* B_dev,
@@ -1395,6 +1453,7 @@ int glu_residual(glu_batch_t b, int32_t nrhs, const double* a_dev, const double*
   glu::LaunchCounter lc;
   glu::launch_residual(b->plan->P, b->count, nrhs, a_dev, X_dev, B_dev, nullptr, b->norms,
                        resid_dev, transpose, s, lc);
+  note_use(b, s);
   return glu::cuda_status("residual");
 }
 
@@ -1411,6 +1470,7 @@ int glu_refine(glu_batch_t b, int32_t nrhs, const double* a_dev, const double* B
   int64_t nl = 0;
   int st = do_refine(b, nrhs, a_dev, B_dev, X_dev, steps, transpose, resid_dev,
                      (cudaStream_t)stream, &nl);
+  note_use(b, (cudaStream_t)stream);
   b->launches = nl;
   return st;
 }
@@ -1433,6 +1493,7 @@ int glu_get_lu(glu_batch_t b, int32_t instance, double* val_dev, void* stream) {
   glu::DeviceGuard g(b->plan->device);
   glu::LaunchCounter lc;
   glu::launch_export_lu(b->plan->P, b->vals, instance, val_dev, (cudaStream_t)stream, lc);
+  note_use(b, (cudaStream_t)stream);
   return glu::cuda_status("export LU");
 }
 
@@ -1443,6 +1504,7 @@ int glu_graph_capture(glu_batch_t b, const double* a_dev, int32_t nrhs, const do
   if (nrhs > 0 && (!B_dev || !X_dev || !b->plan->has_solve))
     return set_error(GLU_NOT_READY, "solve inputs / maps missing");
   glu::DeviceGuard g(b->plan->device);
+  b->untracked = true;
   cudaStream_t s = (cudaStream_t)stream;
   if (!s) {
     if (!b->own_stream && cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking))
@@ -1604,6 +1666,7 @@ int glu_group_capture(int32_t nbatch, const glu_batch_t* batches, const double* 
   int64_t total = 0;
   for (int i = 0; i < nbatch && st == GLU_OK; ++i) {
     glu_batch_t b = batches[i];
+    b->untracked = true;
     cudaStream_t bs = g->streams[i];
     cudaStreamWaitEvent(bs, fork, 0);            // the branch joins the capture here
     glu::LaunchCounter lc;

@@ -207,10 +207,11 @@ int glu_batch_create(glu_plan_t p, int32_t count, glu_batch_t* out);
  * 256-byte aligned device memory) -- used to stay inside a memory budget. */
 int glu_batch_slots_per_instance(glu_plan_t p, uint64_t* slots);
 int glu_batch_create_external(glu_plan_t p, int32_t count, double* storage_dev, glu_batch_t* out);
-/* The device buffers of a destroyed batch (glu_batch_create, at most 1 GiB over all plans) may be kept
- * with the library for the plan's next batch of the same count; they are released when the plan is
- * destroyed or when an allocation of this library would fail.  A batch must not be destroyed while
- * one of its graphs or groups will still be launched. */
+/* The device buffers of a destroyed batch (glu_batch_create, at most 1 GiB over all plans; not of one
+ * whose work was captured in a graph) may be kept with the library for the plan's next batch of the
+ * same count, whose creation waits for the work the destroyed one had put on its streams; they are
+ * released when the plan is destroyed or when an allocation of this library would fail.  A batch
+ * must not be destroyed while one of its graphs or groups will still be launched. */
 int glu_batch_destroy(glu_batch_t b);
 
 /* Loads values for instances [first, first+count): a_dev holds count rows of nnz_a doubles in

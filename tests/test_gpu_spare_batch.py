@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import gc
+import threading
 
 import numpy as np
 import pytest
@@ -102,3 +103,69 @@ def test_memory_is_given_back_when_an_allocation_needs_it(call):
     finally:
         del rest
         torch.cuda.empty_cache()
+
+
+def test_a_batch_made_while_another_thread_captures():
+    """Taking over a destroyed batch's buffers waits for their last use only: a capture in another
+    thread goes on, and its graph runs."""
+    import torch
+    n = 200
+    plan = plan_for(n)
+    a = matrices(n, 2, 4)
+    val = torch.as_tensor(a.reshape(2, -1), device="cuda")
+    b = torch.ones((2, 1, n), dtype=torch.float64, device="cuda")
+    x, s = torch.empty_like(b), torch.cuda.Stream()
+    ones = torch.ones(8, device="cuda")
+
+    def use():
+        batch = glu.Batch(plan, 2)
+        batch.load_lu_values(val, stream=s)
+        batch.refactor(0.0, stream=s)
+        batch.solve(b, out=x, stream=s)
+        s.synchronize()
+        return batch
+
+    use()                                     # destroyed: its buffers are there for the next
+    x.zero_()
+    made = []
+    thread = threading.Thread(target=lambda: made.append(use()))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream(), capture_error_mode="thread_local"):
+        twice = ones * 2.0
+        thread.start()
+        thread.join()
+        twice = twice + 1.0
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((twice == 3.0).all())
+    check_solve(torch, made[0].get_lu(1).cpu().numpy(), b[1], x[1], False)
+
+
+def test_a_captured_batch_is_not_taken_over():
+    """A graph of a batch's work may still run after the batch: the plan's next batch has buffers of
+    its own."""
+    import torch
+    n = 200
+    plan = plan_for(n)
+    a = matrices(n, 2, 5)
+    val = torch.as_tensor(a.reshape(2, -1), device="cuda")
+    b = torch.ones((2, 1, n), dtype=torch.float64, device="cuda")
+    x, y = torch.empty_like(b), torch.empty_like(b)
+    batch = glu.Batch(plan, 2)
+    batch.load_lu_values(val)
+    batch.refactor(0.0)
+    batch.solve(b, out=x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        batch.solve(b, out=x)
+    for _ in range(20):
+        graph.replay()
+    del batch                                 # with the graph's solves under way
+    batch = glu.Batch(plan, 2)
+    batch.load_lu_values(2.0 * val)
+    batch.refactor(0.0)
+    batch.solve(b, out=y)
+    torch.cuda.synchronize()
+    torch.testing.assert_close(y, 0.5 * x, rtol=1e-12, atol=0.0)
+    check_solve(torch, batch.get_lu(1).cpu().numpy(), b[1], y[1], False)
