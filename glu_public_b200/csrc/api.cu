@@ -146,8 +146,8 @@ struct glu_batch_s {
   int64_t r_vectors = 0;
   int64_t ylen = 0;
   int64_t y_vectors = 0;
-  double* xbuf = nullptr;       // solved values of the dense block and the fronts (trsv.cu),
-                                // then the solve's failure word
+  double* xbuf = nullptr;       // solved values of the dataflow solves (trsv.cu), x_len of them,
+  int64_t x_len = 0;            // then the solve's failure word
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaStream_t own_stream = nullptr;
@@ -190,6 +190,25 @@ int check_plan(glu_plan_t p) {
   return GLU_OK;
 }
 
+// The plan as a solve of nrhs vectors an instance sees it: without fronts, the sparse columns have
+// solved values only where they are solved as a dataflow.
+glu::PlanDev solve_plan(glu_batch_t b, int nrhs) {
+  glu::PlanDev P = b->plan->P;
+  if (b->plan->hp.fronts.empty() && !glu::sparse_solve_flows(P, b->count, nrhs)) P.fx_len = 0;
+  return P;
+}
+
+// Solved values that any solve of at most `vectors` vectors in all needs.
+int64_t solve_values(glu_batch_t b, int64_t vectors) {
+  glu::PlanDev P = b->plan->P;
+  const int64_t all = glu::solve_buffer(P) * vectors;
+  if (!b->plan->hp.fronts.empty()) return all;
+  const int64_t flow = std::min(vectors, glu::sparse_flow_vectors(P, b->count));
+  const int64_t most = glu::solve_buffer(P) * flow;
+  P.fx_len = 0;
+  return std::max(most, glu::solve_buffer(P) * vectors);
+}
+
 int ensure_workspace(glu_batch_t b, int64_t vectors, cudaStream_t s) {
   if (b->y_vectors >= vectors) return GLU_OK;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -201,12 +220,13 @@ int ensure_workspace(glu_batch_t b, int64_t vectors, cudaStream_t s) {
   if (b->xbuf) cudaFree(b->xbuf);
   b->y = nullptr;
   b->xbuf = nullptr;
-  b->y_vectors = 0;
+  b->y_vectors = b->x_len = 0;
   const int dev = b->plan->device;
+  const int64_t x_len = solve_values(b, vectors);
   if (!glu::device_alloc(&b->y, sizeof(double) * b->ylen * vectors, dev) ||
-      !glu::device_alloc(&b->xbuf,
-                         sizeof(double) * (glu::solve_buffer(b->plan->P) * vectors + 1), dev))
+      !glu::device_alloc(&b->xbuf, sizeof(double) * (x_len + 1), dev))
     return set_error(GLU_MEMORY_OVERFLOW, "solve workspace allocation failed");
+  b->x_len = x_len;
   b->y_vectors = vectors;
   return GLU_OK;
 }
@@ -372,7 +392,7 @@ int do_refine(glu_batch_t b, int nrhs, const double* a, const double* B, double*
 int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose, bool fresh,
              cudaStream_t s) {
   glu_plan_s* pl = b->plan;
-  const glu::PlanDev& P = pl->P;
+  const glu::PlanDev P = solve_plan(b, nrhs);
   const glu::HostPlan& hp = pl->hp;
   int st = ensure_workspace(b, (int64_t)b->count * nrhs, s);
   if (st) return st;
@@ -380,7 +400,7 @@ int do_solve(glu_batch_t b, int nrhs, const double* B, double* X, int transpose,
   double* y = b->y;
   const int64_t yl = b->ylen;
   const int cnt = b->count;
-  int* serr = reinterpret_cast<int*>(b->xbuf + glu::solve_buffer(P) * b->y_vectors);
+  int* serr = reinterpret_cast<int*>(b->xbuf + b->x_len);
   glu::launch_solve_permute_in(P, cnt, nrhs, B, y, yl, transpose, b->xbuf, serr, b->status, fresh, s,
                                lc);
   auto dense = [&] {
@@ -566,7 +586,7 @@ static size_t batch_bytes(const glu_batch_s* b) {
   const glu::HostPlan& hp = b->plan->hp;
   const size_t doubles = ((size_t)hp.blob + (size_t)hp.front_area +
                           2 * (size_t)hp.ntp * hp.hubs_p) * b->count +
-                         (size_t)(b->ylen + glu::solve_buffer(b->plan->P)) * b->y_vectors +
+                         (size_t)b->ylen * b->y_vectors + (size_t)b->x_len +
                          ((size_t)hp.n + 4) * b->r_vectors;
   return sizeof(double) * doubles;
 }

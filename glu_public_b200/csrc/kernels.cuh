@@ -186,8 +186,10 @@ void launch_front_flow(const PlanDev& P, const double* vals, int count, int nrhs
 void launch_solve_level(const PlanDev& P, const double* vals, int count, int nrhs, double* y,
                         int64_t ylen, const int32_t* cols, int begin, int ncols, int nlong,
                         const FrontLevelSolve& L, int which, cudaStream_t s, LaunchCounter& lc);
-// plans without fronts: whether the sparse columns are solved as a dataflow, one launch per phase
+// plans without fronts: whether the sparse columns are solved as a dataflow, one launch per phase,
+// and the most vectors of `count` instances for which they are
 bool sparse_solve_flows(const PlanDev& P, int count, int nrhs);
+int64_t sparse_flow_vectors(const PlanDev& P, int count);
 // one such phase (which 0: L, with the rows t .. n of L21; 1: U; 2: U^T; 3: L^T), `items` the sparse
 // columns in the levels' order (trsv.cu)
 void launch_sparse_flow(const PlanDev& P, const double* vals, int count, int nrhs, double* y,

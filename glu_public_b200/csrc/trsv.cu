@@ -817,8 +817,11 @@ void launch_front_flow(const PlanDev& P, const double* vals, int count, int nrhs
 // whole passes (rows, groups of right-hand sides counted): n = 2,000 385 / 405 us (1,562),
 // 64 x n = 2,000 0.993 / 1.003 ms (99,968), 8 groups at n = 20,000 0.798 / 0.884 ms (124,928),
 // 10 groups transposed 1.055 / 1.276 ms (156,160), 256 x n = 2,000 3.01 / 2.92 ms (399,872).
+int64_t sparse_flow_vectors(const PlanDev& P, int count) {
+  return P.t > 0 ? 200000 / ((int64_t)count * P.t) * 4 * count : 0;
+}
 bool sparse_solve_flows(const PlanDev& P, int count, int nrhs) {
-  return P.t > 0 && (int64_t)count * ((nrhs + 3) / 4) * P.t <= 200000;
+  return (int64_t)count * nrhs <= sparse_flow_vectors(P, count);
 }
 
 void launch_sparse_flow(const PlanDev& P, const double* vals, int count, int nrhs, double* y,

@@ -179,3 +179,40 @@ def test_assembly_of_the_dense_block(count):
         lu = np.zeros((n, n))                 # [column, row]
         lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
         check_lu(torch, lu, np.ascontiguousarray(a.T * scale[i])[None])
+
+
+def test_workspace_of_many_vectors():
+    """Vectors solved level by level hold one copy of themselves in the workspace and nothing for the
+    dataflow, which fewer of them take: these find room in the same workspace, also under capture."""
+    import torch
+    n, nrhs = 1100, 40000
+    a = long_columns(n, 7)
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, dense_threshold=2.0, front_min_w=0)
+    idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
+    plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
+    batch = glu.Batch(plan, 1)
+    batch.load_lu_values(torch.as_tensor(sym.val[None], device="cuda"))
+    batch.refactor(0.0)
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    b = torch.randn((1, nrhs, n), dtype=torch.float64, device="cuda", generator=gen)
+    x = torch.empty_like(b)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    batch.solve(b, out=x)
+    torch.cuda.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] <= 8 * n * nrhs + (64 << 20)
+    cp = sym.sym_c_ptr.astype(np.int64)
+    lu = np.zeros((n, n))
+    lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(0).cpu().numpy()
+    check_solve(torch, lu, b[0, -9:], x[0, -9:], False)
+    for k in (1, 9, 727, 729):
+        few, y = b[:, :k].contiguous(), torch.empty_like(b[:, :k])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            batch.solve(few, out=y)
+        graph.replay()
+        torch.cuda.synchronize()
+        check_solve(torch, lu, few[0], y[0], False)
