@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -89,6 +90,8 @@ static bool device_alloc(T** p, size_t bytes, int device) {
 
 struct glu_plan_s {
   int device = 0;
+  std::atomic<int> refs{1};     // the caller's handle and every batch, spare ones too
+  bool destroyed = false;       // the handle is gone (under g_spares_mu)
   glu::HostPlan hp;
   glu::PlanDev P{};
   std::vector<void*> allocs;
@@ -552,6 +555,16 @@ static void drop_graph(glu_batch_s* b) {
   b->graph = nullptr;
 }
 
+// Gives up one reference to a plan; the last one frees it.
+static void plan_release(glu_plan_s* p) {
+  if (p->refs.fetch_sub(1) > 1) return;
+  {
+    glu::DeviceGuard g(p->device);
+    for (void* a : p->allocs) cudaFree(a);
+  }
+  delete p;
+}
+
 // Releases everything a batch holds.
 static void batch_free(glu_batch_s* b) {
   if (!b) return;
@@ -568,6 +581,7 @@ static void batch_free(glu_batch_s* b) {
                   (void*)b->xbuf, (void*)b->gbuf, (void*)b->fbuf, (void*)b->rbuf,
                   (void*)b->norms, (void*)b->pdesc, (void*)b->pbar})
     if (q) cudaFree(q);
+  plan_release(b->plan);
   delete b;
 }
 
@@ -623,6 +637,7 @@ static bool keep_spare(glu_batch_s* b) {
   b->loaded = b->factored = false;
   b->launches = 0;
   std::lock_guard<std::mutex> lock(g_spares_mu);
+  if (b->plan->destroyed) return false;
   try {
     g_spares.push_back(b);
   } catch (const std::exception&) {
@@ -1047,11 +1062,12 @@ int glu_plan_stat(glu_plan_t p, int i, double* v) {
 int glu_plan_destroy(glu_plan_t p) {
   if (!p) return GLU_OK;
   {
-    glu::DeviceGuard g(p->device);
-    batch_free(take_spare(p, 0));
-    for (void* a : p->allocs) cudaFree(a);
+    std::lock_guard<std::mutex> lock(g_spares_mu);
+    p->destroyed = true;                       // batches destroyed from now on are not kept
   }
-  delete p;
+  glu::DeviceGuard g(p->device);
+  batch_free(take_spare(p, 0));
+  plan_release(p);
   return GLU_OK;
 }
 
@@ -1162,6 +1178,7 @@ static int batch_alloc(glu_plan_t p, int32_t count, double* storage, glu_batch_t
   glu_batch_s* b = new (std::nothrow) glu_batch_s();
   if (!b) return set_error(GLU_MEMORY_OVERFLOW, "host allocation failed");
   b->plan = p;
+  p->refs.fetch_add(1);
   b->count = count;
   b->ylen = (int64_t)p->hp.n + (int64_t)(p->hp.ntp - p->hp.nt);
   const size_t bytes = sizeof(double) * (size_t)p->hp.blob * count;
@@ -1169,7 +1186,7 @@ static int batch_alloc(glu_plan_t p, int32_t count, double* storage, glu_batch_t
     b->vals = storage;
   } else {
     if (!glu::device_alloc(&b->vals, bytes, p->device)) {
-      delete b;
+      batch_free(b);
       return set_error(GLU_MEMORY_OVERFLOW, "cudaMalloc of %zu bytes for %d instances failed",
                        bytes, count);
     }

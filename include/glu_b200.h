@@ -199,6 +199,7 @@ int glu_plan_set_solve_maps(glu_plan_t p, const uint32_t* col_perm, const uint32
  * entries of heavy dense columns (applied by their own CTAs when the batch is a few matrices),
  * 26 widest front (columns). */
 int glu_plan_stat(glu_plan_t p, int i, double* value);
+/* The plan's memory goes with the last of its batches. */
 int glu_plan_destroy(glu_plan_t p);
 
 /* ---- batch: `count` value instances of one plan, factored in place on the device ---- */

@@ -169,3 +169,27 @@ def test_a_captured_batch_is_not_taken_over():
     torch.cuda.synchronize()
     torch.testing.assert_close(y, 0.5 * x, rtol=1e-12, atol=0.0)
     check_solve(torch, batch.get_lu(1).cpu().numpy(), b[1], y[1], False)
+
+
+def test_a_batch_outlives_its_plan():
+    """A plan destroyed before its batch (the order of a garbage collection) stays until the batch
+    goes; nothing of it is kept for another plan."""
+    import torch
+    n, count = 300, 16
+    torch.cuda.synchronize()
+    gc.collect()
+    a = matrices(n, count, 6)
+    val = torch.as_tensor(a.reshape(count, -1), device="cuda")
+    b = torch.ones((count, 1, n), dtype=torch.float64, device="cuda")
+    for k in range(3):
+        plan = plan_for(n + 64 * k)
+        batch = glu.Batch(plan, count)
+        assert glu.lib().glu_plan_destroy(plan.h) == 0
+        plan.h = None
+        if k == 0:
+            batch.load_lu_values(val)
+            batch.refactor(0.0)
+            x = batch.solve(b)
+            check_solve(torch, batch.get_lu(3).cpu().numpy(), b[3], x[3], False)
+        assert glu.lib().glu_batch_destroy(batch.h) == 0
+        batch.h = None
