@@ -540,19 +540,16 @@ __global__ void k_permute_out(PlanDev P, int nrhs, const double* y, double* X,
   const int64_t v = blockIdx.y;
   const double* yv = y + v * ylen;
   double* xv = X + v * P.n;
-  if (*(const volatile int32_t*)(status + v / nrhs) & kSolveGaveUp) {   // not a solution
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < P.n;
-         k += (int64_t)gridDim.x * blockDim.x)
-      xv[k] = __longlong_as_double(kNaN);
-    return;
-  }
+  const bool gave_up = status[v / nrhs] & kSolveGaveUp;   // not a solution
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < P.n;
        k += (int64_t)gridDim.x * blockDim.x) {
     if (!transpose) {            // symbolic.cc:238-245
-      const double b = yv[P.row_perm_inv[k]];
-      xv[k] = P.row_scale ? b * P.row_scale[k] : b;
+      double b = yv[P.row_perm_inv[k]];
+      b = P.row_scale ? b * P.row_scale[k] : b;
+      xv[k] = gave_up ? __longlong_as_double(kNaN) : b;
     } else {                     // lambda[col_perm[k]] = col_scale_perm[k] * w[k]
-      xv[P.col_perm[k]] = P.col_scale_perm ? P.col_scale_perm[k] * yv[k] : yv[k];
+      const double w = P.col_scale_perm ? P.col_scale_perm[k] * yv[k] : yv[k];
+      xv[P.col_perm[k]] = gave_up ? __longlong_as_double(kNaN) : w;
     }
   }
 }

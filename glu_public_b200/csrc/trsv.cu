@@ -19,8 +19,8 @@
 // U is divided row by row by its diagonal while the CTA waits (one more rounding of each entry, a
 // division less on the chain of pivots: 0.94 -> 0.38 ms together with the polled values, against
 // progress counters that needed a fence and a second look).  Where that rounding has no bound or
-// something overflows, the rows are solved undivided (solve_block; the look costs 2 us of 554 of a
-// transposed solve at n = 20,000).
+// something overflows, the rows are solved undivided (solve_block; the look costs 5 us of 480 of a
+// solve at n = 20,000).
 //
 // It replaces the reference's dense part of Symbolic_Matrix::solve (src/symbolic.cc:221-236).
 #include <cuda_runtime.h>
@@ -46,15 +46,15 @@ constexpr int kDs = 66;              // column stride of a staged triangle: rows
 
 template <int NV>
 constexpr int flow_smem() {
-  return (kB * kDs + 2 * kB * NV + 4 * NV * kB + kB + 1) * 8;
+  return (kB * kDs + 2 * kB * NV + 4 * NV * kB + kB) * 8;
 }
 
 // The 64 x 64 triangle at T (T[i + kDs * j]) for one vector, rows lane and lane + 32 in r0 and r1.
-// which: 0 = L (unit lower, forward), 1 = U (backward), 2 = U^T (forward), 3 = L^T (backward), the
-// rows of which 1 and 2 divided by their diagonal beforehand.
-// Each solved value is broadcast and pushed into the remaining rows.
-template <int WHICH>
-__device__ __forceinline__ void triangle(const double* __restrict__ T, int lane, double& r0,
+// which: 0 = L (unit lower, forward), 1 = U (backward), 2 = U^T (forward), 3 = L^T (backward).
+// Each solved value is broadcast and pushed into the remaining rows.  DIV: divide by the diagonal
+// (which 1, 2) with its reciprocals rc; otherwise the rows were divided by it beforehand.
+template <int WHICH, bool DIV>
+__device__ __forceinline__ void triangle(const double* __restrict__ T, const double* __restrict__ rc, int lane, double& r0,
                                          double& r1) {
   constexpr bool fwd = WHICH == 0 || WHICH == 2;
   constexpr int si = WHICH < 2 ? 1 : kDs, sj = WHICH < 2 ? kDs : 1;   // M(i, j) = T[i si + j sj]
@@ -67,7 +67,10 @@ __device__ __forceinline__ void triangle(const double* __restrict__ T, int lane,
     for (int q = 0; q < 32; ++q) {
       const int p = fwd ? q : 31 - q;         // lane of the pivot
       const int j = lo ? p : p + 32;
-      const double xj = __shfl_sync(0xffffffffu, lo ? r0 : r1, p);
+      double x = lo ? r0 : r1;
+      if (DIV) x = quotient(x, T[j * (kDs + 1)], rc[j]);
+      const double xj = __shfl_sync(0xffffffffu, x, p);
+      if (DIV && lane == p) (lo ? r0 : r1) = xj;
       const bool rest = fwd ? lane > p : lane < p;
       if (lo) {
         if (rest) r0 -= c0[j * sj] * xj;
@@ -93,8 +96,8 @@ struct DiagBlock {
   }
 };
 
-// The same solve for which 1 and 2 with the rows as they are and a division per pivot, for the
-// blocks and vectors that the divided rows do not serve (see solve_block).
+// The same solve for which 1 and 2 from where the block lies, with a division per pivot, for the
+// vectors that the divided rows do not serve (see solve_block).
 template <int WHICH>
 __device__ __forceinline__ double2 triangle_divide(DiagBlock M, double r0, double r1) {
   static_assert(WHICH == 1 || WHICH == 2, "");
@@ -115,19 +118,21 @@ __device__ __forceinline__ double2 triangle_divide(DiagBlock M, double r0, doubl
 
 // Rows of the staged triangle divided by their diagonal (U: row i; U^T: column i of U), its
 // reciprocals in rc: the division leaves the chain of pivots for one more rounding of each entry.
-// *lost is set where a quotient drops below the normal range and with it the rounding's bound.
+// Where a quotient by more than 2^64 drops below the normal range, and with it the rounding's bound,
+// the first row to be solved is made NaN, which solve_block takes up.  (By less, the entry was
+// below 2^-958, as some fill of large blocks is, and is off by 2^-1011 at most.)
 template <bool TRANS>
-__device__ __forceinline__ void divide_rows(double* Ds, const double* rc, int* lost) {
+__device__ __forceinline__ void divide_rows(double* Ds, double* rc) {
   bool low = false;
   for (int e = threadIdx.x; e < kB * kB; e += 256) {
     const int i = e % kB, j = e / kB, d = TRANS ? j : i;
     if (i < j) {
-      const double v = Ds[i + j * kDs], q = quotient(v, Ds[d * (kDs + 1)], rc[d]);
+      const double v = Ds[i + j * kDs], dd = Ds[d * (kDs + 1)], q = quotient(v, dd, rc[d]);
       Ds[i + j * kDs] = q;
-      low |= (__double2hiint(q) & 0x7ff00000) == 0 && v != 0.0;
+      low |= (__double2hiint(q) & 0x7ff00000) == 0 && v != 0.0 && fabs(dd) > 0x1p64;
     }
   }
-  if (low) *lost = 1;
+  if (low) rc[TRANS ? 0 : kB - 1] = __longlong_as_double(kNaN);
 }
 
 // Rows not finite, a bit each.
@@ -136,33 +141,38 @@ __device__ __forceinline__ unsigned long long bad_rows(double r0, double r1) {
          (unsigned long long)__ballot_sync(0xffffffffu, !finite_bits(r1)) << 32;
 }
 
-// One vector's rows of the block, staged at Ds (diagonal's reciprocals rc).  The divided rows
-// serve if the diagonal's and the quotients' exponents are ordinary (`plain`) and nothing
-// overflows on the way: a quotient may where the undivided sum does not (U(i, j) / d or y / d with
-// d of 2^-900), which shows as the first value that is not finite lying before the first such
-// row of the right-hand side.  Otherwise the rows are solved again with divisions.
+// One vector's rows of the block, staged at Ds (diagonal's reciprocals rc), divided by the diagonal
+// if its exponents are ordinary (`plain`).  That serves unless something is not finite on the way
+// that would be with a division at the end: a quotient overflows where the undivided sum does not
+// (U(i, j) / d or y / d with d of 2^-900), a reciprocal is infinite.  It shows as the first value
+// that is not finite lying before the first such row of the right-hand side; the rows are then
+// solved again from where they lie.
 template <int WHICH>
 __device__ __forceinline__ void solve_block(const double* Ds, const double* rc, int lane,
                                             bool plain, const DiagBlock& M, double& y0,
                                             double& y1) {
   if (WHICH == 0 || WHICH == 3) {
-    triangle<WHICH>(Ds, lane, y0, y1);
+    triangle<WHICH, false>(Ds, rc, lane, y0, y1);
     return;
   }
-  double x0 = quotient(y0, Ds[lane * (kDs + 1)], rc[lane]);
-  double x1 = quotient(y1, Ds[(lane + 32) * (kDs + 1)], rc[lane + 32]);
-  triangle<WHICH>(Ds, lane, x0, x1);
-  if (!plain || __any_sync(0xffffffffu, !finite_bits(x0) || !finite_bits(x1))) {
-    const unsigned long long in = bad_rows(y0, y1), out = bad_rows(x0, x1);
-    if (!plain || (WHICH == 2 ? (unsigned)__ffsll(out) - 1u < (unsigned)__ffsll(in) - 1u
-                              : __clzll(out) < __clzll(in))) {
-      const double2 x = triangle_divide<WHICH == 2 ? 2 : 1>(M, y0, y1);
-      x0 = x.x;
-      x1 = x.y;
+  const double w0 = y0, w1 = y1;
+  if (plain) {
+    y0 = quotient(y0, Ds[lane * (kDs + 1)], rc[lane]);
+    y1 = quotient(y1, Ds[(lane + 32) * (kDs + 1)], rc[lane + 32]);
+    triangle<WHICH, false>(Ds, rc, lane, y0, y1);
+    if (!__any_sync(0xffffffffu, !finite_bits(y0) || !finite_bits(y1))) return;
+  } else {
+    triangle<WHICH, true>(Ds, rc, lane, y0, y1);
+  }
+  if (__any_sync(0xffffffffu, !finite_bits(y0) || !finite_bits(y1))) {
+    const unsigned long long in = bad_rows(w0, w1), out = bad_rows(y0, y1);
+    if (WHICH == 2 ? (unsigned)__ffsll(out) - 1u < (unsigned)__ffsll(in) - 1u
+                   : __clzll(out) < __clzll(in)) {
+      const double2 x = triangle_divide<WHICH == 2 ? 2 : 1>(M, w0, w1);
+      y0 = x.x;
+      y1 = x.y;
     }
   }
-  y0 = x0;
-  y1 = x1;
 }
 
 __device__ __forceinline__ double ld_relaxed(const double* p) {
@@ -220,7 +230,6 @@ __device__ bool flow_phase(const double* __restrict__ D, int64_t ld, int nblk, c
   double* xs = Ds + kB * kDs;                 // [2][kB][NV]
   double* red = xs + 2 * kB * NV;             // [4][NV][kB]
   double* rc = red + 4 * NV * kB;
-  int* lost = reinterpret_cast<int*>(rc + kB);
   const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
   const int vec = warp % NV;                  // the vector whose triangle this warp solves
   for (int o = r; o < nblk; o += G) {
@@ -280,10 +289,9 @@ __device__ bool flow_phase(const double* __restrict__ D, int64_t ld, int nblk, c
           rc[tid] = 1.0 / d;
           const int ex = (__double2hiint(d) >> 20) & 0x7ff;
           odd = ex < 64 || ex > 0x7ff - 64;
-          if (tid == 0) *lost = 0;
         }
         plain = !__syncthreads_or(odd);
-        if (plain) divide_rows<trans>(Ds, rc, lost);
+        if (plain) divide_rows<trans>(Ds, rc);
       }
     };
     for (int k = 0; k < o; ++k) {
@@ -342,8 +350,7 @@ __device__ bool flow_phase(const double* __restrict__ D, int64_t ld, int nblk, c
     y0 -= s0;
     y1 -= s1;
     // every warp solves (NV < 8: some the same vector), so that no branch holds the shuffles
-    solve_block<WHICH>(Ds, rc, lane, plain && (!diag || *lost == 0),
-                       DiagBlock{D + b + b * ld, ld, nullptr, 0, kB}, y0, y1);
+    solve_block<WHICH>(Ds, rc, lane, plain, DiagBlock{D + b + b * ld, ld, nullptr, 0, kB}, y0, y1);
     if (warp < nv) {
       double* xo = xb + vec * xl + b + lane;
       st_relaxed(xo, unsolved(y0) ? __longlong_as_double(kNaN) : y0);
@@ -453,7 +460,6 @@ __device__ bool front_block(const PlanDev& P, const double* __restrict__ V, int 
   double* xs = Ds + kB * kDs;                 // [2][kB][NV]
   double* red = xs + 2 * kB * NV;             // [4][NV][kB]
   double* rc = red + 4 * NV * kB;
-  int* lost = reinterpret_cast<int*>(rc + kB);
   const int tid = threadIdx.x, lane = tid % kWarp, warp = tid / kWarp;
   const int vec = warp % NV;
   const int s0 = P.fs0[f], w = P.fw[f], nblk = (w + kB - 1) / kB;
@@ -522,11 +528,10 @@ __device__ bool front_block(const PlanDev& P, const double* __restrict__ V, int 
       if (diag) rc[tid] = 1.0 / d;
       const int ex = (__double2hiint(d) >> 20) & 0x7ff;
       odd = ex < 64 || ex > 0x7ff - 64;
-      if (tid == 0) *lost = 0;
     }
     if (diag) {
       plain = !__syncthreads_or(odd);
-      if (plain) divide_rows<trans>(Ds, rc, lost);
+      if (plain) divide_rows<trans>(Ds, rc);
     }
   };
   for (int k = 0; k < o; ++k) {
@@ -581,8 +586,7 @@ __device__ bool front_block(const PlanDev& P, const double* __restrict__ V, int 
   }
   y0 -= t0;
   y1 -= t1;
-  solve_block<WHICH>(Ds, rc, lane, plain && (!diag || *lost == 0),
-                     DiagBlock{V, 0, lp, b, min(kB, w - b)}, y0, y1);
+  solve_block<WHICH>(Ds, rc, lane, plain, DiagBlock{V, 0, lp, b, min(kB, w - b)}, y0, y1);
   if (warp < nv) {
     double* xo = xb + vec * xl + b;
 #pragma unroll

@@ -76,9 +76,9 @@ def test_front_solves(nrhs, transpose, dense_threshold):
 @pytest.mark.parametrize("count", [24, 40, 57])
 def test_instances_behind_a_wait_that_gave_up(count, transpose):
     """A front of eleven row blocks in more instances than the GPU takes at once, with a bound of a
-    nanosecond: the first instance's diagonals are at the bottom of the exponent range, so that its
-    blocks take long and the waits for them give up.  Whatever a CTA that gave up had left to do
-    belongs to other instances too: each is flagged or right."""
+    nanosecond: the first instance's rows cannot be divided by their diagonals in advance, so that
+    its blocks take long and the waits for them give up.  Whatever a CTA that gave up had left to
+    do belongs to other instances too: each is flagged or right."""
     import torch
     w, n = 700, 760
     rng = np.random.default_rng(4)
@@ -94,17 +94,15 @@ def test_instances_behind_a_wait_that_gave_up(count, transpose):
     idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
     plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
     batch = glu.Batch(plan, count)
-    scale = np.ones(count)
-    scale[0] = 2.0 ** -990
     b = torch.as_tensor(rng.standard_normal((count, 1, n)), device="cuda")
-    b[0] *= 2.0 ** -990
-    batch.load_lu_values(torch.as_tensor(scale[:, None] * sym.val[None], device="cuda"))
+    col = np.repeat(np.arange(n), np.diff(sym.sym_c_ptr.astype(np.int64)))
+    val = np.repeat(sym.val[None], count, 0)
+    val[0] *= np.where(col == sym.sym_r_idx, 2.0 ** 700, 2.0 ** -400)
+    batch.load_lu_values(torch.as_tensor(val, device="cuda"))
     batch.refactor(0.0)
     x = batch.solve(b, transpose=transpose)
     flagged = batch.status() & 8
     assert flagged[0]
-    cp = sym.sym_c_ptr.astype(np.int64)
-    col = np.repeat(np.arange(n), np.diff(cp))
     for i in np.flatnonzero(flagged == 0):
         lu = np.zeros((n, n))                 # [column, row]
         lu[col, sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
