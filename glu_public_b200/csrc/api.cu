@@ -181,6 +181,7 @@ struct glu_batch_s {
   };
   std::vector<Use> uses;
   size_t nuses = 0;             // of the events made, those in use
+  bool on_default = false;      // used on the default stream, which needs no event until the end
   bool untracked = false;
 };
 
@@ -506,10 +507,9 @@ int batch_residual_view(glu_batch_t b, const PlanDev** P, int* count, int* devic
 }
 }  // namespace glu
 
-// Notes that the call has put work of the batch on stream s.
-static void note_use(glu_batch_s* b, cudaStream_t s) {
+// Records an event after the batch's work on stream s.
+static void note_event(glu_batch_s* b, cudaStream_t s) {
   constexpr size_t kMaxUses = 4;
-  if (b->untracked || !b->own_vals) return;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
   bool ok = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
@@ -530,6 +530,17 @@ static void note_use(glu_batch_s* b, cudaStream_t s) {
     cudaGetLastError();
     b->untracked = true;
   }
+}
+
+// Notes that the call has put work of the batch on stream s.  (An event after every call costs some
+// 1 us; the default stream is always there to record one when the batch is destroyed.)
+static void note_use(glu_batch_s* b, cudaStream_t s) {
+  if (b->untracked || !b->own_vals) return;
+  if (s == nullptr || s == cudaStreamLegacy) {
+    b->on_default = true;
+    return;
+  }
+  note_event(b, s);
 }
 
 // Clears what a new batch has cleared, once the work noted on its buffers is done; waits for that
@@ -634,6 +645,9 @@ static bool glu::free_spares(int device) {
 static bool keep_spare(glu_batch_s* b) {
   const size_t bytes = batch_bytes(b);
   if (!b->own_vals || b->untracked || bytes > kSpareBytes) return false;
+  if (b->on_default) note_event(b, cudaStreamLegacy);
+  if (b->untracked) return false;
+  b->on_default = false;
   b->loaded = b->factored = false;
   b->launches = 0;
   std::lock_guard<std::mutex> lock(g_spares_mu);
