@@ -158,9 +158,11 @@ __device__ __forceinline__ ColGroup cta_group() {
 // Measured, sparse levels of one refactorization: n = 20,000 1.13 -> 0.39 ms (a few pairs of 2,860
 // updates in columns of 2,850 pairs), 512 x 512 x 2 nodes 9.4 -> 6.8 ms, 64 x n = 20,000 5.6 -> 3.0 ms;
 // sharing long pairs in pieces wherever there are fewer than groups, not a quarter as many: 128 x 128
-// x 2 nodes 2.15 ms against 1.88.  Without a dense block, where a column has up to a thousand pairs
-// of a thousand updates: 64 x n = 2,000 8.5 -> 6.1 ms, one n = 4,960 17.2 -> 17.3, four of them 15.9 ->
-// 16.8 (the row loop unrolled by two: 6.95, 19.5 and 16.7).
+// x 2 nodes 2.15 ms against 1.88.  A pair that a group has to itself goes four rows at a time, or the
+// long columns of a plan without a dense block (up to a thousand pairs of a thousand updates, a pair
+// a warp) have one load in flight: one n = 4,960 17.3 -> 10.3 ms, four of them 16.8 -> 10.4 (15.0 with
+// a loop over the pairs alone), eight 16.4 -> 15.2, 128 x 128 x 2 nodes 4.09 -> 3.91 ms a pass;
+// 64 x n = 2,000 without a dense block 8.5 -> 6.1 ms before that.
 __device__ __forceinline__ void apply_pairs(const PlanDev& P, double* __restrict__ V, uint32_t c,
                                             const double* __restrict__ Lc, uint32_t nL, int64_t w,
                                             int64_t W, int il, int width, unsigned mask) {
@@ -200,6 +202,25 @@ __device__ __forceinline__ void apply_pairs(const PlanDev& P, double* __restrict
       u = V[P.pair_uslot[mine]];
     }
     const int n = (int)min((int64_t)width, (q1 - q + W - 1) / W);
+    if (n == 1) {                              // a pair by itself: four of its rows in flight
+      const uint32_t ns = __shfl_sync(mask, nsp, 0, width);
+      const int32_t* tm = P.tmap + __shfl_sync(mask, mo, 0, width);
+      const double us = __shfl_sync(mask, u, 0, width);
+      for (uint32_t k0 = il; k0 < ns; k0 += 4 * width) {
+        int32_t t[4];
+        double l[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const uint32_t k = k0 + h * width;
+          t[h] = k < ns ? tm[k] : -1;
+          l[h] = k < ns ? Lc[k] : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          if (t[h] >= 0) atomicAdd(V + t[h], -(l[h] * us));
+      }
+      continue;
+    }
     for (int i = 0; i < n; i += 4) {
       const int32_t* tm[4];
       uint32_t ns[4], most = 0;

@@ -118,6 +118,32 @@ def test_long_and_short_pairs(options):
         check_lu(torch, lu, np.ascontiguousarray(a.T * s)[None])
 
 
+@pytest.mark.parametrize("pairs", [1, 7, 8, 9, 17])
+@pytest.mark.parametrize("options", [{}, dict(sparse_persistent=0, sparse_warps_per_col=8, level_warps_per_sm=0),
+                                     dict(sparse_persistent=0, sparse_warps_per_col=1, sparse_col_lanes=8)])
+def test_a_pair_to_itself(pairs, options):
+    """Columns of the LENGTHS with about a pair for each group of lanes that shares them: a pair alone
+    takes its rows four at a time.  |L U - A| <= 4 n u |L| |U|."""
+    import torch
+    n = 1100
+    a = long_columns(n, 13)
+    for k in range(len(LENGTHS)):
+        a[3 + 2 * k, 60 + 20 * k:60 + 20 * k + pairs] = 0.02
+    a[np.arange(n), np.arange(n)] += 1.0
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, **{"dense_threshold": 2.0, "front_min_w": 0, **options})
+    batch = glu.Batch(plan, 2)
+    batch.load_lu_values(torch.as_tensor(np.stack([sym.val, -3.0 * sym.val]), device="cuda"))
+    batch.refactor(0.0)
+    cp = sym.sym_c_ptr.astype(np.int64)
+    for i, s in enumerate((1.0, -3.0)):
+        lu = np.zeros((n, n))                 # [column, row]
+        lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
+        check_lu(torch, lu, np.ascontiguousarray(a.T * s)[None])
+
+
 @pytest.mark.parametrize("transpose", [False, True])
 def test_residual_of_long_rows(transpose):
     """r = b - op(A) x with rows of 63 to 1,100 entries: within 2 n u |A| |x| of numpy's."""
