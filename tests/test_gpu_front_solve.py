@@ -73,6 +73,34 @@ def test_front_solves(nrhs, transpose, dense_threshold):
 
 
 @pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("nrhs", [1, 3])
+def test_front_solves_of_many_instances(nrhs, transpose):
+    """More row blocks than the GPU takes at once: a CTA has several, of different instances."""
+    import torch
+    a = fronts_matrix(12)
+    n, count = a.shape[0], 150
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, dense_threshold=2.0, front_min_flops=1.0)
+    assert plan.stat("front_w_max") >= 200    # four row blocks at least
+    idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
+    plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
+    batch = glu.Batch(plan, count)
+    batch.load_lu_values(torch.as_tensor(np.linspace(1.0, 2.0, count)[:, None] * sym.val[None],
+                                         device="cuda"))
+    batch.refactor(0.0)
+    b = torch.as_tensor(np.random.default_rng(1).standard_normal((count, nrhs, n)), device="cuda")
+    x = batch.solve(b, transpose=transpose)
+    assert not batch.status().any()
+    col = np.repeat(np.arange(n), np.diff(sym.sym_c_ptr.astype(np.int64)))
+    for i in range(0, count, 7):
+        lu = np.zeros((n, n))                 # [column, row]
+        lu[col, sym.sym_r_idx] = batch.get_lu(i).cpu().numpy()
+        check_solve(torch, lu, b[i], x[i], transpose)
+
+
+@pytest.mark.parametrize("transpose", [False, True])
 @pytest.mark.parametrize("count", [24, 40, 57])
 def test_instances_behind_a_wait_that_gave_up(count, transpose):
     """A front of eleven row blocks in more instances than the GPU takes at once, with a bound of a

@@ -242,3 +242,32 @@ def test_workspace_of_many_vectors():
         graph.replay()
         torch.cuda.synchronize()
         check_solve(torch, lu, few[0], y[0], False)
+
+
+@pytest.mark.parametrize("transpose", [False, True])
+@pytest.mark.parametrize("count", [1, 30, 150])
+def test_rows_whose_waits_give_up(count, transpose):
+    """The rows' dataflow with a bound of a nanosecond: every instance is flagged, and NaN, or right."""
+    import torch
+    n = 1100
+    a = long_columns(n, 7)
+    col, row = np.nonzero(a.T)
+    ap = np.searchsorted(col, np.arange(n + 1)).astype(np.uint32)
+    sym = glu.SymbolicMatrix(n).analyze(row.astype(np.uint32), ap, a[row, col])
+    plan = glu.Plan(sym, dense_threshold=2.0, front_min_w=0, sparse_persistent=0, level_wait_ms=1e-6)
+    idx, one = np.arange(n, dtype=np.uint32), np.ones(n)
+    plan.set_solve_maps(glu.NicsluArrays(n, idx, idx, idx, idx, one, one, 0))
+    batch = glu.Batch(plan, count)
+    batch.load_lu_values(torch.as_tensor(sym.val, device="cuda").repeat(count, 1))
+    batch.refactor(0.0)
+    b = torch.as_tensor(np.random.default_rng(3).standard_normal((count, 1, n)), device="cuda")
+    x = batch.solve(b, transpose=transpose)
+    flagged = batch.status()
+    assert not (flagged & ~8).any()
+    assert bool(x[torch.as_tensor(flagged != 0, device="cuda")].isnan().all())
+    cp = sym.sym_c_ptr.astype(np.int64)
+    lu = np.zeros((n, n))
+    lu[np.repeat(np.arange(n), np.diff(cp)), sym.sym_r_idx] = batch.get_lu(0).cpu().numpy()
+    good = np.flatnonzero(flagged == 0)
+    if good.size:
+        check_solve(torch, lu, b[good, 0], x[good, 0], transpose)
