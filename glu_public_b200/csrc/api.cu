@@ -175,12 +175,12 @@ struct glu_batch_s {
   // the end of the last work on each stream the batch was used on, for the next owner of its buffers
   // to wait for; `untracked`: its work is in a graph, which may be launched anywhere, or on more
   // streams than this
+  static constexpr int kMaxUses = 4;
   struct Use {
     unsigned long long stream;  // cudaStreamGetId: a later stream of the same handle is another
-    cudaEvent_t done;
-  };
-  std::vector<Use> uses;
-  size_t nuses = 0;             // of the events made, those in use
+    cudaEvent_t done;           // made when first needed
+  } uses[kMaxUses] = {};
+  int nuses = 0;
   bool on_default = false;      // used on the default stream, which needs no event until the end
   bool untracked = false;
 };
@@ -509,27 +509,27 @@ int batch_residual_view(glu_batch_t b, const PlanDev** P, int* count, int* devic
 
 // Records an event after the batch's work on stream s.
 static void note_event(glu_batch_s* b, cudaStream_t s) {
-  constexpr size_t kMaxUses = 4;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
-  bool ok = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone &&
-            cudaStreamGetId(s, &id) == cudaSuccess;
-  size_t i = 0;
-  while (ok && i < b->nuses && b->uses[i].stream != id) ++i;
-  if (ok && i == b->uses.size()) {
-    cudaEvent_t e = nullptr;
-    ok = i < kMaxUses && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-    if (ok) b->uses.push_back({id, e});
+  bool ok = cudaStreamIsCapturing(s, &cs) == cudaSuccess &&
+            (cs != cudaStreamCaptureStatusNone || cudaStreamGetId(s, &id) == cudaSuccess);
+  int i = 0;
+  while (i < b->nuses && b->uses[i].stream != id) ++i;
+  if (ok && (cs != cudaStreamCaptureStatusNone || i == glu_batch_s::kMaxUses)) {
+    b->untracked = true;
+    return;
   }
-  if (ok) {
-    b->uses[i].stream = id;
-    b->nuses = std::max(b->nuses, i + 1);
-    ok = cudaEventRecord(b->uses[i].done, s) == cudaSuccess;
-  }
+  glu_batch_s::Use* u = b->uses + i;
+  ok = ok &&
+       (u->done || cudaEventCreateWithFlags(&u->done, cudaEventDisableTiming) == cudaSuccess) &&
+       cudaEventRecord(u->done, s) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     b->untracked = true;
+    return;
   }
+  u->stream = id;
+  b->nuses = std::max(b->nuses, i + 1);
 }
 
 // Notes that the call has put work of the batch on stream s.  (An event after every call costs some
@@ -549,7 +549,7 @@ static bool batch_clear(glu_batch_s* b, size_t gbytes) {
   if (!b->own_stream &&
       cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking) != cudaSuccess)
     return false;
-  for (size_t i = 0; i < b->nuses; ++i)
+  for (int i = 0; i < b->nuses; ++i)
     if (cudaStreamWaitEvent(b->own_stream, b->uses[i].done, 0) != cudaSuccess) return false;
   b->nuses = 0;
   return (gbytes == 0 || cudaMemsetAsync(b->gbuf, 0, gbytes, b->own_stream) == cudaSuccess) &&
@@ -581,7 +581,8 @@ static void batch_free(glu_batch_s* b) {
   if (!b) return;
   drop_graph(b);
   if (b->own_stream) cudaStreamDestroy(b->own_stream);
-  for (const glu_batch_s::Use& u : b->uses) cudaEventDestroy(u.done);
+  for (const glu_batch_s::Use& u : b->uses)
+    if (u.done) cudaEventDestroy(u.done);
   for (int i = 0; i < glu_batch_s::kFrontStreams; ++i) {
     if (b->fstream[i]) cudaStreamDestroy(b->fstream[i]);
     if (b->fjoin[i]) cudaEventDestroy(b->fjoin[i]);
@@ -1301,10 +1302,11 @@ int glu_load_values(glu_batch_t b, int32_t first, int32_t count, const double* a
   glu::launch_prepare_blob(b->plan->P, b->vals, first, count, asm_ok, s, lc);
   glu::launch_ingest(b->plan->P, b->vals, first, count, a_dev, s, lc);
   cudaMemsetAsync(b->asm_flag + first, asm_ok ? 1 : 0, count, s);
-  note_use(b, s);
   b->loaded = true;
   b->factored = false;
-  return glu::cuda_status("load values");
+  const int st = glu::cuda_status("load values");
+  note_use(b, s);
+  return st;
 }
 
 int glu_load_lu_values(glu_batch_t b, int32_t first, int32_t count, const double* val_dev,
@@ -1318,10 +1320,11 @@ int glu_load_lu_values(glu_batch_t b, int32_t first, int32_t count, const double
   glu::launch_prepare_blob(b->plan->P, b->vals, first, count, false, s, lc);
   glu::launch_load_lu(b->plan->P, b->vals, first, count, val_dev, s, lc);
   cudaMemsetAsync(b->asm_flag + first, 0, count, s);
-  note_use(b, s);
   b->loaded = true;
   b->factored = false;
-  return glu::cuda_status("load LU values");
+  const int st = glu::cuda_status("load LU values");
+  note_use(b, s);
+  return st;
 }
 
 int glu_refactor(glu_batch_t b, double pert, void* stream) {
@@ -1504,8 +1507,9 @@ int glu_residual(glu_batch_t b, int32_t nrhs, const double* a_dev, const double*
   glu::LaunchCounter lc;
   glu::launch_residual(b->plan->P, b->count, nrhs, a_dev, X_dev, B_dev, nullptr, b->norms,
                        resid_dev, transpose, s, lc);
+  st = glu::cuda_status("residual");
   note_use(b, s);
-  return glu::cuda_status("residual");
+  return st;
 }
 
 int glu_refine(glu_batch_t b, int32_t nrhs, const double* a_dev, const double* B_dev,
@@ -1544,8 +1548,9 @@ int glu_get_lu(glu_batch_t b, int32_t instance, double* val_dev, void* stream) {
   glu::DeviceGuard g(b->plan->device);
   glu::LaunchCounter lc;
   glu::launch_export_lu(b->plan->P, b->vals, instance, val_dev, (cudaStream_t)stream, lc);
+  const int st = glu::cuda_status("export LU");
   note_use(b, (cudaStream_t)stream);
-  return glu::cuda_status("export LU");
+  return st;
 }
 
 int glu_graph_capture(glu_batch_t b, const double* a_dev, int32_t nrhs, const double* B_dev,
