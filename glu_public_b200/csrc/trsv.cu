@@ -54,7 +54,8 @@ constexpr int flow_smem() {
 // Each solved value is broadcast and pushed into the remaining rows.  DIV: divide by the diagonal
 // (which 1, 2) with its reciprocals rc; otherwise the rows were divided by it beforehand.
 template <int WHICH, bool DIV>
-__device__ __forceinline__ void triangle(const double* __restrict__ T, const double* __restrict__ rc, int lane, double& r0,
+__device__ __forceinline__ void triangle(const double* __restrict__ T,
+                                         const double* __restrict__ rc, int lane, double& r0,
                                          double& r1) {
   constexpr bool fwd = WHICH == 0 || WHICH == 2;
   constexpr int si = WHICH < 2 ? 1 : kDs, sj = WHICH < 2 ? kDs : 1;   // M(i, j) = T[i si + j sj]
